@@ -63,7 +63,10 @@ template <typename T>
 struct StoutBufs {
     std::vector<LinkPlanes<T>> lv;   // lv[k] = links after k+1 stout levels
     std::vector<AlgPlanes<T>> Q;     // Q[k] = exponent of level k -> k+1
-    AlgPlanes<T> lam{nullptr, 0};
+    // derivative: Lambda, the transported derivative, the plaquette terms at the site and
+    // away from it (twelve plane fields)
+    AlgPlanes<T> lam{nullptr, 0}, dir{nullptr, 0}, loc{nullptr, 0}, rem{nullptr, 0};
+    // matrix derivatives of the one-thread-per-link form (allocated on its first use)
     LinkPlanes<T> za{nullptr, 0}, zp{nullptr, 0};
 };
 
@@ -229,9 +232,9 @@ struct mag_ctx {
         return alloc((void**)&l.p, sizeof(cplx<T>) * 4 * LinkPlanes<T>::kElems * (size_t)vpad);
     }
     template <typename T>
-    int alloc_alg(AlgPlanes<T>& a) {
+    int alloc_alg(AlgPlanes<T>& a, int planes = 4) {
         a.vpad = vpad;
-        return alloc((void**)&a.p, sizeof(T) * 32 * (size_t)vpad);
+        return alloc((void**)&a.p, sizeof(T) * 8 * planes * (size_t)vpad);
     }
     template <typename T>
     int alloc_stout(StoutBufs<T>& b, bool backward) {
@@ -243,8 +246,9 @@ struct mag_ctx {
         }
         if (backward && p.n_stout > 0) {
             MAG_TRY(alloc_alg(b.lam));
-            MAG_TRY(alloc_links(b.za));
-            MAG_TRY(alloc_links(b.zp));
+            MAG_TRY(alloc_alg(b.dir));
+            MAG_TRY(alloc_alg(b.loc));
+            MAG_TRY(alloc_alg(b.rem, 12));
         }
         return MAG_OK;
     }
@@ -410,8 +414,47 @@ struct mag_ctx {
     // A sharded context exchanges halos (hx) after every launch whose output a
     // later kernel reads across the shard boundary: the links whose force is
     // taken, each smeared level, the double links and Lambda of each level.
+    //
+    // Smeared links: the top level's force is the derivative with respect to the top
+    // links in the Lie algebra (the force kernel, beta/3 included; everything after it
+    // is linear), and each level maps it to the level below (kernels_smear.cu).
     template <typename T>
     void force_eval(LinkPlanes<T> Uin, AlgPlanes<T> Fout, StoutBufs<T>& b) {
+        if (gather[sizeof(T) == 8 ? 0 : 1]) return force_eval_gather(Uin, Fout, b);
+        hx(Uin);
+        LinkPlanes<T> cur = Uin;
+        for (int k = 0; k < p.n_stout; k++) {
+            launch_stout_forward<T>(geom, cur, b.lv[k], b.Q[k], var<T>(KF_STOUT_FWD), stream);
+            cur = b.lv[k];
+            hx(cur);
+        }
+        if (iwasaki) {
+            launch_double_link<T>(geom, cur, wbuf<T>(), stream);
+            hx(wbuf<T>());
+        }
+        launch_force<T>(geom, cur, wbuf<T>(), Fout, iwasaki, var<T>(KF_FORCE), stream);
+        if (p.n_stout > 0) launch_lambda<T>(geom, b.Q[p.n_stout - 1], Fout, b.lam, b.dir, stream);
+        for (int k = p.n_stout - 1; k >= 0; k--) {
+            hx(b.lam);
+            launch_plaq_chain<T>(geom, k == 0 ? Uin : b.lv[k - 1], b.lam, b.loc, b.rem, stream);
+            if (k == 0) launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, nullptr, Fout, stream);
+            else launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, &b.Q[k - 1], b.lam, stream);
+        }
+        if (any_mag) launch_constraint_fixup<T>(geom, Uin, Fout, stream);
+    }
+
+    // The force by the one-thread-per-link kernels with matrix derivatives, whose launch
+    // shapes mag_set_kernel_variant selects: after such a call the context's forces of
+    // that precision take this form.
+    bool gather[2] = {false, false};
+    template <typename T>
+    int ensure_gather(StoutBufs<T>& b) {
+        if (p.n_stout == 0 || b.zp.p) return MAG_OK;
+        if (!b.za.p) MAG_TRY(alloc_links(b.za));
+        return alloc_links(b.zp);
+    }
+    template <typename T>
+    void force_eval_gather(LinkPlanes<T> Uin, AlgPlanes<T> Fout, StoutBufs<T>& b) {
         hx(Uin);
         if (p.n_stout == 0) {
             if (iwasaki) {
@@ -459,7 +502,7 @@ struct mag_ctx {
     void launch_one(KernelFamily f, int v, StoutBufs<T>& b, LinkPlanes<T> Uin, AlgPlanes<T> Fo, LinkPlanes<T> zs) {
         const int L = p.n_stout;
         switch (f) {
-            case KF_FORCE: launch_force<T>(geom, Uin, wbuf<T>(), Fo, iwasaki, v, stream); break;
+            case KF_FORCE: launch_force<T>(geom, L ? b.lv[L - 1] : Uin, wbuf<T>(), Fo, iwasaki, v, stream); break;
             case KF_STAPLE:
                 launch_staple_dagger<T>(geom, L ? b.lv[L - 1] : Uin, wbuf<T>(), L ? b.za : zs, iwasaki, v, stream);
                 break;
@@ -468,6 +511,14 @@ struct mag_ctx {
             case KF_STOUT_CHAIN: launch_stout_chain<T>(geom, Uin, b.lam, b.zp, b.za, v, stream); break;
             default: break;
         }
+    }
+
+    // one launch of a kernel of the derivative's plaquette form, on the thin links
+    template <typename T>
+    void launch_smear(const std::string& w, StoutBufs<T>& b, LinkPlanes<T> Uin, AlgPlanes<T> Fo) {
+        if (w == "lambda") launch_lambda<T>(geom, b.Q[0], Fo, b.lam, b.dir, stream);
+        else if (w == "plaq_chain") launch_plaq_chain<T>(geom, Uin, b.lam, b.loc, b.rem, stream);
+        else launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, &b.Q[0], b.lam, stream);
     }
 
     template <typename T>
@@ -492,7 +543,8 @@ struct mag_ctx {
         force_eval<T>(Uin, Fo, b);
         std::vector<KernelFamily> fams;
         if (p.n_stout == 0) fams = {KF_FORCE};
-        else fams = {KF_STAPLE, KF_STOUT_FWD, KF_STOUT_LAMBDA, KF_STOUT_CHAIN};
+        else if (gather[sizeof(T) == 8 ? 0 : 1]) fams = {KF_STAPLE, KF_STOUT_FWD, KF_STOUT_LAMBDA, KF_STOUT_CHAIN};
+        else fams = {KF_FORCE, KF_STOUT_FWD};
         // Every variant is timed (the report shows them all), but the choice is made among the
         // one-thread-per-link register caps only: those compute bit-identical results, so a run does not
         // depend on timing noise.  The direction-split shapes add their parts in another order (results

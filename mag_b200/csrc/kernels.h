@@ -98,6 +98,25 @@ template <typename T>
 void launch_stout_chain_force(const DevGeom& g, LinkPlanes<T> Ul, AlgPlanes<T> Lam, LinkPlanes<T> Zp, AlgPlanes<T> F,
                               int v, cudaStream_t s);
 
+// ---- stout smearing on plaquettes (kernels_smear.cu); S: six plane fields, Rem: twelve
+// one forward level: Q and U' = e^{iQ} U from the plaquettes S of U
+template <typename T>
+void launch_stout_level(const DevGeom& g, LinkPlanes<T> U, LinkPlanes<T> Uout, AlgPlanes<T> Q, AlgPlanes<T> S,
+                        cudaStream_t s);
+// Lambda and Dir = e^{-i ad_Q} x of a level from the derivative x = X with respect to its smeared links
+template <typename T>
+void launch_lambda(const DevGeom& g, AlgPlanes<T> Q, AlgPlanes<T> X, AlgPlanes<T> Lam, AlgPlanes<T> Dir,
+                   cudaStream_t s);
+// the plaquette terms of Lambda: those of the links at x into Loc, the others into Rem at x
+template <typename T>
+void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
+                       cudaStream_t s);
+// x = Dir + Loc + the Rem terms that belong to a link: Out = Lambda and Dir of the level below with
+// exponents *Q, or Out = x itself when Q is null (the thin links)
+template <typename T>
+void launch_chain_gather(const DevGeom& g, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir, const AlgPlanes<T>* Q,
+                         AlgPlanes<T> Out, cudaStream_t s);
+
 // ---- streaming kernels (kernels_update.cu)
 template <typename TU, typename TX>
 void launch_evolve(const DevGeom& g, LinkPlanes<TU> Uin, LinkPlanes<TU> Uout, AlgPlanes<TX> X, double eps,

@@ -1,0 +1,253 @@
+// kernels_smear.cu -- stout smearing and its derivative on plaquettes (plaq_ops.cuh).
+//
+// A level is two launches, forward and backward alike: one over plaquettes (a block
+// of six warps holds the six planes of a 32-site tile), whose results go to memory
+// as algebra elements, and one over links, which adds up the terms of its six
+// plaquettes (three at the site, three at x - nu) and does the rest of the level.
+//
+// Backward, per link and level: about 1450 multiply-adds instead of 3456 in the
+// one-thread-per-link chain rule and 156 instead of 450 loaded reals, because a
+// plaquette is formed once for its four links; the price is 1.8 KB per site (FP64)
+// of intermediate results.  Measured at 32^4 (ms per launch): chain rule + Lambda
+// 1.65 + 0.57 FP64, 0.69 + 0.24 FP32 before; k_plaq_chain + k_chain_gather 0.70 +
+// 0.33 FP64, 0.38 + 0.17 FP32.  k_chain_gather (2.0 KB per site) runs at the HBM
+// rate (6.6 TB/s at FP64); k_plaq_chain at about half the FP64 pipe, 12 warps per SM.
+#include "kernels.h"
+#include "plaq_ops.cuh"
+
+namespace magb {
+
+namespace {
+
+constexpr int kPlaqBlock = 6 * MAG_TILE;
+constexpr int kLinkBlock = 4 * MAG_TILE;
+
+// plane of warp w: (0,1) (0,2) (0,3) (1,2) (1,3) (2,3)
+__device__ __forceinline__ void plane_of(int w, int& p, int& q) {
+    p = w < 3 ? 0 : w < 5 ? 1 : 2;
+    q = w < 3 ? w + 1 : w < 5 ? w - 1 : 3;
+}
+// index of the plane of directions i != j
+__device__ __forceinline__ int plane_index(int i, int j) {
+    const int p = i < j ? i : j, q = i < j ? j : i;
+    return p == 0 ? q - 1 : p + q;
+}
+
+__device__ __forceinline__ bool locate_tile(const DevGeom& g, ChainInfo& ci, Site& st) {
+    const int gs = blockIdx.x * MAG_TILE + (threadIdx.x & 31);
+    ci = g.chains[g.c2c[gs / MAG_CHUNK]];
+    const int s = gs - ci.off;
+    if (s >= ci.V) return false;
+    decode(ci, s, st);
+    return true;
+}
+
+// S = (P - P^dag) / 2i of every plaquette (plane fields 0..5 of S)
+template <typename T>
+__global__ void __launch_bounds__(kPlaqBlock) k_plaq_sin(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S) {
+    ChainInfo ci;
+    Site st;
+    if (!locate_tile(g, ci, st)) return;
+    const int w = threadIdx.x >> 5;
+    int p, q;
+    plane_of(w, p, q);
+    const int gp = nb_sel(ci, st, p, 1), gq = nb_sel(ci, st, q, 1);
+    const mat3<T> P =
+        plaquette(U.load_rows01(p, st.g), U.load(q, gp), U.load(p, gq), U.load_rows01(q, st.g));
+    S.store(w, st.g, plaq_sin(P, T(1)));
+}
+
+// Q = -i rho TA(stp U^dag) (field-multi.h:32-39) from the plaquettes at x and x - nu, U' = e^{iQ} U
+template <typename T>
+__global__ void __launch_bounds__(kLinkBlock) k_stout_apply(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S,
+                                                            LinkPlanes<T> Uout, AlgPlanes<T> Q) {
+    ChainInfo ci;
+    Site st;
+    if (!locate_tile(g, ci, st)) return;
+    const int mu = threadIdx.x >> 5;
+    herm8<T> sum = herm_zero<T>();
+#pragma unroll 1
+    for (int i = 0; i < 3; i++) {
+        const int nu = i + (i >= mu ? 1 : 0), w = plane_index(mu, nu), gm = nb_sel(ci, st, nu, -1);
+        const T sign = mu < nu ? T(-1) : T(1);
+        herm8<T> y = transport_dn(U.load(nu, gm), S.load(w, gm));
+        const herm8<T> up = S.load(w, st.g);
+#pragma unroll
+        for (int k = 0; k < 8; k++) sum.h[k] = fmaT(sign, up.h[k] - y.h[k], sum.h[k]);
+    }
+    const herm8<T> q = scaled(sum, (T)ci.rho);
+    Q.store(mu, st.g, q);
+    Uout.store(mu, st.g, mul(expiQ(q), U.load(mu, st.g)));
+}
+
+// Lambda and e^{-i ad_Q} x of the last level's derivative x = X(link)
+template <typename T>
+__global__ void __launch_bounds__(kLinkBlock) k_lambda(DevGeom g, AlgPlanes<T> Q, AlgPlanes<T> X, AlgPlanes<T> Lam,
+                                                       AlgPlanes<T> Dir) {
+    ChainInfo ci;
+    Site st;
+    if (!locate_tile(g, ci, st)) return;
+    const int mu = threadIdx.x >> 5;
+    herm8<T> lam, dir;
+    lambda_adjoint(Q.load(mu, st.g), X.load(mu, st.g), lam, dir);
+    Lam.store(mu, st.g, lam);
+    Dir.store(mu, st.g, dir);
+}
+
+// Chain rule over the plaquettes.  The variation of rho Tr(M S), M = Lambda_d -
+// Lambda_a + D - A with A = a Lambda_b a^dag, D = d Lambda_c d^dag (the plaquette's
+// part of sum Tr(Lambda dQ): Q_a = -rho S, Q_d = rho S, Q_b = -rho a^dag S a,
+// Q_c = rho d^dag S d), with respect to the four links is
+//   y_a = G+ + i [S, A],  y_d = G- - i [S, D],  y_b = a^dag G+ a,  y_c = d^dag G- d,
+//   G+- = +-{C, M} / 2 + i [S, M] / 2,  C = (P + P^dag) / 2.
+// y_a and y_d, summed over the planes through shared memory, go to Loc; y_b and y_c
+// belong to the links (x+p, q) and (x+q, p) and go to the plane fields Rem[3 link + i]
+// at x, i = the plane's other direction counted without the link's own.
+template <typename T, int MINB>
+__global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_chain(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> Lam,
+                                                                 AlgPlanes<T> Loc, AlgPlanes<T> Rem) {
+    constexpr int kPieces = AlgPlanes<T>::kPieces, kPer = AlgPlanes<T>::kPer;
+    __shared__ alg_piece<T> sm[12][kPieces][MAG_TILE];
+    ChainInfo ci;
+    Site st;
+    const bool ok = locate_tile(g, ci, st);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (ok) {
+        int p, q;
+        plane_of(w, p, q);
+        const int gp = nb_sel(ci, st, p, 1), gq = nb_sel(ci, st, q, 1);
+        const int ip = 3 * p + q - 1, iq = 3 * q + p;
+        // this thread's two slots; they hold A and D until y_a and y_d replace them
+        auto put = [&](int i, const herm8<T>& h) {
+#pragma unroll
+            for (int j = 0; j < kPieces; j++)
+#pragma unroll
+                for (int k = 0; k < kPer; k++) sm[i][j][lane].v[k] = h.h[j * kPer + k];
+        };
+        auto get = [&](int i) {
+            herm8<T> h;
+#pragma unroll
+            for (int j = 0; j < kPieces; j++)
+#pragma unroll
+                for (int k = 0; k < kPer; k++) h.h[j * kPer + k] = sm[i][j][lane].v[k];
+            return h;
+        };
+        // a and d are loaded again (L1) for each use instead of staying in registers
+        auto link = [&](int d) {
+            asm volatile("" ::: "memory");
+            return U.load(d, st.g);
+        };
+        const mat3<T> P =
+            plaquette(U.load_rows01(p, st.g), U.load(q, gp), U.load(p, gq), U.load_rows01(q, st.g));
+        const herm8<T> S = plaq_sin(P, (T)ci.rho);
+        const herm9<T> C = plaq_cos(P, (T)ci.rho);
+        herm8<T> M = transport_nd(link(q), Lam.load(p, gq));
+        put(iq, M);
+        {
+            const herm8<T> A = transport_nd(link(p), Lam.load(q, gp));
+            put(ip, A);
+            herm_sub(M, A);
+        }
+        herm_add(M, Lam.load(q, st.g));
+        herm_sub(M, Lam.load(p, st.g));
+        const herm8<T> anti = anticomm_half(C, M);
+        herm8<T> gm = comm_i(S, M);
+#pragma unroll
+        for (int k = 0; k < 8; k++) gm.h[k] *= T(0.5);
+        herm8<T> gpl = gm;
+        herm_add(gpl, anti);
+        herm_sub(gm, anti);
+        asm volatile("" ::: "memory");
+        herm8<T> y = comm_i(S, get(ip));
+        herm_add(y, gpl);
+        put(ip, y);
+        y = gm;
+        herm_sub(y, comm_i(S, get(iq)));
+        put(iq, y);
+        Rem.store(iq, st.g, transport_dn(link(p), gpl));
+        Rem.store(ip, st.g, transport_dn(link(q), gm));
+    }
+    __syncthreads();
+    if (!ok) return;
+    for (int r = w; r < 4 * kPieces; r += 6) {
+        const int mu = r / kPieces, j = r - mu * kPieces;
+        alg_piece<T> a = sm[3 * mu][j][lane];
+        const alg_piece<T> b = sm[3 * mu + 1][j][lane], c = sm[3 * mu + 2][j][lane];
+#pragma unroll
+        for (int k = 0; k < kPer; k++) a.v[k] = (a.v[k] + b.v[k]) + c.v[k];
+        const_cast<alg_piece<T>*>(Loc.at(mu, st.g))[j * MAG_TILE] = a;
+    }
+}
+
+// x = Dir + Loc(x) + sum_nu Rem(x - nu): the derivative with respect to the level's
+// links; then Lambda and Dir of the level below, or (LAST) the force itself
+template <typename T, bool LAST>
+__global__ void __launch_bounds__(kLinkBlock) k_chain_gather(DevGeom g, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
+                                                             AlgPlanes<T> Dir, AlgPlanes<T> Q, AlgPlanes<T> Out) {
+    ChainInfo ci;
+    Site st;
+    if (!locate_tile(g, ci, st)) return;
+    const int mu = threadIdx.x >> 5;
+    herm8<T> x = Dir.load(mu, st.g);
+    herm_add(x, Loc.load(mu, st.g));
+    herm8<T> r[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const int nu = i + (i >= mu ? 1 : 0);
+        r[i] = Rem.load(3 * mu + i, nb_sel(ci, st, nu, -1));
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) herm_add(x, r[i]);
+    if (LAST) {
+        Out.store(mu, st.g, x);
+    } else {
+        herm8<T> lam, dir;
+        lambda_adjoint(Q.load(mu, st.g), x, lam, dir);
+        Out.store(mu, st.g, lam);
+        Dir.store(mu, st.g, dir);
+    }
+}
+
+unsigned tiles(const DevGeom& g) { return (unsigned)(g.vpad / MAG_TILE); }
+
+}  // namespace
+
+template <typename T>
+void launch_stout_level(const DevGeom& g, LinkPlanes<T> U, LinkPlanes<T> Uout, AlgPlanes<T> Q, AlgPlanes<T> S,
+                        cudaStream_t s) {
+    k_plaq_sin<T><<<tiles(g), kPlaqBlock, 0, s>>>(g, U, S);
+    k_stout_apply<T><<<tiles(g), kLinkBlock, 0, s>>>(g, U, S, Uout, Q);
+}
+template <typename T>
+void launch_lambda(const DevGeom& g, AlgPlanes<T> Q, AlgPlanes<T> X, AlgPlanes<T> Lam, AlgPlanes<T> Dir,
+                   cudaStream_t s) {
+    k_lambda<T><<<tiles(g), kLinkBlock, 0, s>>>(g, Q, X, Lam, Dir);
+}
+template <typename T>
+void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
+                       cudaStream_t s) {
+    // blocks of six warps per SM: two of FP64 (168 registers, no spills; three would spill 1 KB:
+    // 1.47 against 0.83 ms at 32^4), three of FP32 (96 registers; 0.369 against 0.431 ms)
+    k_plaq_chain<T, sizeof(T) == 8 ? 2 : 3><<<tiles(g), kPlaqBlock, 0, s>>>(g, U, Lam, Loc, Rem);
+}
+template <typename T>
+void launch_chain_gather(const DevGeom& g, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir, const AlgPlanes<T>* Q,
+                         AlgPlanes<T> Out, cudaStream_t s) {
+    if (Q) k_chain_gather<T, false><<<tiles(g), kLinkBlock, 0, s>>>(g, Loc, Rem, Dir, *Q, Out);
+    else k_chain_gather<T, true><<<tiles(g), kLinkBlock, 0, s>>>(g, Loc, Rem, Dir, AlgPlanes<T>{nullptr, 0}, Out);
+}
+
+#define MAG_INSTANTIATE(T)                                                                                          \
+    template void launch_stout_level<T>(const DevGeom&, LinkPlanes<T>, LinkPlanes<T>, AlgPlanes<T>, AlgPlanes<T>,   \
+                                        cudaStream_t);                                                              \
+    template void launch_lambda<T>(const DevGeom&, AlgPlanes<T>, AlgPlanes<T>, AlgPlanes<T>, AlgPlanes<T>,          \
+                                   cudaStream_t);                                                                   \
+    template void launch_plaq_chain<T>(const DevGeom&, LinkPlanes<T>, AlgPlanes<T>, AlgPlanes<T>, AlgPlanes<T>,     \
+                                       cudaStream_t);                                                               \
+    template void launch_chain_gather<T>(const DevGeom&, AlgPlanes<T>, AlgPlanes<T>, AlgPlanes<T>,                  \
+                                         const AlgPlanes<T>*, AlgPlanes<T>, cudaStream_t);
+MAG_INSTANTIATE(float)
+MAG_INSTANTIATE(double)
+#undef MAG_INSTANTIATE
+
+}  // namespace magb

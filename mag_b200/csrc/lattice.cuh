@@ -8,7 +8,7 @@
 //
 // Field layout (x0 fastest inside a chain, as qlat's index_from_coordinate):
 //   link field   : cplx<T> [4 mu][Vpad / 32 tiles][9 elements][32 sites]
-//   algebra field: T       [4 mu][Vpad / 32 tiles][8 compact ][32 sites]
+//   algebra field: 16 bytes [4 mu][Vpad / 32 tiles][8 reals in 16-byte pieces][32 sites]
 // A warp reads 32 consecutive sites of one element: a 512-byte (double) or
 // 256-byte (float) coalesced transaction per matrix element.
 #pragma once
@@ -254,24 +254,43 @@ struct LinkPlanes<float> {
     }
 };
 
+// Algebra fields: the eight reals travel in 16-byte pieces (pairs of doubles, quadruples
+// of floats), piece j of a tile's 32 links in one row: four (two) 128-bit accesses per
+// element instead of eight 64-bit (32-bit) ones.
+template <typename T>
+struct alignas(16) alg_piece {
+    T v[16 / sizeof(T)];
+};
+
 template <typename T>
 struct AlgPlanes {
+    static constexpr int kPer = 16 / sizeof(T), kPieces = 8 / kPer;
     T* p;
     long vpad;
-    MAG_HD const T* at(int mu, int g) const {
-        return p + (long)mu * 8 * vpad + (long)(g / MAG_TILE) * (8 * MAG_TILE) + (g % MAG_TILE);
+    MAG_HD const alg_piece<T>* at(int mu, int g) const {
+        return reinterpret_cast<const alg_piece<T>*>(p) + (long)mu * kPieces * vpad +
+               (long)(g / MAG_TILE) * (kPieces * MAG_TILE) + (g % MAG_TILE);
     }
     MAG_HD herm8<T> load(int mu, int g) const {
         herm8<T> q;
-        const T* b = at(mu, g);
+        const alg_piece<T>* b = at(mu, g);
 #pragma unroll
-        for (int k = 0; k < 8; k++) q.h[k] = b[k * MAG_TILE];
+        for (int j = 0; j < kPieces; j++) {
+            const alg_piece<T> w = b[j * MAG_TILE];
+#pragma unroll
+            for (int k = 0; k < kPer; k++) q.h[j * kPer + k] = w.v[k];
+        }
         return q;
     }
     MAG_HD void store(int mu, int g, const herm8<T>& q) const {
-        T* b = const_cast<T*>(at(mu, g));
+        alg_piece<T>* b = const_cast<alg_piece<T>*>(at(mu, g));
 #pragma unroll
-        for (int k = 0; k < 8; k++) b[k * MAG_TILE] = q.h[k];
+        for (int j = 0; j < kPieces; j++) {
+            alg_piece<T> w;
+#pragma unroll
+            for (int k = 0; k < kPer; k++) w.v[k] = q.h[j * kPer + k];
+            b[j * MAG_TILE] = w;
+        }
     }
 };
 

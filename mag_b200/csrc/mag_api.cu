@@ -192,14 +192,14 @@ int mag_staple(mag_ctx* ctx, int chain, double* host) {
                                         ctx->var<float>(KF_STOUT_FWD), ctx->stream);
             cur = ctx->st32.lv[k];
         }
-        LinkPlanes<float> z = ctx->p.n_stout ? ctx->st32.za : ctx->Uaux32;
+        LinkPlanes<float> z = ctx->Uaux32;
         if (ctx->iwasaki) launch_double_link<float>(ctx->geom, cur, ctx->W32, ctx->stream);
         launch_staple_dagger<float>(ctx->geom, cur, ctx->W32, z, ctx->iwasaki, ctx->var<float>(KF_STAPLE),
                                     ctx->stream);
         launch_links_to_aos_t<float>(z, ci.off, ci.V, ctx->staging, ctx->stream);
     } else {
         LinkPlanes<double> cur = ctx->smear64();
-        LinkPlanes<double> z = ctx->p.n_stout ? ctx->st64.za : ctx->Uaux;
+        LinkPlanes<double> z = ctx->Uaux;
         if (ctx->iwasaki) launch_double_link<double>(ctx->geom, cur, ctx->W64, ctx->stream);
         launch_staple_dagger<double>(ctx->geom, cur, ctx->W64, z, ctx->iwasaki, ctx->var<double>(KF_STAPLE),
                                      ctx->stream);
@@ -605,8 +605,18 @@ int mag_time_kernel(mag_ctx* ctx, const char* which, int reps, double* ms) {
     if (fam >= KF_STOUT_FWD && L == 0) return fail(MAG_ERR_STATE, "mag_time_kernel: no stout levels in this context");
     MAG_TRY(ctx->ensure_tuned());
     // one full force evaluation first, so every intermediate buffer holds live data
-    if (m) ctx->force_eval<float>(ctx->U32, ctx->F32, ctx->st32);
-    else ctx->force_eval<double>(ctx->U, ctx->F, ctx->st64);
+    if (fam == KF_STAPLE || fam == KF_STOUT_LAMBDA || fam == KF_STOUT_CHAIN) {
+        if (m) {
+            MAG_TRY(ctx->ensure_gather(ctx->st32));
+            ctx->force_eval_gather<float>(ctx->U32, ctx->F32, ctx->st32);
+        } else {
+            MAG_TRY(ctx->ensure_gather(ctx->st64));
+            ctx->force_eval_gather<double>(ctx->U, ctx->F, ctx->st64);
+        }
+    } else {
+        if (m) ctx->force_eval<float>(ctx->U32, ctx->F32, ctx->st32);
+        else ctx->force_eval<double>(ctx->U, ctx->F, ctx->st64);
+    }
     if (fam >= 0) {
         const KernelFamily f = (KernelFamily)fam;
         if (m) return ctx->time_one<float>(f, ctx->var<float>(f), reps, ctx->st32, ctx->U32, ctx->F32, ctx->Uaux32, ms);
@@ -640,6 +650,12 @@ int mag_time_kernel(mag_ctx* ctx, const char* which, int reps, double* ms) {
         } else {
             return fail(MAG_ERR_ARG, "mag_time_kernel: unknown kernel '" + w + "'");
         }
+    } else if (w == "lambda" || w == "plaq_chain" || w == "chain_gather") {
+        if (L == 0) return fail(MAG_ERR_STATE, "mag_time_kernel: no stout levels in this context");
+        fn = [&]() {
+            if (m) ctx->launch_smear<float>(w, ctx->st32, ctx->U32, ctx->F32);
+            else ctx->launch_smear<double>(w, ctx->st64, ctx->U, ctx->F);
+        };
     } else if (w == "evolve") {
         fn = [&]() {
             launch_evolve<double, double>(g, ctx->U, ctx->Ubak, ctx->P, 1e-3,
@@ -717,6 +733,13 @@ int mag_set_kernel_variant(mag_ctx* ctx, const char* family, int precision, cons
     if (v < 0 || v >= mag_ctx::variants_of((KernelFamily)f))
         return fail(MAG_ERR_ARG, std::string("mag_set_kernel_variant: no variant '") + variant + "' for " + family);
     MAG_TRY(ctx->ensure_tuned());
+    if (f == KF_STAPLE || f == KF_STOUT_LAMBDA || f == KF_STOUT_CHAIN) {  // kernels of the one-thread-per-link form
+        if ((precision == 1) == ctx->mixed) {
+            if (ctx->mixed) MAG_TRY(ctx->ensure_gather(ctx->st32));
+            else MAG_TRY(ctx->ensure_gather(ctx->st64));
+            ctx->gather[precision] = true;
+        }
+    }
     ctx->tune[f][precision] = v;
     if (ctx->graph) {  // the captured trajectory holds the previous choice
         cudaGraphExecDestroy(ctx->graph);
