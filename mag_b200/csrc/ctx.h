@@ -247,6 +247,8 @@ struct mag_ctx {
         if (backward && p.n_stout > 0) {
             MAG_TRY(alloc_alg(b.lam));
             MAG_TRY(alloc_alg(b.dir));
+        }
+        if (backward) {
             MAG_TRY(alloc_alg(b.loc));
             MAG_TRY(alloc_alg(b.rem, 12));
         }
@@ -421,26 +423,34 @@ struct mag_ctx {
     template <typename T>
     void force_eval(LinkPlanes<T> Uin, AlgPlanes<T> Fout, StoutBufs<T>& b) {
         if (gather[sizeof(T) == 8 ? 0 : 1]) return force_eval_gather(Uin, Fout, b);
+        const int L = p.n_stout;
         hx(Uin);
         LinkPlanes<T> cur = Uin;
-        for (int k = 0; k < p.n_stout; k++) {
+        for (int k = 0; k < L; k++) {
             launch_stout_forward<T>(geom, cur, b.lv[k], b.Q[k], var<T>(KF_STOUT_FWD), stream);
             cur = b.lv[k];
             hx(cur);
         }
+        const AlgPlanes<T>* qtop = L ? &b.Q[L - 1] : nullptr;
         if (iwasaki) {
-            launch_double_link<T>(geom, cur, wbuf<T>(), stream);
-            hx(wbuf<T>());
+            launch_plaq_rect<T>(geom, cur, plaq_buf<T>(), b.loc, b.rem, stream);
+            launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, true, qtop, L ? b.lam : Fout, stream);
+        } else {
+            launch_wilson_force<T>(geom, cur, b.rem, Fout, stream);
+            if (L) launch_lambda<T>(geom, *qtop, Fout, b.lam, b.dir, stream);
         }
-        launch_force<T>(geom, cur, wbuf<T>(), Fout, iwasaki, var<T>(KF_FORCE), stream);
-        if (p.n_stout > 0) launch_lambda<T>(geom, b.Q[p.n_stout - 1], Fout, b.lam, b.dir, stream);
-        for (int k = p.n_stout - 1; k >= 0; k--) {
+        for (int k = L - 1; k >= 0; k--) {
             hx(b.lam);
             launch_plaq_chain<T>(geom, k == 0 ? Uin : b.lv[k - 1], b.lam, b.loc, b.rem, stream);
-            if (k == 0) launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, nullptr, Fout, stream);
-            else launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, &b.Q[k - 1], b.lam, stream);
+            launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, false, k ? &b.Q[k - 1] : nullptr, k ? b.lam : Fout,
+                                   stream);
         }
         if (any_mag) launch_constraint_fixup<T>(geom, Uin, Fout, stream);
+    }
+    // the plaquettes' rows share the double links' buffer (576 of 576 bytes per site in FP64, 288 of 320 in FP32)
+    template <typename T>
+    RowPlanes<T> plaq_buf() const {
+        return RowPlanes<T>{reinterpret_cast<T*>(wbuf<T>().p), vpad};
     }
 
     // The force by the one-thread-per-link kernels with matrix derivatives, whose launch
@@ -516,9 +526,12 @@ struct mag_ctx {
     // one launch of a kernel of the derivative's plaquette form, on the thin links
     template <typename T>
     void launch_smear(const std::string& w, StoutBufs<T>& b, LinkPlanes<T> Uin, AlgPlanes<T> Fo) {
-        if (w == "lambda") launch_lambda<T>(geom, b.Q[0], Fo, b.lam, b.dir, stream);
+        if (w == "stout_level") launch_stout_level<T>(geom, Uin, b.lv[0], b.Q[0], b.rem, stream);
+        else if (w == "lambda") launch_lambda<T>(geom, b.Q[0], Fo, b.lam, b.dir, stream);
         else if (w == "plaq_chain") launch_plaq_chain<T>(geom, Uin, b.lam, b.loc, b.rem, stream);
-        else launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, &b.Q[0], b.lam, stream);
+        else if (w == "chain_gather") launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, false, &b.Q[0], b.lam, stream);
+        else if (iwasaki) launch_plaq_rect<T>(geom, Uin, plaq_buf<T>(), b.loc, b.rem, stream);
+        else launch_wilson_force<T>(geom, Uin, b.rem, Fo, stream);
     }
 
     template <typename T>
@@ -542,9 +555,12 @@ struct mag_ctx {
     int tune_precision(int reps, StoutBufs<T>& b, LinkPlanes<T> Uin, AlgPlanes<T> Fo, LinkPlanes<T> zs) {
         force_eval<T>(Uin, Fo, b);
         std::vector<KernelFamily> fams;
-        if (p.n_stout == 0) fams = {KF_FORCE};
-        else if (gather[sizeof(T) == 8 ? 0 : 1]) fams = {KF_STAPLE, KF_STOUT_FWD, KF_STOUT_LAMBDA, KF_STOUT_CHAIN};
-        else fams = {KF_FORCE, KF_STOUT_FWD};
+        if (gather[sizeof(T) == 8 ? 0 : 1]) {
+            if (p.n_stout == 0) fams = {KF_FORCE};
+            else fams = {KF_STAPLE, KF_STOUT_FWD, KF_STOUT_LAMBDA, KF_STOUT_CHAIN};
+        } else if (p.n_stout > 0) {
+            fams = {KF_STOUT_FWD};
+        }
         // Every variant is timed (the report shows them all), but the choice is made among the
         // one-thread-per-link register caps only: those compute bit-identical results, so a run does not
         // depend on timing noise.  The direction-split shapes add their parts in another order (results
@@ -623,7 +639,7 @@ struct mag_ctx {
         } else {
             MAG_TRY(tune_precision<double>(reps, st64, U, F, Uaux));
         }
-        if (!halo) {
+        if (!halo && gather[mixed ? 1 : 0]) {
             if (mixed) MAG_TRY(tune_order<float>(reps, st32, U32, F32));
             else MAG_TRY(tune_order<double>(reps, st64, U, F));
         }

@@ -111,11 +111,19 @@ void launch_lambda(const DevGeom& g, AlgPlanes<T> Q, AlgPlanes<T> X, AlgPlanes<T
 template <typename T>
 void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
                        cudaStream_t s);
-// x = Dir + Loc + the Rem terms that belong to a link: Out = Lambda and Dir of the level below with
-// exponents *Q, or Out = x itself when Q is null (the thin links)
+// x = Dir + Loc + the Rem terms that belong to a link (top: without Dir, times beta/3): Out = Lambda and Dir of the
+// level below with exponents *Q, or Out = x itself when Q is null (the thin links)
 template <typename T>
-void launch_chain_gather(const DevGeom& g, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir, const AlgPlanes<T>* Q,
-                         AlgPlanes<T> Out, cudaStream_t s);
+void launch_chain_gather(const DevGeom& g, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir, bool top,
+                         const AlgPlanes<T>* Q, AlgPlanes<T> Out, cudaStream_t s);
+// the plaquettes of U into Pl, then the Iwasaki force's plaquette and rectangle terms (without beta/3)
+// into Loc and Rem as launch_plaq_chain leaves them
+template <typename T>
+void launch_plaq_rect(const DevGeom& g, LinkPlanes<T> U, RowPlanes<T> Pl, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
+                      cudaStream_t s);
+// the Wilson force of U
+template <typename T>
+void launch_wilson_force(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> S, AlgPlanes<T> F, cudaStream_t s);
 
 // ---- streaming kernels (kernels_update.cu)
 template <typename TU, typename TX>

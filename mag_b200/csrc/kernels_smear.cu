@@ -42,6 +42,40 @@ __device__ __forceinline__ bool locate_tile(const DevGeom& g, ChainInfo& ci, Sit
     return true;
 }
 
+// The twelve (link, plane) terms of the tile's links that start at its own sites:
+// slot 3 mu + i for the link in direction mu and its i-th other direction.  A thread
+// writes the two slots of its plane; the block adds the three slots of each link.
+template <typename T>
+struct site_terms {
+    static constexpr int kPieces = AlgPlanes<T>::kPieces, kPer = AlgPlanes<T>::kPer;
+    alg_piece<T> v[12][kPieces][MAG_TILE];
+    __device__ __forceinline__ void put(int i, int lane, const herm8<T>& h) {
+#pragma unroll
+        for (int j = 0; j < kPieces; j++)
+#pragma unroll
+            for (int k = 0; k < kPer; k++) v[i][j][lane].v[k] = h.h[j * kPer + k];
+    }
+    __device__ __forceinline__ herm8<T> get(int i, int lane) const {
+        herm8<T> h;
+#pragma unroll
+        for (int j = 0; j < kPieces; j++)
+#pragma unroll
+            for (int k = 0; k < kPer; k++) h.h[j * kPer + k] = v[i][j][lane].v[k];
+        return h;
+    }
+    // after a barrier: the sums of the four links, shared out over the six warps
+    __device__ __forceinline__ void sum_links(const AlgPlanes<T>& Loc, int g, int w, int lane) const {
+        for (int r = w; r < 4 * kPieces; r += 6) {
+            const int mu = r / kPieces, j = r - mu * kPieces;
+            alg_piece<T> a = v[3 * mu][j][lane];
+            const alg_piece<T> b = v[3 * mu + 1][j][lane], c = v[3 * mu + 2][j][lane];
+#pragma unroll
+            for (int k = 0; k < kPer; k++) a.v[k] = (a.v[k] + b.v[k]) + c.v[k];
+            const_cast<alg_piece<T>*>(Loc.at(mu, g))[j * MAG_TILE] = a;
+        }
+    }
+};
+
 // S = (P - P^dag) / 2i of every plaquette (plane fields 0..5 of S)
 template <typename T>
 __global__ void __launch_bounds__(kPlaqBlock) k_plaq_sin(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S) {
@@ -57,7 +91,24 @@ __global__ void __launch_bounds__(kPlaqBlock) k_plaq_sin(DevGeom g, LinkPlanes<T
     S.store(w, st.g, plaq_sin(P, T(1)));
 }
 
-// Q = -i rho TA(stp U^dag) (field-multi.h:32-39) from the plaquettes at x and x - nu, U' = e^{iQ} U
+// -i TA(stp U^dag) of link (x, mu), stp its six staples, from the plaquettes at x and x - nu
+template <typename T>
+__device__ __forceinline__ herm8<T> staple_angle(const LinkPlanes<T>& U, const AlgPlanes<T>& S, const ChainInfo& ci,
+                                                 const Site& st, int mu) {
+    herm8<T> sum = herm_zero<T>();
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const int nu = i + (i >= mu ? 1 : 0), w = plane_index(mu, nu), gm = nb_sel(ci, st, nu, -1);
+        const T sign = mu < nu ? T(-1) : T(1);
+        const herm8<T> y = transport_dn(U.load(nu, gm), S.load(w, gm));
+        const herm8<T> up = S.load(w, st.g);
+#pragma unroll
+        for (int k = 0; k < 8; k++) sum.h[k] = fmaT(sign, up.h[k] - y.h[k], sum.h[k]);
+    }
+    return sum;
+}
+
+// Q = -i rho TA(stp U^dag) (field-multi.h:32-39), U' = e^{iQ} U
 template <typename T>
 __global__ void __launch_bounds__(kLinkBlock) k_stout_apply(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S,
                                                             LinkPlanes<T> Uout, AlgPlanes<T> Q) {
@@ -65,19 +116,120 @@ __global__ void __launch_bounds__(kLinkBlock) k_stout_apply(DevGeom g, LinkPlane
     Site st;
     if (!locate_tile(g, ci, st)) return;
     const int mu = threadIdx.x >> 5;
-    herm8<T> sum = herm_zero<T>();
-#pragma unroll 1
-    for (int i = 0; i < 3; i++) {
-        const int nu = i + (i >= mu ? 1 : 0), w = plane_index(mu, nu), gm = nb_sel(ci, st, nu, -1);
-        const T sign = mu < nu ? T(-1) : T(1);
-        herm8<T> y = transport_dn(U.load(nu, gm), S.load(w, gm));
-        const herm8<T> up = S.load(w, st.g);
-#pragma unroll
-        for (int k = 0; k < 8; k++) sum.h[k] = fmaT(sign, up.h[k] - y.h[k], sum.h[k]);
-    }
-    const herm8<T> q = scaled(sum, (T)ci.rho);
+    const herm8<T> q = scaled(staple_angle(U, S, ci, st, mu), (T)ci.rho);
     Q.store(mu, st.g, q);
     Uout.store(mu, st.g, mul(expiQ(q), U.load(mu, st.g)));
+}
+
+// Wilson force F = i beta/3 TA(U A^dag), A the plaquette staples (field-hmc.h:394-421)
+template <typename T>
+__global__ void __launch_bounds__(kLinkBlock) k_wilson_force(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S,
+                                                             AlgPlanes<T> F) {
+    ChainInfo ci;
+    Site st;
+    if (!locate_tile(g, ci, st)) return;
+    const int mu = threadIdx.x >> 5;
+    F.store(mu, st.g, scaled(staple_angle(U, S, ci, st, mu), (T)(ci.beta / 3.0)));
+}
+
+// rows 0, 1 of every plaquette (plane fields 0..5 of Pl)
+template <typename T>
+__global__ void __launch_bounds__(kPlaqBlock, sizeof(T) == 8 ? 2 : 4) k_plaq(DevGeom g, LinkPlanes<T> U, RowPlanes<T> Pl) {
+    ChainInfo ci;
+    Site st;
+    if (!locate_tile(g, ci, st)) return;
+    const int w = threadIdx.x >> 5;
+    int p, q;
+    plane_of(w, p, q);
+    const mat3<T> x = mul_2r(U.load_rows01(p, st.g), U.load(q, nb_sel(ci, st, p, 1)));
+    const mat3<T> y = mul_su3(U.load_rows01(q, st.g), U.load(p, nb_sel(ci, st, q, 1)));
+    Pl.store(w, st.g, mul_nd_2r(x, y));
+}
+
+// Iwasaki force i TA(U A^dag) without its beta/3, A = c0 staples + c1 rectangles
+// (field-hmc.h:142-198, 226-269), as the loops through each plaquette P: the 1x2
+// rectangles that contain P are its products with the plaquette across each of its
+// four sides,
+//   A P,  A = a P(x+p) a^dag           (b is not on it)
+//   P B,  B = a-^dag P(x-p) a-,  a- = U_p(x-p)  (d is not on it)
+//   P D,  D = d P(x+q) d^dag           (c is not on it)
+//   E P,  E = d-^dag P(x-q) d-,  d- = U_q(x-q)  (a is not on it).
+// A link's term is the (L - L^dag) / 2i of its loops, moved to the link's start along
+// the loop: b's start along a (E P, which does not hold a, is P E there) and c's along
+// d (P B is B P), P E = P (E P) P^dag and B P = P^dag (P B) P.  With R the weighted
+// (L - L^dag) / 2i of the four products and R0 that of P
+//   a: -(R0 + RA + RB + RD),                  d: R0 + RA + RD + RE,
+//   b: -a^dag (R0 + RB + RD + P RE P^dag) a,  c: d^dag (R0 + RA + RE + P^dag RB P) d.
+// Every rectangle is formed twice (from each of its plaquettes) instead of six times,
+// from nine matrices read instead of 24 per direction.  Loc and Rem as in k_plaq_chain.
+template <typename T, int MINB>
+__global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_rect(DevGeom g, LinkPlanes<T> U, RowPlanes<T> Pl,
+                                                                AlgPlanes<T> Loc, AlgPlanes<T> Rem) {
+    __shared__ site_terms<T> sm;
+    ChainInfo ci;
+    Site st;
+    const bool ok = locate_tile(g, ci, st);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (ok) {
+        int p, q;
+        plane_of(w, p, q);
+        const int ip = 3 * p + q - 1, iq = 3 * q + p;
+        const T k0 = (T)ci.c0, k1 = (T)ci.c1;
+        // operands are loaded again for each use (L1) instead of staying in registers
+        auto fresh = []() { asm volatile("" ::: "memory"); };
+        herm8<T> lb, lc, t;
+        {
+            const int gm = nb_sel(ci, st, q, -1);
+            mat3<T> x = mul_dn_2r(U.load_cols01(q, gm), Pl.load(w, gm));
+            x = mul_2r(x, U.load(q, gm));
+            const mat3<T> P = Pl.load(w, st.g);
+            lc = plaq_sin(mul_su3(x, P), k1);  // RE
+            sm.put(iq, lane, lc);
+            lb = transport_nd(P, lc);
+            t = plaq_sin(P, k0);  // R0
+        }
+        fresh();
+        {
+            const int gm = nb_sel(ci, st, p, -1);
+            mat3<T> x = mul_nd_2r(Pl.load_rows01(w, st.g), U.load(p, gm));
+            x = mul_2r(x, Pl.load(w, gm));
+            const herm8<T> r = plaq_sin(mul_su3(x, U.load(p, gm)), k1);  // RB
+            sm.put(ip, lane, r);
+            herm_add(lb, r);
+            herm_add(lc, transport_dn(Pl.load(w, st.g), r));
+        }
+        herm_add(lb, t);
+        herm_add(lc, t);
+        fresh();
+        {
+            mat3<T> x = mul_2r(U.load_rows01(p, st.g), Pl.load(w, nb_sel(ci, st, p, 1)));
+            x = mul_nd_2r(x, U.load(p, st.g));
+            const herm8<T> r = plaq_sin(mul_su3(x, Pl.load(w, st.g)), k1);  // RA
+            herm_add(lc, r);
+            herm_add(t, r);
+        }
+        fresh();
+        Rem.store(ip, st.g, transport_dn(U.load(q, st.g), lc));
+        {
+            mat3<T> x = mul_2r(Pl.load_rows01(w, st.g), U.load(q, st.g));
+            x = mul_2r(x, Pl.load(w, nb_sel(ci, st, q, 1)));
+            const herm8<T> r = plaq_sin(mul_nd_su3(x, U.load(q, st.g)), k1);  // RD
+            herm_add(lb, r);
+            herm_add(t, r);
+        }
+        fresh();
+#pragma unroll
+        for (int k = 0; k < 8; k++) lb.h[k] = -lb.h[k];
+        Rem.store(iq, st.g, transport_dn(U.load(p, st.g), lb));
+        herm8<T> y = sm.get(ip, lane);
+#pragma unroll
+        for (int k = 0; k < 8; k++) y.h[k] = -t.h[k] - y.h[k];
+        sm.put(ip, lane, y);
+        herm_add(t, sm.get(iq, lane));
+        sm.put(iq, lane, t);
+    }
+    __syncthreads();
+    if (ok) sm.sum_links(Loc, st.g, w, lane);
 }
 
 // Lambda and e^{-i ad_Q} x of the last level's derivative x = X(link)
@@ -106,8 +258,7 @@ __global__ void __launch_bounds__(kLinkBlock) k_lambda(DevGeom g, AlgPlanes<T> Q
 template <typename T, int MINB>
 __global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_chain(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> Lam,
                                                                  AlgPlanes<T> Loc, AlgPlanes<T> Rem) {
-    constexpr int kPieces = AlgPlanes<T>::kPieces, kPer = AlgPlanes<T>::kPer;
-    __shared__ alg_piece<T> sm[12][kPieces][MAG_TILE];
+    __shared__ site_terms<T> sm;
     ChainInfo ci;
     Site st;
     const bool ok = locate_tile(g, ci, st);
@@ -117,21 +268,7 @@ __global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_chain(DevGeom g, Link
         plane_of(w, p, q);
         const int gp = nb_sel(ci, st, p, 1), gq = nb_sel(ci, st, q, 1);
         const int ip = 3 * p + q - 1, iq = 3 * q + p;
-        // this thread's two slots; they hold A and D until y_a and y_d replace them
-        auto put = [&](int i, const herm8<T>& h) {
-#pragma unroll
-            for (int j = 0; j < kPieces; j++)
-#pragma unroll
-                for (int k = 0; k < kPer; k++) sm[i][j][lane].v[k] = h.h[j * kPer + k];
-        };
-        auto get = [&](int i) {
-            herm8<T> h;
-#pragma unroll
-            for (int j = 0; j < kPieces; j++)
-#pragma unroll
-                for (int k = 0; k < kPer; k++) h.h[j * kPer + k] = sm[i][j][lane].v[k];
-            return h;
-        };
+        // the thread's two slots hold A and D until y_a and y_d replace them
         // a and d are loaded again (L1) for each use instead of staying in registers
         auto link = [&](int d) {
             asm volatile("" ::: "memory");
@@ -142,10 +279,10 @@ __global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_chain(DevGeom g, Link
         const herm8<T> S = plaq_sin(P, (T)ci.rho);
         const herm9<T> C = plaq_cos(P, (T)ci.rho);
         herm8<T> M = transport_nd(link(q), Lam.load(p, gq));
-        put(iq, M);
+        sm.put(iq, lane, M);
         {
             const herm8<T> A = transport_nd(link(p), Lam.load(q, gp));
-            put(ip, A);
+            sm.put(ip, lane, A);
             herm_sub(M, A);
         }
         herm_add(M, Lam.load(q, st.g));
@@ -158,38 +295,31 @@ __global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_chain(DevGeom g, Link
         herm_add(gpl, anti);
         herm_sub(gm, anti);
         asm volatile("" ::: "memory");
-        herm8<T> y = comm_i(S, get(ip));
+        herm8<T> y = comm_i(S, sm.get(ip, lane));
         herm_add(y, gpl);
-        put(ip, y);
+        sm.put(ip, lane, y);
         y = gm;
-        herm_sub(y, comm_i(S, get(iq)));
-        put(iq, y);
+        herm_sub(y, comm_i(S, sm.get(iq, lane)));
+        sm.put(iq, lane, y);
         Rem.store(iq, st.g, transport_dn(link(p), gpl));
         Rem.store(ip, st.g, transport_dn(link(q), gm));
     }
     __syncthreads();
-    if (!ok) return;
-    for (int r = w; r < 4 * kPieces; r += 6) {
-        const int mu = r / kPieces, j = r - mu * kPieces;
-        alg_piece<T> a = sm[3 * mu][j][lane];
-        const alg_piece<T> b = sm[3 * mu + 1][j][lane], c = sm[3 * mu + 2][j][lane];
-#pragma unroll
-        for (int k = 0; k < kPer; k++) a.v[k] = (a.v[k] + b.v[k]) + c.v[k];
-        const_cast<alg_piece<T>*>(Loc.at(mu, st.g))[j * MAG_TILE] = a;
-    }
+    if (ok) sm.sum_links(Loc, st.g, w, lane);
 }
 
-// x = Dir + Loc(x) + sum_nu Rem(x - nu): the derivative with respect to the level's
-// links; then Lambda and Dir of the level below, or (LAST) the force itself
-template <typename T, bool LAST>
+// x = Loc(x) + sum_nu Rem(x - nu), and Dir unless TOP: the derivative with respect to
+// a level's links (TOP: the gauge force of the top links, beta/3 times the sum); then Lambda and Dir of the
+// level below, or (LAST) the force itself
+template <typename T, bool TOP, bool LAST>
 __global__ void __launch_bounds__(kLinkBlock) k_chain_gather(DevGeom g, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
                                                              AlgPlanes<T> Dir, AlgPlanes<T> Q, AlgPlanes<T> Out) {
     ChainInfo ci;
     Site st;
     if (!locate_tile(g, ci, st)) return;
     const int mu = threadIdx.x >> 5;
-    herm8<T> x = Dir.load(mu, st.g);
-    herm_add(x, Loc.load(mu, st.g));
+    herm8<T> x = Loc.load(mu, st.g);
+    if (!TOP) herm_add(x, Dir.load(mu, st.g));
     herm8<T> r[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) {
@@ -198,6 +328,7 @@ __global__ void __launch_bounds__(kLinkBlock) k_chain_gather(DevGeom g, AlgPlane
     }
 #pragma unroll
     for (int i = 0; i < 3; i++) herm_add(x, r[i]);
+    if (TOP) x = scaled(x, (T)(ci.beta / 3.0));
     if (LAST) {
         Out.store(mu, st.g, x);
     } else {
@@ -231,10 +362,28 @@ void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgP
     k_plaq_chain<T, sizeof(T) == 8 ? 2 : 3><<<tiles(g), kPlaqBlock, 0, s>>>(g, U, Lam, Loc, Rem);
 }
 template <typename T>
-void launch_chain_gather(const DevGeom& g, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir, const AlgPlanes<T>* Q,
-                         AlgPlanes<T> Out, cudaStream_t s) {
-    if (Q) k_chain_gather<T, false><<<tiles(g), kLinkBlock, 0, s>>>(g, Loc, Rem, Dir, *Q, Out);
-    else k_chain_gather<T, true><<<tiles(g), kLinkBlock, 0, s>>>(g, Loc, Rem, Dir, AlgPlanes<T>{nullptr, 0}, Out);
+void launch_chain_gather(const DevGeom& g, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir, bool top,
+                         const AlgPlanes<T>* Q, AlgPlanes<T> Out, cudaStream_t s) {
+    const AlgPlanes<T> q = Q ? *Q : AlgPlanes<T>{nullptr, 0};
+#define L_(TOP, LAST) k_chain_gather<T, TOP, LAST><<<tiles(g), kLinkBlock, 0, s>>>(g, Loc, Rem, Dir, q, Out)
+    if (top && Q) L_(true, false);
+    else if (top) L_(true, true);
+    else if (Q) L_(false, false);
+    else L_(false, true);
+#undef L_
+}
+template <typename T>
+void launch_plaq_rect(const DevGeom& g, LinkPlanes<T> U, RowPlanes<T> Pl, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
+                      cudaStream_t s) {
+    k_plaq<T><<<tiles(g), kPlaqBlock, 0, s>>>(g, U, Pl);
+    // two blocks of six warps per SM in both precisions (three: 0.81 against 0.75 ms FP32 at 32^4,
+    // twice as slow in FP64, from spills)
+    k_plaq_rect<T, 2><<<tiles(g), kPlaqBlock, 0, s>>>(g, U, Pl, Loc, Rem);
+}
+template <typename T>
+void launch_wilson_force(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> S, AlgPlanes<T> F, cudaStream_t s) {
+    k_plaq_sin<T><<<tiles(g), kPlaqBlock, 0, s>>>(g, U, S);
+    k_wilson_force<T><<<tiles(g), kLinkBlock, 0, s>>>(g, U, S, F);
 }
 
 #define MAG_INSTANTIATE(T)                                                                                          \
@@ -244,8 +393,11 @@ void launch_chain_gather(const DevGeom& g, AlgPlanes<T> Loc, AlgPlanes<T> Rem, A
                                    cudaStream_t);                                                                   \
     template void launch_plaq_chain<T>(const DevGeom&, LinkPlanes<T>, AlgPlanes<T>, AlgPlanes<T>, AlgPlanes<T>,     \
                                        cudaStream_t);                                                               \
-    template void launch_chain_gather<T>(const DevGeom&, AlgPlanes<T>, AlgPlanes<T>, AlgPlanes<T>,                  \
-                                         const AlgPlanes<T>*, AlgPlanes<T>, cudaStream_t);
+    template void launch_chain_gather<T>(const DevGeom&, AlgPlanes<T>, AlgPlanes<T>, AlgPlanes<T>, bool,            \
+                                         const AlgPlanes<T>*, AlgPlanes<T>, cudaStream_t);                          \
+    template void launch_plaq_rect<T>(const DevGeom&, LinkPlanes<T>, RowPlanes<T>, AlgPlanes<T>, AlgPlanes<T>,      \
+                                      cudaStream_t);                                                                \
+    template void launch_wilson_force<T>(const DevGeom&, LinkPlanes<T>, AlgPlanes<T>, AlgPlanes<T>, cudaStream_t);
 MAG_INSTANTIATE(float)
 MAG_INSTANTIATE(double)
 #undef MAG_INSTANTIATE

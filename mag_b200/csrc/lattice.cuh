@@ -254,6 +254,48 @@ struct LinkPlanes<float> {
     }
 };
 
+// Fields of special unitary matrices kept as their first two rows (the third is
+// reconstructed on load): six complex elements in 16-byte pieces.
+template <typename T>
+struct RowPlanes {
+    static constexpr int kPer = 16 / (2 * sizeof(T)), kPieces = 6 / kPer;
+    struct alignas(16) piece {
+        cplx<T> v[kPer];
+    };
+    T* p;
+    long vpad;
+    MAG_HD const piece* at(int w, int g) const {
+        return reinterpret_cast<const piece*>(p) + (long)w * kPieces * vpad +
+               (long)(g / MAG_TILE) * (kPieces * MAG_TILE) + (g % MAG_TILE);
+    }
+    MAG_HD mat3<T> load_rows01(int w, int g) const {
+        mat3<T> m;
+        const piece* b = at(w, g);
+#pragma unroll
+        for (int j = 0; j < kPieces; j++) {
+            const piece x = b[j * MAG_TILE];
+#pragma unroll
+            for (int k = 0; k < kPer; k++) m.e[(j * kPer + k) / 3][(j * kPer + k) % 3] = x.v[k];
+        }
+        return m;
+    }
+    MAG_HD mat3<T> load(int w, int g) const {
+        mat3<T> m = load_rows01(w, g);
+        reconstruct_row2(m);
+        return m;
+    }
+    MAG_HD void store(int w, int g, const mat3<T>& m) const {
+        piece* b = const_cast<piece*>(at(w, g));
+#pragma unroll
+        for (int j = 0; j < kPieces; j++) {
+            piece x;
+#pragma unroll
+            for (int k = 0; k < kPer; k++) x.v[k] = m.e[(j * kPer + k) / 3][(j * kPer + k) % 3];
+            b[j * MAG_TILE] = x;
+        }
+    }
+};
+
 // Algebra fields: the eight reals travel in 16-byte pieces (pairs of doubles, quadruples
 // of floats), piece j of a tile's 32 links in one row: four (two) 128-bit accesses per
 // element instead of eight 64-bit (32-bit) ones.

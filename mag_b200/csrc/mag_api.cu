@@ -605,7 +605,7 @@ int mag_time_kernel(mag_ctx* ctx, const char* which, int reps, double* ms) {
     if (fam >= KF_STOUT_FWD && L == 0) return fail(MAG_ERR_STATE, "mag_time_kernel: no stout levels in this context");
     MAG_TRY(ctx->ensure_tuned());
     // one full force evaluation first, so every intermediate buffer holds live data
-    if (fam == KF_STAPLE || fam == KF_STOUT_LAMBDA || fam == KF_STOUT_CHAIN) {
+    if (fam == KF_FORCE || fam == KF_STAPLE || fam == KF_STOUT_LAMBDA || fam == KF_STOUT_CHAIN) {
         if (m) {
             MAG_TRY(ctx->ensure_gather(ctx->st32));
             ctx->force_eval_gather<float>(ctx->U32, ctx->F32, ctx->st32);
@@ -650,8 +650,9 @@ int mag_time_kernel(mag_ctx* ctx, const char* which, int reps, double* ms) {
         } else {
             return fail(MAG_ERR_ARG, "mag_time_kernel: unknown kernel '" + w + "'");
         }
-    } else if (w == "lambda" || w == "plaq_chain" || w == "chain_gather") {
-        if (L == 0) return fail(MAG_ERR_STATE, "mag_time_kernel: no stout levels in this context");
+    } else if (w == "stout_level" || w == "lambda" || w == "plaq_chain" || w == "chain_gather" ||
+               w == "plaq_force") {
+        if (L == 0 && w != "plaq_force") return fail(MAG_ERR_STATE, "mag_time_kernel: no stout levels in this context");
         fn = [&]() {
             if (m) ctx->launch_smear<float>(w, ctx->st32, ctx->U32, ctx->F32);
             else ctx->launch_smear<double>(w, ctx->st64, ctx->U, ctx->F);
@@ -733,7 +734,7 @@ int mag_set_kernel_variant(mag_ctx* ctx, const char* family, int precision, cons
     if (v < 0 || v >= mag_ctx::variants_of((KernelFamily)f))
         return fail(MAG_ERR_ARG, std::string("mag_set_kernel_variant: no variant '") + variant + "' for " + family);
     MAG_TRY(ctx->ensure_tuned());
-    if (f == KF_STAPLE || f == KF_STOUT_LAMBDA || f == KF_STOUT_CHAIN) {  // kernels of the one-thread-per-link form
+    if (f != KF_STOUT_FWD) {  // kernels of the one-thread-per-link form
         if ((precision == 1) == ctx->mixed) {
             if (ctx->mixed) MAG_TRY(ctx->ensure_gather(ctx->st32));
             else MAG_TRY(ctx->ensure_gather(ctx->st64));

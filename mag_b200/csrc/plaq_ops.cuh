@@ -21,6 +21,14 @@
 
 namespace magb {
 
+// x / 3, the product with the rounded 1/3 corrected by its remainder (FP32's 1/3 is
+// 3e-8 off, always to the same side)
+template <typename T>
+MAG_HD T third(T x) {
+    const T t = x * T(1.0 / 3.0);
+    return fmaT(fmaT(T(-3), t, x), T(1.0 / 3.0), t);
+}
+
 // i [A, B] of Hermitian traceless matrices (Hermitian traceless)
 template <typename T>
 MAG_HD herm8<T> comm_i(const herm8<T>& A, const herm8<T>& B) {
@@ -80,7 +88,7 @@ MAG_HD herm8<T> anticomm_half(const herm9<T>& C, const herm8<T>& M) {
     const T r02 = fmaT(z[2], M.h[4], z[3] * M.h[5]);
     const T r12 = fmaT(z[4], M.h[6], z[5] * M.h[7]);
     const T d0 = fmaT(c0, M.h[0], r01 + r02), d1 = fmaT(c1, M.h[1], r01 + r12), d2 = fmaT(c2, m2, r02 + r12);
-    const T t = (d0 + d1 + d2) * T(1.0 / 3.0);
+    const T t = third(d0 + d1 + d2);
     herm8<T> r;
     r.h[0] = d0 - t;
     r.h[1] = d1 - t;
@@ -209,7 +217,7 @@ MAG_HD void herm_sub(herm8<T>& r, const herm8<T>& y) {
 // Hermitian traceless part of (P - P^dag) / 2i, times s
 template <typename T>
 MAG_HD herm8<T> plaq_sin(const mat3<T>& P, T s) {
-    const T t = (P.e[0][0].im + P.e[1][1].im + P.e[2][2].im) * T(1.0 / 3.0), h = T(0.5) * s;
+    const T t = third(P.e[0][0].im + P.e[1][1].im + P.e[2][2].im), h = T(0.5) * s;
     herm8<T> r;
     r.h[0] = s * (P.e[0][0].im - t);
     r.h[1] = s * (P.e[1][1].im - t);
