@@ -244,13 +244,20 @@ struct mag_ctx {
             MAG_TRY(alloc_links(b.lv[k]));
             MAG_TRY(alloc_alg(b.Q[k]));
         }
-        if (backward && p.n_stout > 0) {
-            MAG_TRY(alloc_alg(b.lam));
-            MAG_TRY(alloc_alg(b.dir));
-        }
-        if (backward) {
-            MAG_TRY(alloc_alg(b.loc));
-            MAG_TRY(alloc_alg(b.rem, 12));
+        // the algebra fields of the force in one allocation; a forward-only set needs the six
+        // plane fields of the smearing (in rem) and nothing else
+        AlgPlanes<T> all{nullptr, 0};
+        const int nlam = backward && p.n_stout > 0 ? 8 : 0;
+        const int planes = backward ? 16 + nlam : p.n_stout > 0 ? 6 : 0;
+        if (!planes) return MAG_OK;
+        MAG_TRY(alloc_alg(all, planes));
+        const size_t plane = 8 * (size_t)vpad;
+        b.rem = AlgPlanes<T>{all.p, vpad};
+        if (!backward) return MAG_OK;
+        b.loc = AlgPlanes<T>{all.p + 12 * plane, vpad};
+        if (nlam) {
+            b.lam = AlgPlanes<T>{all.p + 16 * plane, vpad};
+            b.dir = AlgPlanes<T>{all.p + 20 * plane, vpad};
         }
         return MAG_OK;
     }
@@ -427,7 +434,7 @@ struct mag_ctx {
         hx(Uin);
         LinkPlanes<T> cur = Uin;
         for (int k = 0; k < L; k++) {
-            launch_stout_forward<T>(geom, cur, b.lv[k], b.Q[k], var<T>(KF_STOUT_FWD), stream);
+            forward_level(cur, b, k);
             cur = b.lv[k];
             hx(cur);
         }
@@ -446,6 +453,15 @@ struct mag_ctx {
                                    stream);
         }
         if (any_mag) launch_constraint_fixup<T>(geom, Uin, Fout, stream);
+    }
+    // Smearing level k of `cur`.  FP64: over plaquettes (0.64 against 0.80 ms at 32^4 for the
+    // one-thread-per-link kernel at its best shape).  FP32: one thread per link at 102
+    // registers; over plaquettes it takes 0.34 against 0.38 ms, but a force's FP32 error
+    // grows by 15-30% with the transports of its angles.
+    template <typename T>
+    void forward_level(LinkPlanes<T> cur, StoutBufs<T>& b, int k) {
+        if constexpr (sizeof(T) == 8) launch_stout_level<T>(geom, cur, b.lv[k], b.Q[k], b.rem, stream);
+        else launch_stout_forward<T>(geom, cur, b.lv[k], b.Q[k], 3, stream);
     }
     // the plaquettes' rows share the double links' buffer (576 of 576 bytes per site in FP64, 288 of 320 in FP32)
     template <typename T>
@@ -500,7 +516,7 @@ struct mag_ctx {
         LinkPlanes<double> cur = U;
         hx(cur);
         for (int k = 0; k < p.n_stout; k++) {
-            launch_stout_forward<double>(geom, cur, st64.lv[k], st64.Q[k], var<double>(KF_STOUT_FWD), stream);
+            forward_level(cur, st64, k);
             cur = st64.lv[k];
             hx(cur);
         }
@@ -526,7 +542,7 @@ struct mag_ctx {
     // one launch of a kernel of the derivative's plaquette form, on the thin links
     template <typename T>
     void launch_smear(const std::string& w, StoutBufs<T>& b, LinkPlanes<T> Uin, AlgPlanes<T> Fo) {
-        if (w == "stout_level") launch_stout_level<T>(geom, Uin, b.lv[0], b.Q[0], b.rem, stream);
+        if (w == "stout_level") forward_level(Uin, b, 0);
         else if (w == "lambda") launch_lambda<T>(geom, b.Q[0], Fo, b.lam, b.dir, stream);
         else if (w == "plaq_chain") launch_plaq_chain<T>(geom, Uin, b.lam, b.loc, b.rem, stream);
         else if (w == "chain_gather") launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, false, &b.Q[0], b.lam, stream);
@@ -548,19 +564,16 @@ struct mag_ctx {
         return MAG_OK;
     }
 
-    // The tuner: time every register-cap variant of every kernel family the
-    // integrator uses, on live data, and keep the fastest.  Variants compute
+    // The tuner of the one-thread-per-link form: time every register-cap variant of
+    // every kernel family, on live data, and keep the fastest.  Variants compute
     // identical results (same instructions, different register allocation).
     template <typename T>
     int tune_precision(int reps, StoutBufs<T>& b, LinkPlanes<T> Uin, AlgPlanes<T> Fo, LinkPlanes<T> zs) {
-        force_eval<T>(Uin, Fo, b);
+        MAG_TRY(ensure_gather(b));
+        force_eval_gather<T>(Uin, Fo, b);
         std::vector<KernelFamily> fams;
-        if (gather[sizeof(T) == 8 ? 0 : 1]) {
-            if (p.n_stout == 0) fams = {KF_FORCE};
-            else fams = {KF_STAPLE, KF_STOUT_FWD, KF_STOUT_LAMBDA, KF_STOUT_CHAIN};
-        } else if (p.n_stout > 0) {
-            fams = {KF_STOUT_FWD};
-        }
+        if (p.n_stout == 0) fams = {KF_FORCE};
+        else fams = {KF_STAPLE, KF_STOUT_FWD, KF_STOUT_LAMBDA, KF_STOUT_CHAIN};
         // Every variant is timed (the report shows them all), but the choice is made among the
         // one-thread-per-link register caps only: those compute bit-identical results, so a run does not
         // depend on timing noise.  The direction-split shapes add their parts in another order (results
@@ -602,9 +615,9 @@ struct mag_ctx {
             geom.tile = tl;
             geom.gpr = (int)(row / kForceBlockSites);
             geom.L2 = c.L[2];
-            force_eval<T>(Uin, Fo, b);
+            force_eval_gather<T>(Uin, Fo, b);
             MAG_CUDA(cudaEventRecord(ev0, stream));
-            for (int i = 0; i < reps; i++) force_eval<T>(Uin, Fo, b);
+            for (int i = 0; i < reps; i++) force_eval_gather<T>(Uin, Fo, b);
             MAG_CUDA(cudaEventRecord(ev1, stream));
             MAG_TRY(sync("tune order"));
             float t = 0.f;
@@ -620,33 +633,17 @@ struct mag_ctx {
     }
 
     int autotune(int reps) {
-        if (mixed) {
-            MAG_TRY(tune_precision<float>(reps, st32, U32, F32, Uaux32));
-            if (p.n_stout > 0) {
-                // the FP64 forward smearing of the Hamiltonian
-                double best = 1e300;
-                for (int v = 0; v < kNumRegVariants; v++) {
-                    double ms = 0.0;
-                    StoutBufs<double> b = st64;
-                    MAG_TRY(time_one<double>(KF_STOUT_FWD, v, reps, b, U, F, Ubak, &ms));
-                    tune_ms[KF_STOUT_FWD][0][v] = ms;
-                    if (ms < best) {
-                        best = ms;
-                        tune[KF_STOUT_FWD][0] = v;
-                    }
-                }
-            }
-        } else {
-            MAG_TRY(tune_precision<double>(reps, st64, U, F, Uaux));
-        }
-        if (!halo && gather[mixed ? 1 : 0]) {
+        if (mixed) MAG_TRY(tune_precision<float>(reps, st32, U32, F32, Uaux32));
+        else MAG_TRY(tune_precision<double>(reps, st64, U, F, Uaux));
+        if (!halo) {
             if (mixed) MAG_TRY(tune_order<float>(reps, st32, U32, F32));
             else MAG_TRY(tune_order<double>(reps, st64, U, F));
         }
         tuned = true;
         return MAG_OK;
     }
-    int ensure_tuned() { return tuned ? MAG_OK : autotune(3); }
+    // the plaquette form has no launch shapes to choose
+    int ensure_tuned() { return tuned || !gather[mixed ? 1 : 0] ? MAG_OK : autotune(3); }
 
     void hamiltonian_sums(bool is_new) {
         launch_kinetic_sum(geom, P, partial, sums, is_new ? SLOT_KIN_NEW : SLOT_KIN_OLD, stream);

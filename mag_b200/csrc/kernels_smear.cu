@@ -78,7 +78,7 @@ struct site_terms {
 
 // S = (P - P^dag) / 2i of every plaquette (plane fields 0..5 of S)
 template <typename T>
-__global__ void __launch_bounds__(kPlaqBlock) k_plaq_sin(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S) {
+__global__ void __launch_bounds__(kPlaqBlock, 4) k_plaq_sin(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S) {
     ChainInfo ci;
     Site st;
     if (!locate_tile(g, ci, st)) return;
@@ -110,7 +110,7 @@ __device__ __forceinline__ herm8<T> staple_angle(const LinkPlanes<T>& U, const A
 
 // Q = -i rho TA(stp U^dag) (field-multi.h:32-39), U' = e^{iQ} U
 template <typename T>
-__global__ void __launch_bounds__(kLinkBlock) k_stout_apply(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S,
+__global__ void __launch_bounds__(kLinkBlock, 5) k_stout_apply(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S,
                                                             LinkPlanes<T> Uout, AlgPlanes<T> Q) {
     ChainInfo ci;
     Site st;
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kLinkBlock) k_stout_apply(DevGeom g, LinkPlane
     const int mu = threadIdx.x >> 5;
     const herm8<T> q = scaled(staple_angle(U, S, ci, st, mu), (T)ci.rho);
     Q.store(mu, st.g, q);
-    Uout.store(mu, st.g, mul(expiQ(q), U.load(mu, st.g)));
+    Uout.store(mu, st.g, exp_times(q, U.load(mu, st.g)));
 }
 
 // Wilson force F = i beta/3 TA(U A^dag), A the plaquette staples (field-hmc.h:394-421)

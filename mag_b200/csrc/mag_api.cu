@@ -188,8 +188,7 @@ int mag_staple(mag_ctx* ctx, int chain, double* host) {
     if (ctx->mixed) {
         LinkPlanes<float> cur = ctx->U32;
         for (int k = 0; k < ctx->p.n_stout; k++) {
-            launch_stout_forward<float>(ctx->geom, cur, ctx->st32.lv[k], ctx->st32.Q[k],
-                                        ctx->var<float>(KF_STOUT_FWD), ctx->stream);
+            ctx->forward_level(cur, ctx->st32, k);
             cur = ctx->st32.lv[k];
         }
         LinkPlanes<float> z = ctx->Uaux32;
@@ -603,16 +602,11 @@ int mag_time_kernel(mag_ctx* ctx, const char* which, int reps, double* ms) {
     for (int f = 0; f < KF_COUNT; f++)
         if (w == kFamNames[f]) fam = f;
     if (fam >= KF_STOUT_FWD && L == 0) return fail(MAG_ERR_STATE, "mag_time_kernel: no stout levels in this context");
-    MAG_TRY(ctx->ensure_tuned());
     // one full force evaluation first, so every intermediate buffer holds live data
-    if (fam == KF_FORCE || fam == KF_STAPLE || fam == KF_STOUT_LAMBDA || fam == KF_STOUT_CHAIN) {
-        if (m) {
-            MAG_TRY(ctx->ensure_gather(ctx->st32));
-            ctx->force_eval_gather<float>(ctx->U32, ctx->F32, ctx->st32);
-        } else {
-            MAG_TRY(ctx->ensure_gather(ctx->st64));
-            ctx->force_eval_gather<double>(ctx->U, ctx->F, ctx->st64);
-        }
+    if (fam >= 0) {
+        if (!ctx->tuned) MAG_TRY(ctx->autotune(3));
+        if (m) ctx->force_eval_gather<float>(ctx->U32, ctx->F32, ctx->st32);
+        else ctx->force_eval_gather<double>(ctx->U, ctx->F, ctx->st64);
     } else {
         if (m) ctx->force_eval<float>(ctx->U32, ctx->F32, ctx->st32);
         else ctx->force_eval<double>(ctx->U, ctx->F, ctx->st64);
@@ -733,14 +727,13 @@ int mag_set_kernel_variant(mag_ctx* ctx, const char* family, int precision, cons
     if (f < 0) return fail(MAG_ERR_ARG, std::string("mag_set_kernel_variant: unknown family '") + family + "'");
     if (v < 0 || v >= mag_ctx::variants_of((KernelFamily)f))
         return fail(MAG_ERR_ARG, std::string("mag_set_kernel_variant: no variant '") + variant + "' for " + family);
-    MAG_TRY(ctx->ensure_tuned());
-    if (f != KF_STOUT_FWD) {  // kernels of the one-thread-per-link form
-        if ((precision == 1) == ctx->mixed) {
-            if (ctx->mixed) MAG_TRY(ctx->ensure_gather(ctx->st32));
-            else MAG_TRY(ctx->ensure_gather(ctx->st64));
-            ctx->gather[precision] = true;
-        }
+    // the variants are the one-thread-per-link kernels': this precision's forces take that form
+    if ((precision == 1) == ctx->mixed) {
+        if (ctx->mixed) MAG_TRY(ctx->ensure_gather(ctx->st32));
+        else MAG_TRY(ctx->ensure_gather(ctx->st64));
+        ctx->gather[precision] = true;
     }
+    MAG_TRY(ctx->ensure_tuned());
     ctx->tune[f][precision] = v;
     if (ctx->graph) {  // the captured trajectory holds the previous choice
         cudaGraphExecDestroy(ctx->graph);

@@ -254,6 +254,67 @@ MAG_HD mat3<T> plaquette(const mat3<T>& a, const mat3<T>& b, const mat3<T>& c, c
     return mul_nd_su3(x, y);
 }
 
+// e^{iQ} U = (f0 + f1 Q + f2 Q^2) U of a special unitary U: rows 0, 1 of e^{iQ} and of
+// the product, the third reconstructed; the coefficients are those of expiQ
+template <typename T>
+MAG_HD mat3<T> exp_times(const herm8<T>& q, const mat3<T>& U) {
+    const T h0 = q.h[0], h1 = q.h[1], h2 = -q.h[0] - q.h[1];
+    const cplx<T> z01 = mk(q.h[2], q.h[3]), z02 = mk(q.h[4], q.h[5]), z12 = mk(q.h[6], q.h[7]);
+    const T n01 = fmaT(z01.re, z01.re, z01.im * z01.im);
+    const T n02 = fmaT(z02.re, z02.re, z02.im * z02.im);
+    const T n12 = fmaT(z12.re, z12.re, z12.im * z12.im);
+    // rows 0, 1 of Q^2 (Hermitian): 00, 11 and 01, 02, 12
+    const T s00 = fmaT(h0, h0, n01 + n02), s11 = fmaT(h1, h1, n01 + n12), s22 = fmaT(h2, h2, n02 + n12);
+    cplx<T> s01 = mk(-h2 * z01.re, -h2 * z01.im), s02 = mk(-h1 * z02.re, -h1 * z02.im),
+            s12 = mk(-h0 * z12.re, -h0 * z12.im);
+    cmac<false, true, false>(s01, z02, z12);
+    cmac<false, false, false>(s02, z01, z12);
+    cmac<true, false, false>(s12, z01, z02);
+    const T c1 = T(0.5) * (s00 + s11 + s22);
+    if (c1 == T(0)) return U;  // the reference's c1 = 0 branch (field-hmc.h:95)
+    // det Q = Tr Q^3 / 3
+    const cplx<T> p = cmul<false, false>(z01, z12);
+    T c0 = fmaT(p.re, z02.re, p.im * z02.im);
+    c0 = fmaT(T(2), c0, h0 * h1 * h2);
+    c0 = fmaT(-h0, n12, c0);
+    c0 = fmaT(-h1, n02, c0);
+    c0 = fmaT(-h2, n01, c0);
+    cplx<T> f0, f1, f2;
+    if constexpr (sizeof(T) == 4) {
+        ch_coef_f c;
+        if (!ch_series<false>(c0, c1, c)) c = ch_to_float(ch_coefficients<false>((double)c0, (double)c1));
+        f0 = mk(c.f0r, c.f0i);
+        f1 = mk(c.f1r, c.f1i);
+        f2 = mk(c.f2r, c.f2i);
+    } else {
+        double f[6];
+        if (ch_series_exp_d(c0, c1, f)) {
+            f0 = mk<T>(f[0], f[1]);
+            f1 = mk<T>(f[2], f[3]);
+            f2 = mk<T>(f[4], f[5]);
+        } else {
+            const ch_coef c = ch_coefficients<false>(c0, c1);
+            f0 = mk<T>(c.f0r, c.f0i);
+            f1 = mk<T>(c.f1r, c.f1i);
+            f2 = mk<T>(c.f2r, c.f2i);
+        }
+    }
+    mat3<T> e;
+    auto diag = [&](T x, T s) { return mk(fmaT(f2.re, s, fmaT(f1.re, x, f0.re)), fmaT(f2.im, s, fmaT(f1.im, x, f0.im))); };
+    auto off = [&](cplx<T> x, cplx<T> s) {
+        cplx<T> r = cmul<false, false>(f1, x);
+        cmac<false, false, false>(r, f2, s);
+        return r;
+    };
+    e.e[0][0] = diag(h0, s00);
+    e.e[0][1] = off(z01, s01);
+    e.e[0][2] = off(z02, s02);
+    e.e[1][0] = off(conj(z01), conj(s01));
+    e.e[1][1] = diag(h1, s11);
+    e.e[1][2] = off(z12, s12);
+    return mul_su3(e, U);
+}
+
 // y <- prod_{j=1..n} (1 + e^{-i ad_Q / 2^j}) / 2 y, so that phi(-i ad_Q) x =
 // phi(-i ad_Q / 2^n) y from y = x (phi(2z) = phi(z) (1 + e^z) / 2).  Out of line: only
 // |Q| beyond the series of lambda_adjoint comes here, and the exponential's registers
