@@ -800,15 +800,45 @@ struct mag_ctx {
         return MAG_OK;
     }
 
+    // loops in the temporal gauge: gauge, gauged links and Polyakov lines of the largest chain,
+    // block partials, results and the unitarity flag
+    cplx<double>* wg_links = nullptr;
+    dd2 *wg_part = nullptr, *wg_out = nullptr;
+    size_t wg_parts = 0;
+    int wg_rt = 0;
+    int ensure_gauged(int RT, size_t parts) {
+        if (!wg_links) {
+            const size_t vp = ((size_t)max_v + MAG_TILE - 1) / MAG_TILE * MAG_TILE;
+            MAG_TRY(alloc((void**)&wg_links, sizeof(cplx<double>) * 9 * 5 * vp));
+        }
+        if (RT > wg_rt) {
+            cudaStreamSynchronize(stream);
+            free_one(wg_out);
+            wg_out = nullptr;
+            wg_rt = 0;
+            MAG_TRY(alloc((void**)&wg_out, sizeof(dd2) * (RT + 1)));
+            wg_rt = RT;
+        }
+        if (parts > wg_parts) {
+            cudaStreamSynchronize(stream);
+            free_one(wg_part);
+            wg_part = nullptr;
+            wg_parts = 0;
+            MAG_TRY(alloc((void**)&wg_part, sizeof(dd2) * parts));
+            wg_parts = parts;
+        }
+        return MAG_OK;
+    }
+
     int chain_ok(int c) {
         if (c < 0 || c >= nchain) return fail(MAG_ERR_ARG, "chain index out of range");
         return MAG_OK;
     }
 
-    // read per-chain double-double sums back to the host
-    int read_sums(std::vector<dd2>& out) {
-        out.resize((size_t)NUM_SLOTS * nchain);
-        MAG_CUDA(cudaMemcpyAsync(out.data(), sums, sizeof(dd2) * out.size(), cudaMemcpyDeviceToHost, stream));
+    // read a chain's double-double sums back to the host
+    int read_sums(int chain, dd2 out[NUM_SLOTS]) {
+        MAG_CUDA(cudaMemcpyAsync(out, sums + chain * NUM_SLOTS, sizeof(dd2) * NUM_SLOTS, cudaMemcpyDeviceToHost,
+                                 stream));
         return sync("read sums");
     }
 

@@ -139,11 +139,13 @@ void launch_link_copy(const DevGeom& g, LinkPlanes<double> src, LinkPlanes<doubl
 void launch_restore_rejected(const DevGeom& g, LinkPlanes<double> backup, LinkPlanes<double> U,
                              LinkPlanes<float> U32, const ChainState* st, cudaStream_t s);
 
-// ---- reductions (kernels_update.cu); partial must hold vpad / MAG_CHUNK * 2 dd2
+// ---- reductions (kernels_update.cu), over every chain or, with only = the info of chain `chain`, over
+// that chain alone (the same sums; the other chains' slots keep what they hold); partial must hold vpad / MAG_CHUNK * 2 dd2
 template <typename T>
 void launch_action_sums(const DevGeom& g, LinkPlanes<T> U, bool with_rect, dd2* partial, dd2* sums, int slot_plaq,
-                        int slot_rect, cudaStream_t s);
-void launch_kinetic_sum(const DevGeom& g, AlgPlanes<double> P, dd2* partial, dd2* sums, int slot, cudaStream_t s);
+                        int slot_rect, cudaStream_t s, const ChainInfo* only = nullptr, int chain = 0);
+void launch_kinetic_sum(const DevGeom& g, AlgPlanes<double> P, dd2* partial, dd2* sums, int slot, cudaStream_t s,
+                        const ChainInfo* only = nullptr, int chain = 0);
 void launch_accept(const DevGeom& g, const AcceptArgs& a, dd2* sums, ChainState* st,
                    const unsigned long long* reunit, TrajRecord* rec, long long* traj_counter, cudaStream_t s);
 // completes rec[] with the thin plaquette, appends it to hist[(counter - *hist_base) * nchain + c]
@@ -235,6 +237,16 @@ void launch_demon_sweeps(const DemonJob* jobs, int njobs, double* aos, const Dem
 // out[((i * Tmax + T-1) * nchain + c) * Rmax + R-1] (i = spatial direction)
 void launch_wilson_planar(const DevGeom& g, LinkPlanes<double> U, int Rmax, int Tmax, LinkPlanes<double> lines,
                           LinkPlanes<double> tl, LinkPlanes<double> tl2, dd2* partial, dd2* out, cudaStream_t s);
+// the same for one chain of unitary links in the temporal gauge: out[(R-1) * Tmax + T-1] = the sum over
+// the three directions and the chain's sites.  nx = wilson_gauged_sites must not be 0; scratch G (one
+// direction) and V (three) of ci.V sites, P of L0 L1 L2 sites (one direction), part of
+// wilson_gauged_partials entries; *bad (zeroed by the caller) is set when a link is not unitary, and the
+// sums are then not the loops.
+int wilson_gauged_sites(const ChainInfo& ci, int Tmax);
+size_t wilson_gauged_partials(const ChainInfo& ci, int Rmax, int Tmax);
+cudaError_t launch_wilson_gauged(const ChainInfo& ci, LinkPlanes<double> U, int Rmax, int Tmax, LinkPlanes<double> G,
+                                 LinkPlanes<double> V, LinkPlanes<double> P, dd2* part, dd2* out, int* bad,
+                                 cudaStream_t s);
 // sum over sites (coarse sites x = 0 mod coarse_mag when coarse_mag > 0) and
 // npath closed paths of ReTr; dirs[npath][plen], 0..3 forward, 4..7 backward,
 // -1 ends a shorter path; out[c]

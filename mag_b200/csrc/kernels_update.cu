@@ -180,28 +180,30 @@ __global__ void k_restore(DevGeom g, LinkPlanes<double> backup, LinkPlanes<doubl
 
 // ---------------------------------------------------------------- reductions
 template <typename T>
-__global__ void k_action_partials(DevGeom g, LinkPlanes<T> U, int with_rect, dd2* partial) {
+__global__ void k_action_partials(DevGeom g, LinkPlanes<T> U, int with_rect, int block0, dd2* partial) {
     ChainInfo ci;
     Site st;
     dd2 p = {0.0, 0.0}, r = {0.0, 0.0};
-    if (locate(g, blockIdx.x * blockDim.x + threadIdx.x, ci, st) && interior(ci, st)) {
+    const int blk = block0 + blockIdx.x;
+    if (locate(g, blk * blockDim.x + threadIdx.x, ci, st) && interior(ci, st)) {
         p.hi = site_plaquette(U, ci, st);
         if (with_rect) r.hi = site_rectangle(U, ci, st);
     }
     p = block_reduce(p);
     r = block_reduce(r);
     if (threadIdx.x == 0) {
-        partial[2 * blockIdx.x] = p;
-        partial[2 * blockIdx.x + 1] = r;
+        partial[2 * blk] = p;
+        partial[2 * blk + 1] = r;
     }
 }
 
 // kinetic energy sum of Re Tr(P^2), constrained-last links excluded (field-hmc.h:605-620)
-__global__ void k_kinetic_partials(DevGeom g, AlgPlanes<double> P, dd2* partial) {
+__global__ void k_kinetic_partials(DevGeom g, AlgPlanes<double> P, int block0, dd2* partial) {
     ChainInfo ci;
     Site st;
     dd2 k = {0.0, 0.0};
-    if (locate(g, blockIdx.x * blockDim.x + threadIdx.x, ci, st) && interior(ci, st)) {
+    const int blk = block0 + blockIdx.x;
+    if (locate(g, blk * blockDim.x + threadIdx.x, ci, st) && interior(ci, st)) {
         double acc = 0.0;
 #pragma unroll
         for (int mu = 0; mu < 4; mu++) {
@@ -211,7 +213,7 @@ __global__ void k_kinetic_partials(DevGeom g, AlgPlanes<double> P, dd2* partial)
         k.hi = acc;
     }
     k = block_reduce(k);
-    if (threadIdx.x == 0) partial[2 * blockIdx.x] = k;
+    if (threadIdx.x == 0) partial[2 * blk] = k;
 }
 
 // per chain: sum the partials of its blocks in block order
@@ -229,8 +231,8 @@ __global__ void k_link_trace_partials(DevGeom g, LinkPlanes<double> U, dd2* part
     k = block_reduce(k);
     if (threadIdx.x == 0) partial[2 * blockIdx.x] = k;
 }
-__global__ void k_finalize(DevGeom g, const dd2* partial, int nq, dd2* sums, int slot0, double scale0) {
-    const int c = blockIdx.x;
+__global__ void k_finalize(DevGeom g, const dd2* partial, int chain0, int nq, dd2* sums, int slot0, double scale0) {
+    const int c = chain0 + blockIdx.x;
     const ChainInfo ci = g.chains[c];
     const int b0 = ci.off / kBlock, b1 = (ci.off + ci.V + kBlock - 1) / kBlock;
     for (int q = 0; q < nq; q++) {
@@ -530,26 +532,40 @@ void launch_restore_rejected(const DevGeom& g, LinkPlanes<double> backup, LinkPl
     k_restore<<<dim3(blocks(g), 4), kBlock, 0, s>>>(g, backup, U, U32, st);
 }
 
+namespace {
+// blocks and chains of a reduction over the whole geometry or one chain
+struct SumRange {
+    int block0, nblocks, chain0, nchains;
+};
+SumRange sum_range(const DevGeom& g, const ChainInfo* only, int chain) {
+    if (!only) return SumRange{0, (int)blocks(g), 0, g.nchain};
+    return SumRange{only->off / kBlock, (only->V + kBlock - 1) / kBlock, chain, 1};
+}
+}  // namespace
+
 template <typename T>
 void launch_action_sums(const DevGeom& g, LinkPlanes<T> U, bool with_rect, dd2* partial, dd2* sums, int slot_plaq,
-                        int slot_rect, cudaStream_t s) {
-    k_action_partials<T><<<blocks(g), kBlock, 0, s>>>(g, U, with_rect ? 1 : 0, partial);
-    k_finalize<<<g.nchain, kBlock, 0, s>>>(g, partial, 1, sums, slot_plaq, 1.0);
-    if (with_rect) k_finalize<<<g.nchain, kBlock, 0, s>>>(g, partial + 1, 1, sums, slot_rect, 1.0);
+                        int slot_rect, cudaStream_t s, const ChainInfo* only, int chain) {
+    const SumRange r = sum_range(g, only, chain);
+    k_action_partials<T><<<r.nblocks, kBlock, 0, s>>>(g, U, with_rect ? 1 : 0, r.block0, partial);
+    k_finalize<<<r.nchains, kBlock, 0, s>>>(g, partial, r.chain0, 1, sums, slot_plaq, 1.0);
+    if (with_rect) k_finalize<<<r.nchains, kBlock, 0, s>>>(g, partial + 1, r.chain0, 1, sums, slot_rect, 1.0);
 }
 template void launch_action_sums<double>(const DevGeom&, LinkPlanes<double>, bool, dd2*, dd2*, int, int,
-                                         cudaStream_t);
+                                         cudaStream_t, const ChainInfo*, int);
 template void launch_action_sums<float>(const DevGeom&, LinkPlanes<float>, bool, dd2*, dd2*, int, int,
-                                        cudaStream_t);
+                                        cudaStream_t, const ChainInfo*, int);
 
 void launch_link_trace_sum(const DevGeom& g, LinkPlanes<double> U, dd2* partial, dd2* sums, int slot,
                            cudaStream_t s) {
     k_link_trace_partials<<<blocks(g), kBlock, 0, s>>>(g, U, partial);
-    k_finalize<<<g.nchain, kBlock, 0, s>>>(g, partial, 1, sums, slot, 1.0);
+    k_finalize<<<g.nchain, kBlock, 0, s>>>(g, partial, 0, 1, sums, slot, 1.0);
 }
-void launch_kinetic_sum(const DevGeom& g, AlgPlanes<double> P, dd2* partial, dd2* sums, int slot, cudaStream_t s) {
-    k_kinetic_partials<<<blocks(g), kBlock, 0, s>>>(g, P, partial);
-    k_finalize<<<g.nchain, kBlock, 0, s>>>(g, partial, 1, sums, slot, 0.5);
+void launch_kinetic_sum(const DevGeom& g, AlgPlanes<double> P, dd2* partial, dd2* sums, int slot, cudaStream_t s,
+                        const ChainInfo* only, int chain) {
+    const SumRange r = sum_range(g, only, chain);
+    k_kinetic_partials<<<r.nblocks, kBlock, 0, s>>>(g, P, r.block0, partial);
+    k_finalize<<<r.nchains, kBlock, 0, s>>>(g, partial, r.chain0, 1, sums, slot, 0.5);
 }
 
 void launch_accept(const DevGeom& g, const AcceptArgs& a, dd2* sums, ChainState* st,

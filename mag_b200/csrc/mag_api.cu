@@ -215,11 +215,11 @@ int mag_action(mag_ctx* ctx, int chain, double* plaq, double* rect, double* acti
     MAG_TRY(ctx->chain_ok(chain));
     LinkPlanes<double> top = ctx->smear64();
     launch_action_sums<double>(ctx->geom, top, true, ctx->partial, ctx->sums, SLOT_PLAQ_THIN, SLOT_RECT_THIN,
-                               ctx->stream);
+                               ctx->stream, &ctx->hc[chain], chain);
     MAG_TRY(ctx->check("mag_action"));
-    std::vector<dd2> s;
-    MAG_TRY(ctx->read_sums(s));
-    const dd2 pl = s[chain * NUM_SLOTS + SLOT_PLAQ_THIN], re = s[chain * NUM_SLOTS + SLOT_RECT_THIN];
+    dd2 s[NUM_SLOTS];
+    MAG_TRY(ctx->read_sums(chain, s));
+    const dd2 pl = s[SLOT_PLAQ_THIN], re = s[SLOT_RECT_THIN];
     if (plaq) *plaq = pl.hi + pl.lo;
     if (rect) *rect = re.hi + re.lo;
     const hdd a = ctx->action_value(chain, pl, re);
@@ -231,11 +231,11 @@ int mag_plaquette(mag_ctx* ctx, int chain, double* avg) {
     if (!ctx || !avg) return MAG_ERR_ARG;
     MAG_TRY(ctx->chain_ok(chain));
     launch_action_sums<double>(ctx->geom, ctx->U, false, ctx->partial, ctx->sums, SLOT_SCRATCH, SLOT_SCRATCH,
-                               ctx->stream);
+                               ctx->stream, &ctx->hc[chain], chain);
     MAG_TRY(ctx->check("mag_plaquette"));
-    std::vector<dd2> s;
-    MAG_TRY(ctx->read_sums(s));
-    const dd2 pl = s[chain * NUM_SLOTS + SLOT_SCRATCH];
+    dd2 s[NUM_SLOTS];
+    MAG_TRY(ctx->read_sums(chain, s));
+    const dd2 pl = s[SLOT_SCRATCH];
     *avg = (pl.hi + pl.lo) / (18.0 * ctx->hc[chain].V);
     return MAG_OK;
 }
@@ -243,11 +243,12 @@ int mag_plaquette(mag_ctx* ctx, int chain, double* avg) {
 int mag_kinetic(mag_ctx* ctx, int chain, double* kin) {
     if (!ctx || !kin) return MAG_ERR_ARG;
     MAG_TRY(ctx->chain_ok(chain));
-    launch_kinetic_sum(ctx->geom, ctx->P, ctx->partial, ctx->sums, SLOT_SCRATCH, ctx->stream);
+    launch_kinetic_sum(ctx->geom, ctx->P, ctx->partial, ctx->sums, SLOT_SCRATCH, ctx->stream, &ctx->hc[chain],
+                       chain);
     MAG_TRY(ctx->check("mag_kinetic"));
-    std::vector<dd2> s;
-    MAG_TRY(ctx->read_sums(s));
-    const dd2 k = s[chain * NUM_SLOTS + SLOT_SCRATCH];
+    dd2 s[NUM_SLOTS];
+    MAG_TRY(ctx->read_sums(chain, s));
+    const dd2 k = s[SLOT_SCRATCH];
     *kin = k.hi + k.lo;
     return MAG_OK;
 }
@@ -257,9 +258,8 @@ int mag_hamiltonian(mag_ctx* ctx, int chain, double out[3]) {
     MAG_TRY(ctx->chain_ok(chain));
     ctx->hamiltonian_sums(false);
     MAG_TRY(ctx->check("mag_hamiltonian"));
-    std::vector<dd2> s;
-    MAG_TRY(ctx->read_sums(s));
-    const dd2* S = s.data() + chain * NUM_SLOTS;
+    dd2 S[NUM_SLOTS];
+    MAG_TRY(ctx->read_sums(chain, S));
     const hdd a = ctx->action_value(chain, S[SLOT_PLAQ_OLD], S[SLOT_RECT_OLD]);
     const hdd k = hdd{S[SLOT_KIN_OLD].hi, S[SLOT_KIN_OLD].lo};
     const hdd h = h_add(a, k);
@@ -849,10 +849,43 @@ int mag_wilson_loop(mag_ctx* ctx, int chain, const int r[3], int T, double* out)
     return MAG_OK;
 }
 
+// one chain's planar loops in the temporal gauge; *unitary = false: a link is not unitary, out is not written
+static int wilson_gauged(mag_ctx* ctx, int chain, int Rmax, int Tmax, double* out, bool* unitary) {
+    const ChainInfo& ci = ctx->hc[chain];
+    const int RT = Rmax * Tmax;
+    MAG_TRY(ctx->ensure_gauged(RT, wilson_gauged_partials(ci, Rmax, Tmax)));
+    const long vp = ((long)ci.V + MAG_TILE - 1) / MAG_TILE * MAG_TILE;
+    const LinkPlanes<double> G{ctx->wg_links, vp}, V{ctx->wg_links + 9 * vp, vp}, P{ctx->wg_links + 36 * vp, vp};
+    int* bad = reinterpret_cast<int*>(ctx->wg_out + RT);
+    MAG_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
+    MAG_CUDA(cudaMemsetAsync(bad, 0, sizeof(dd2), ctx->stream));
+    MAG_CUDA(launch_wilson_gauged(ci, ctx->U, Rmax, Tmax, G, V, P, ctx->wg_part, ctx->wg_out, bad, ctx->stream));
+    MAG_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
+    std::vector<dd2> h(RT + 1);
+    MAG_CUDA(cudaMemcpyAsync(h.data(), ctx->wg_out, sizeof(dd2) * h.size(), cudaMemcpyDeviceToHost, ctx->stream));
+    MAG_TRY(ctx->sync("mag_wilson_loops"));
+    int flag = 0;
+    std::memcpy(&flag, &h[RT], sizeof flag);
+    *unitary = flag == 0;
+    if (flag) return MAG_OK;
+    float ms = 0.f;
+    MAG_CUDA(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
+    ctx->last_measure_ms = ms;
+    const double norm = 3.0 * ci.V;  // perm.size() * V (field-wloop.h:98)
+    for (int k = 0; k < RT; k++) out[k] = (h[k].hi + h[k].lo) / norm;
+    return MAG_OK;
+}
+
 int mag_wilson_loops(mag_ctx* ctx, int chain, int Rmax, int Tmax, double* out) {
     if (!ctx || !out || Rmax < 1 || Tmax < 1 || Rmax > 64 || Tmax > 64)
         return fail(MAG_ERR_ARG, "mag_wilson_loops: bad arguments");
     MAG_TRY(ctx->chain_ok(chain));
+    if (wilson_gauged_sites(ctx->hc[chain], Tmax) > 0) {
+        bool unitary = false;
+        MAG_TRY(wilson_gauged(ctx, chain, Rmax, Tmax, out, &unitary));
+        if (unitary) return MAG_OK;
+    }
+    // any links, any extent: the line products of every chain
     MAG_TRY(ctx->ensure_meas(Rmax, Tmax, true));
     const long vp = ctx->vpad;
     LinkPlanes<double> lines{ctx->wl_lines, vp};

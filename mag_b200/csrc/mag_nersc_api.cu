@@ -67,13 +67,13 @@ namespace {
 // avg_plaquette (field-matrix.h:387-389) and avg_real_trace (:391-405) of one chain
 int plaq_and_trace(mag_ctx* ctx, int chain, double* plaq, double* trace) {
     launch_action_sums<double>(ctx->geom, ctx->U, false, ctx->partial, ctx->sums, SLOT_SCRATCH, SLOT_SCRATCH,
-                               ctx->stream);
+                               ctx->stream, &ctx->hc[chain], chain);
     launch_link_trace_sum(ctx->geom, ctx->U, ctx->partial, ctx->sums, SLOT_SCRATCH2, ctx->stream);
     MAG_TRY(ctx->check("NERSC plaquette"));
-    std::vector<dd2> s;
-    MAG_TRY(ctx->read_sums(s));
+    dd2 s[NUM_SLOTS];
+    MAG_TRY(ctx->read_sums(chain, s));
     const double V = (double)ctx->hc[chain].V;
-    const dd2 pl = s[chain * NUM_SLOTS + SLOT_SCRATCH], tr = s[chain * NUM_SLOTS + SLOT_SCRATCH2];
+    const dd2 pl = s[SLOT_SCRATCH], tr = s[SLOT_SCRATCH2];
     *plaq = (pl.hi + pl.lo) / (18.0 * V);
     *trace = (tr.hi + tr.lo) / (12.0 * V);
     return MAG_OK;
