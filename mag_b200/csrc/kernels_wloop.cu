@@ -14,7 +14,7 @@
 //   W_i(R, T)(x, t) = ReTr(S_R(x, t) S_R(x, t + T)^dag):
 // no product at all, 18 multiply-adds.  The lines of a few spatial sites over all t
 // stay in shared memory while R grows; nothing but the gauged links is read.
-// 24^3 x 48, R, T <= 8: 10.9 ms by line products, 1.28 ms so.
+// 24^3 x 48, R, T <= 8: 10.9 ms by line products, 0.98 ms so.
 #include "gauge_ops.cuh"
 #include "kernels.h"
 
@@ -240,16 +240,19 @@ __global__ void __launch_bounds__(kBlock) k_gauge_links(ChainInfo ci, LinkPlanes
     V.store(i, s, mul_nd(mul(G.load(0, s), u), G.load(0, sn)));
 }
 
-// One block: NX spatial sites (blockDim = NX times the groups of four time slices, in
+// One block: NX spatial sites (blockDim = NX times the groups of three time slices, in
 // whole warps), direction i = blockIdx.y.  Shared memory holds S_R of the sites for
-// t in [0, Lt + Tmax).  A thread extends the lines of its four slices, then takes the
-// traces of its four slices with the slices up to T + 3 later, each read once for four
-// loops.  A block walks the groups of NX sites with stride gridDim.x and adds up its
+// t in [0, Lt + Tmax).  A thread extends the lines of its three slices, then takes the
+// traces of its slices with the slices up to T + 2 later, each read once for three
+// loops.  Bound by shared-memory reads (36 cycles per matrix and warp against 9 for a
+// trace's multiply-adds) and the warps that registers and the 72 KB allow: three slices
+// at 168 registers 0.98 ms at 24^3 x 48 (R, T <= 8), four at 208 or 232 1.25, two at
+// 128 1.11; 48^3 x 96: 15.9, 23.8 and 24.9 ms.  A block walks the groups of NX sites with stride gridDim.x and adds up its
 // part[((i Rmax + R-1) Tmax + T-1) gridDim.x + block].
-constexpr int kSlices = 4, kTChunk = 8;
+constexpr int kSlices = 3, kTChunk = 8;
 constexpr int kGaugedBlocks = 592;  // per direction at most: four per SM
 template <int NX>
-__global__ void __launch_bounds__(256) k_wloop_gauged(ChainInfo ci, LinkPlanes<double> V, LinkPlanes<double> P,
+__global__ void __maxnreg__(168) k_wloop_gauged(ChainInfo ci, LinkPlanes<double> V, LinkPlanes<double> P,
                                                       int Rmax, int Tmax, dd2* part) {
     extern __shared__ __align__(16) unsigned char wsm[];
     cplx<double>* S = reinterpret_cast<cplx<double>*>(wsm);  // [Lt + Tmax][9][NX]
@@ -354,7 +357,7 @@ unsigned blocks(const DevGeom& g) { return (unsigned)((g.vpad + kBlock - 1) / kB
 }  // namespace
 
 // Shapes of k_wloop_gauged: the most spatial sites per block (32 down to 1) whose lines
-// take at most 72 KB (three blocks per SM) and whose four-slice groups fit 256 threads;
+// take at most 72 KB (three blocks per SM) and whose slice groups fit 256 threads;
 // 0: none, the chain is too long in time.
 int wilson_gauged_sites(const ChainInfo& ci, int Tmax) {
     if (Tmax > ci.L[3]) return 0;
