@@ -142,6 +142,7 @@ struct mag_ctx {
     StoutBufs<float> st32;
     dd2* partial = nullptr;
     dd2* sums = nullptr;
+    dd2* h_sums = nullptr;  // pinned: one chain's sums, written by the reductions of the measurement calls
     ChainState* cstate = nullptr;
     unsigned long long* reunit = nullptr;
     TrajRecord* rec = nullptr;
@@ -205,6 +206,8 @@ struct mag_ctx {
 
     void release() {
         pin.release();
+        if (h_sums) cudaFreeHost(h_sums);
+        h_sums = nullptr;
         if (graph) cudaGraphExecDestroy(graph);
         graph = nullptr;
         for (void* a : allocs) cudaFree(a);
@@ -372,7 +375,8 @@ struct mag_ctx {
             MAG_TRY(alloc_stout(st64, true));
             if (iwasaki) MAG_TRY(alloc_links(W64));
         }
-        MAG_TRY(alloc((void**)&partial, sizeof(dd2) * 2 * (nchunk + 1)));
+        MAG_TRY(alloc((void**)&partial, sizeof(dd2) * 2 * (vpad / MAG_TILE)));
+        MAG_CUDA(cudaHostAlloc((void**)&h_sums, sizeof(dd2) * NUM_SLOTS, cudaHostAllocMapped));
         MAG_TRY(alloc((void**)&sums, sizeof(dd2) * NUM_SLOTS * n));
         MAG_TRY(alloc((void**)&cstate, sizeof(ChainState) * n));
         MAG_TRY(alloc((void**)&reunit, sizeof(unsigned long long) * n));
@@ -648,7 +652,7 @@ struct mag_ctx {
     void hamiltonian_sums(bool is_new) {
         launch_kinetic_sum(geom, P, partial, sums, is_new ? SLOT_KIN_NEW : SLOT_KIN_OLD, stream);
         LinkPlanes<double> top = smear64();
-        launch_action_sums<double>(geom, top, true, partial, sums, is_new ? SLOT_PLAQ_NEW : SLOT_PLAQ_OLD,
+        launch_action_sums(geom, top, true, partial, sums, is_new ? SLOT_PLAQ_NEW : SLOT_PLAQ_OLD,
                                    is_new ? SLOT_RECT_NEW : SLOT_RECT_OLD, stream);
         if (is_new) hreduce({SLOT_KIN_NEW, SLOT_PLAQ_NEW, SLOT_RECT_NEW}, true);
         else hreduce({SLOT_KIN_OLD, SLOT_PLAQ_OLD, SLOT_RECT_OLD}, false);
@@ -714,7 +718,7 @@ struct mag_ctx {
         launch_accept(geom, a, sums, cstate, reunit, rec, traj_counter, stream);
         launch_restore_rejected(geom, Ubak, U, mixed ? U32 : LinkPlanes<float>{nullptr, 0}, cstate, stream);
         hx(U);
-        launch_action_sums<double>(geom, U, false, partial, sums, SLOT_PLAQ_THIN, SLOT_RECT_THIN, stream);
+        launch_action_sums(geom, U, false, partial, sums, SLOT_PLAQ_THIN, SLOT_RECT_THIN, stream);
         hreduce({SLOT_PLAQ_THIN, SLOT_RECT_THIN}, false);
         launch_record_plaquette(geom, sums, rec, hist, hist_base, kHistCap, traj_counter, stream);
         if (halo_rc != MAG_OK) return halo_rc;
@@ -835,6 +839,7 @@ struct mag_ctx {
         return MAG_OK;
     }
 
+    OneChain one_chain(int c) const { return OneChain{&hc[c], c, h_sums}; }
     // read a chain's double-double sums back to the host
     int read_sums(int chain, dd2 out[NUM_SLOTS]) {
         MAG_CUDA(cudaMemcpyAsync(out, sums + chain * NUM_SLOTS, sizeof(dd2) * NUM_SLOTS, cudaMemcpyDeviceToHost,

@@ -328,47 +328,35 @@ MAG_HD mat3<TU> evolve_link(const mat3<TU>& u, const AlgPlanes<TX>& X, double ep
     return r;
 }
 
-// ReTr of the six plaquettes at x (field-matrix.h:202-221 get_plaq)
-template <typename T>
-MAG_HD double site_plaquette(const LinkPlanes<T>& U, const ChainInfo& ci, const Site& st) {
-    double s = 0.0;
-#pragma unroll 1
-    for (int mu = 1; mu < 4; mu++) {
-        const mat3<T> umu = U.load(mu, st.g);
-#pragma unroll 1
-        for (int nu = 0; nu < mu; nu++) {
-            const mat3<T> m = mul(umu, U.load(nu, nb(ci, st, mu, 1)));
-            const mat3<T> n = mul(U.load(nu, st.g), U.load(mu, nb(ci, st, nu, 1)));
-            s += (double)retr(mul_nd(m, n));
-        }
+// ReTr of the plaquette of plane p, q at x (field-matrix.h:202-221 get_plaq) and, with
+// RECT, of the two 1x2 rectangles that start there (:249-297 get_rectangular), for any
+// matrices: the corner products A = U_p(x) U_q(x+p) and B (p and q exchanged) serve all
+// three loops, and a loop is the inner product of its two halves.  A rolled loop over
+// the two corners: unrolled, the four matrices that are live spill.  put / get keep A
+// until the second corner (shared memory).
+template <bool RECT, typename T, typename Put, typename Get>
+MAG_HD void plane_loops(const LinkPlanes<T>& U, const ChainInfo& ci, const Site& st, int p, int q, double& plaq,
+                        double& rect, Put put, Get get) {
+    if (!RECT) {
+        const mat3<T> A = mul(U.load(p, st.g), U.load(q, nb_sel(ci, st, p, 1)));
+        plaq = (double)retr_mul_nd(A, mul(U.load(q, st.g), U.load(p, nb_sel(ci, st, q, 1))));
+        return;
     }
-    return s;
-}
-
-// ReTr of the twelve 1x2 rectangles at x (field-matrix.h:249-297 get_rectangular)
-template <typename T>
-MAG_HD double site_rectangle(const LinkPlanes<T>& U, const ChainInfo& ci, const Site& st) {
-    double s = 0.0;
+    rect = 0.0;
 #pragma unroll 1
-    for (int mu = 1; mu < 4; mu++) {
-        const mat3<T> umu = U.load(mu, st.g);
-        const int gm = nb(ci, st, mu, 1);
-#pragma unroll 1
-        for (int nu = 0; nu < mu; nu++) {
-            const mat3<T> unu = U.load(nu, st.g);
-            const int gn = nb(ci, st, nu, 1);
-            const int gmn = nb(ci, st, mu, 1, nu, 1);
-            // (U_mu(x) U_nu(x+mu) U_nu(x+mu+nu))^dag vs U_nu(x) U_nu(x+nu) U_mu(x+2nu)
-            mat3<T> a = mul(mul(umu, U.load(nu, gm)), U.load(nu, gmn));
-            mat3<T> b = mul(mul(unu, U.load(nu, gn)), U.load(mu, nb(ci, st, nu, 2)));
-            s += (double)retr(mul_nd(b, a));
-            // (U_mu(x) U_mu(x+mu) U_nu(x+2mu))^dag vs U_nu(x) U_mu(x+nu) U_mu(x+mu+nu)
-            a = mul(mul(umu, U.load(mu, gm)), U.load(nu, nb(ci, st, mu, 2)));
-            b = mul(mul(unu, U.load(mu, gn)), U.load(mu, gmn));
-            s += (double)retr(mul_nd(b, a));
-        }
+    for (int k = 0; k < 2; k++) {
+        const int gp = nb_sel(ci, st, p, 1), gq = nb_sel(ci, st, q, 1);
+        mat3<T> A = mul(U.load(p, st.g), U.load(q, gp));
+        if (k == 0) put(A);
+        else plaq = (double)retr_mul_nd(A, get());
+        // two links along q: A U_q(x+p+q) against U_q(x) U_q(x+q) U_p(x+2q)
+        A = mul(A, U.load(q, gp + gq - st.g));
+        const mat3<T> y = mul(U.load(q, gq), U.load(p, nb_sel(ci, st, q, 2)));
+        rect += (double)retr_mul_nd(A, mul(U.load(q, st.g), y));
+        const int t = p;
+        p = q;
+        q = t;
     }
-    return s;
 }
 
 }  // namespace magb

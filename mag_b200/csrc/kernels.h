@@ -139,13 +139,18 @@ void launch_link_copy(const DevGeom& g, LinkPlanes<double> src, LinkPlanes<doubl
 void launch_restore_rejected(const DevGeom& g, LinkPlanes<double> backup, LinkPlanes<double> U,
                              LinkPlanes<float> U32, const ChainState* st, cudaStream_t s);
 
-// ---- reductions (kernels_update.cu), over every chain or, with only = the info of chain `chain`, over
-// that chain alone (the same sums; the other chains' slots keep what they hold); partial must hold vpad / MAG_CHUNK * 2 dd2
-template <typename T>
-void launch_action_sums(const DevGeom& g, LinkPlanes<T> U, bool with_rect, dd2* partial, dd2* sums, int slot_plaq,
-                        int slot_rect, cudaStream_t s, const ChainInfo* only = nullptr, int chain = 0);
+// ---- reductions (kernels_update.cu), over every chain or over one alone (the same sums; the other
+// chains' slots keep what they hold), which then also go to host[slot] (pinned, when not null);
+// partial must hold vpad / MAG_TILE * 2 dd2
+struct OneChain {
+    const ChainInfo* info;
+    int chain;
+    dd2* host;
+};
+void launch_action_sums(const DevGeom& g, LinkPlanes<double> U, bool with_rect, dd2* partial, dd2* sums, int slot_plaq,
+                        int slot_rect, cudaStream_t s, const OneChain* only = nullptr);
 void launch_kinetic_sum(const DevGeom& g, AlgPlanes<double> P, dd2* partial, dd2* sums, int slot, cudaStream_t s,
-                        const ChainInfo* only = nullptr, int chain = 0);
+                        const OneChain* only = nullptr);
 void launch_accept(const DevGeom& g, const AcceptArgs& a, dd2* sums, ChainState* st,
                    const unsigned long long* reunit, TrajRecord* rec, long long* traj_counter, cudaStream_t s);
 // completes rec[] with the thin plaquette, appends it to hist[(counter - *hist_base) * nchain + c]

@@ -47,7 +47,7 @@ __device__ __forceinline__ double dd_val(dd2 a) { return a.hi + a.lo; }
 
 // deterministic block reduction (fixed shuffle tree)
 __device__ dd2 block_reduce(dd2 v) {
-    __shared__ dd2 sm[kBlock / 32];
+    __shared__ dd2 sm[32];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         dd2 w;
@@ -179,21 +179,102 @@ __global__ void k_restore(DevGeom g, LinkPlanes<double> backup, LinkPlanes<doubl
 }
 
 // ---------------------------------------------------------------- reductions
-template <typename T>
-__global__ void k_action_partials(DevGeom g, LinkPlanes<T> U, int with_rect, int block0, dd2* partial) {
+// One block per 32-site tile, one warp per plane: a site's loops are summed in
+// shared memory as plain doubles, the tile's sites as double-doubles.  partial[2 tile]
+// plaquettes, [2 tile + 1] rectangles.  Bound by load latency at the twelve warps per SM
+// that 168 registers allow; eight products per plane with the rectangles (thirteen
+// when each loop was formed apart: 0.81 ms at 32^4).
+constexpr int kPlaneBlock = 6 * MAG_TILE;
+template <bool RECT>
+__global__ void __launch_bounds__(kPlaneBlock, 2) k_action_partials(DevGeom g, LinkPlanes<double> U, int tile0,
+                                                                    dd2* partial) {
+    __shared__ double sm[RECT ? 2 : 1][6][MAG_TILE];
+    __shared__ cplx<double> keep[RECT ? 6 : 1][9][MAG_TILE];
     ChainInfo ci;
     Site st;
-    dd2 p = {0.0, 0.0}, r = {0.0, 0.0};
-    const int blk = block0 + blockIdx.x;
-    if (locate(g, blk * blockDim.x + threadIdx.x, ci, st) && interior(ci, st)) {
-        p.hi = site_plaquette(U, ci, st);
-        if (with_rect) r.hi = site_rectangle(U, ci, st);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, tile = tile0 + blockIdx.x;
+    double pl = 0.0, re = 0.0;
+    if (locate(g, tile * MAG_TILE + lane, ci, st) && interior(ci, st)) {
+        const int p = w < 3 ? 0 : w < 5 ? 1 : 2, q = w < 3 ? w + 1 : w < 5 ? w - 1 : 3;
+        plane_loops<RECT>(
+            U, ci, st, p, q, pl, re,
+            [&](const mat3<double>& m) {
+#pragma unroll
+                for (int k = 0; k < 9; k++) keep[RECT ? w : 0][k][lane] = m.e[k / 3][k % 3];
+            },
+            [&]() {
+                mat3<double> m;
+#pragma unroll
+                for (int k = 0; k < 9; k++) m.e[k / 3][k % 3] = keep[RECT ? w : 0][k][lane];
+                return m;
+            });
     }
-    p = block_reduce(p);
-    r = block_reduce(r);
-    if (threadIdx.x == 0) {
-        partial[2 * blk] = p;
-        partial[2 * blk + 1] = r;
+    sm[0][w][lane] = pl;
+    if (RECT) sm[RECT ? 1 : 0][w][lane] = re;
+    __syncthreads();
+    if (w < (RECT ? 2 : 1)) {
+        double s = sm[w][0][lane];
+#pragma unroll
+        for (int k = 1; k < 6; k++) s += sm[w][k][lane];
+        dd2 v = {s, 0.0};
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            dd2 r;
+            r.hi = __shfl_down_sync(0xffffffffu, v.hi, o);
+            r.lo = __shfl_down_sync(0xffffffffu, v.lo, o);
+            v = dd_add(v, r);
+        }
+        if (lane == 0) partial[2 * tile + w] = v;
+    }
+}
+
+// The same partials, bit for bit, with one thread per site (the planes in the same order)
+template <bool RECT>
+__global__ void __launch_bounds__(128, 3) k_action_sites(DevGeom g, LinkPlanes<double> U, int tile0, int ntile,
+                                                         dd2* partial) {
+    __shared__ cplx<double> keep[RECT ? 9 : 1][128];
+    ChainInfo ci;
+    Site st;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x * 4 + w, tile = tile0 + t;
+    double pl = 0.0, re = 0.0;
+    if (t < ntile && locate(g, tile * MAG_TILE + lane, ci, st) && interior(ci, st)) {
+#pragma unroll 1
+        for (int k = 0; k < 6; k++) {
+            const int p = k < 3 ? 0 : k < 5 ? 1 : 2, q = k < 3 ? k + 1 : k < 5 ? k - 1 : 3;
+            double a, b = 0.0;
+            plane_loops<RECT>(
+                U, ci, st, p, q, a, b,
+                [&](const mat3<double>& m) {
+#pragma unroll
+                    for (int j = 0; j < 9; j++) keep[RECT ? j : 0][threadIdx.x] = m.e[j / 3][j % 3];
+                },
+                [&]() {
+                    mat3<double> m;
+#pragma unroll
+                    for (int j = 0; j < 9; j++) m.e[j / 3][j % 3] = keep[RECT ? j : 0][threadIdx.x];
+                    return m;
+                });
+            pl = k ? pl + a : a;
+            re = k ? re + b : b;
+        }
+    }
+    if (t >= ntile) return;
+    dd2 v = {pl, 0.0}, r = {re, 0.0};
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        dd2 x;
+        x.hi = __shfl_down_sync(0xffffffffu, v.hi, o);
+        x.lo = __shfl_down_sync(0xffffffffu, v.lo, o);
+        v = dd_add(v, x);
+        if (RECT) {
+            x.hi = __shfl_down_sync(0xffffffffu, r.hi, o);
+            x.lo = __shfl_down_sync(0xffffffffu, r.lo, o);
+            r = dd_add(r, x);
+        }
+    }
+    if (lane == 0) {
+        partial[2 * tile] = v;
+        if (RECT) partial[2 * tile + 1] = r;
     }
 }
 
@@ -216,7 +297,6 @@ __global__ void k_kinetic_partials(DevGeom g, AlgPlanes<double> P, int block0, d
     if (threadIdx.x == 0) partial[2 * blk] = k;
 }
 
-// per chain: sum the partials of its blocks in block order
 // sum over mu of ReTr U(x, mu) (avg_real_trace, field-matrix.h:391-405)
 __global__ void k_link_trace_partials(DevGeom g, LinkPlanes<double> U, dd2* partial) {
     ChainInfo ci;
@@ -231,16 +311,22 @@ __global__ void k_link_trace_partials(DevGeom g, LinkPlanes<double> U, dd2* part
     k = block_reduce(k);
     if (threadIdx.x == 0) partial[2 * blockIdx.x] = k;
 }
-__global__ void k_finalize(DevGeom g, const dd2* partial, int chain0, int nq, dd2* sums, int slot0, double scale0) {
-    const int c = chain0 + blockIdx.x;
+// sums[chain][slot] = scale times the sum of the chain's partials (2 b + q for its units of
+// `unit` sites, q = blockIdx.y going to slot0 or slot1), also to host[slot] when given
+__global__ void k_finalize(DevGeom g, const dd2* partial, int unit, int chain0, dd2* sums, int slot0, int slot1,
+                           double scale, dd2* host) {
+    const int c = chain0 + blockIdx.x, q = blockIdx.y;
     const ChainInfo ci = g.chains[c];
-    const int b0 = ci.off / kBlock, b1 = (ci.off + ci.V + kBlock - 1) / kBlock;
-    for (int q = 0; q < nq; q++) {
-        dd2 v = {0.0, 0.0};
-        for (int b = b0 + threadIdx.x; b < b1; b += blockDim.x) v = dd_add(v, partial[2 * b + q]);
-        v = block_reduce(v);
-        if (threadIdx.x == 0) sums[c * NUM_SLOTS + slot0 + q] = q == 0 ? dd_mul(v, scale0) : v;
-        __syncthreads();
+    const int b0 = ci.off / unit, b1 = (ci.off + ci.V + unit - 1) / unit;
+    dd2 v = {0.0, 0.0};
+#pragma unroll 4
+    for (int b = b0 + threadIdx.x; b < b1; b += blockDim.x) v = dd_add(v, partial[2 * b + q]);
+    v = block_reduce(v);
+    if (threadIdx.x == 0) {
+        const int slot = q ? slot1 : slot0;
+        v = dd_mul(v, scale);
+        sums[c * NUM_SLOTS + slot] = v;
+        if (host) host[slot] = v;
     }
 }
 
@@ -533,39 +619,48 @@ void launch_restore_rejected(const DevGeom& g, LinkPlanes<double> backup, LinkPl
 }
 
 namespace {
-// blocks and chains of a reduction over the whole geometry or one chain
+// units (tiles or blocks of `unit` sites) and chains of a reduction over the whole geometry or one chain
 struct SumRange {
-    int block0, nblocks, chain0, nchains;
+    int unit, first, count, chain0, nchains;
+    dd2* host;
 };
-SumRange sum_range(const DevGeom& g, const ChainInfo* only, int chain) {
-    if (!only) return SumRange{0, (int)blocks(g), 0, g.nchain};
-    return SumRange{only->off / kBlock, (only->V + kBlock - 1) / kBlock, chain, 1};
+SumRange sum_range(const DevGeom& g, int unit, const OneChain* only) {
+    if (!only) return SumRange{unit, 0, (int)((g.vpad + unit - 1) / unit), 0, g.nchain, nullptr};
+    const ChainInfo& ci = *only->info;
+    return SumRange{unit, ci.off / unit, (ci.V + unit - 1) / unit, only->chain, 1, only->host};
+}
+void finalize(const DevGeom& g, const SumRange& r, const dd2* partial, int nq, dd2* sums, int slot0, int slot1,
+              double scale, cudaStream_t s) {
+    // enough threads that each adds a few tens of partials
+    k_finalize<<<dim3(r.nchains, nq), r.count > 4096 ? 1024 : kBlock, 0, s>>>(g, partial, r.unit, r.chain0, sums, slot0,
+                                                                             slot1, scale, r.host);
 }
 }  // namespace
 
-template <typename T>
-void launch_action_sums(const DevGeom& g, LinkPlanes<T> U, bool with_rect, dd2* partial, dd2* sums, int slot_plaq,
-                        int slot_rect, cudaStream_t s, const ChainInfo* only, int chain) {
-    const SumRange r = sum_range(g, only, chain);
-    k_action_partials<T><<<r.nblocks, kBlock, 0, s>>>(g, U, with_rect ? 1 : 0, r.block0, partial);
-    k_finalize<<<r.nchains, kBlock, 0, s>>>(g, partial, r.chain0, 1, sums, slot_plaq, 1.0);
-    if (with_rect) k_finalize<<<r.nchains, kBlock, 0, s>>>(g, partial + 1, r.chain0, 1, sums, slot_rect, 1.0);
+void launch_action_sums(const DevGeom& g, LinkPlanes<double> U, bool with_rect, dd2* partial, dd2* sums,
+                        int slot_plaq, int slot_rect, cudaStream_t s, const OneChain* only) {
+    const SumRange r = sum_range(g, MAG_TILE, only);
+    // a thread per site once the sites alone fill the GPU: 16^3 x 32 0.103 against 0.109 ms with
+    // rectangles and 16^4 0.037 against 0.040 without, 32^4 0.69 against 0.80 and 0.27 against 0.35;
+    // below, a warp per plane: 16^4 0.055 against 0.062, 8^4 0.0126 against 0.026
+    if (r.count >= (with_rect ? 3072 : 1536)) {
+        if (with_rect) k_action_sites<true><<<(r.count + 3) / 4, 128, 0, s>>>(g, U, r.first, r.count, partial);
+        else k_action_sites<false><<<(r.count + 3) / 4, 128, 0, s>>>(g, U, r.first, r.count, partial);
+    } else if (with_rect) k_action_partials<true><<<r.count, kPlaneBlock, 0, s>>>(g, U, r.first, partial);
+    else k_action_partials<false><<<r.count, kPlaneBlock, 0, s>>>(g, U, r.first, partial);
+    finalize(g, r, partial, with_rect ? 2 : 1, sums, slot_plaq, slot_rect, 1.0, s);
 }
-template void launch_action_sums<double>(const DevGeom&, LinkPlanes<double>, bool, dd2*, dd2*, int, int,
-                                         cudaStream_t, const ChainInfo*, int);
-template void launch_action_sums<float>(const DevGeom&, LinkPlanes<float>, bool, dd2*, dd2*, int, int,
-                                        cudaStream_t, const ChainInfo*, int);
 
 void launch_link_trace_sum(const DevGeom& g, LinkPlanes<double> U, dd2* partial, dd2* sums, int slot,
                            cudaStream_t s) {
     k_link_trace_partials<<<blocks(g), kBlock, 0, s>>>(g, U, partial);
-    k_finalize<<<g.nchain, kBlock, 0, s>>>(g, partial, 0, 1, sums, slot, 1.0);
+    finalize(g, sum_range(g, kBlock, nullptr), partial, 1, sums, slot, slot, 1.0, s);
 }
 void launch_kinetic_sum(const DevGeom& g, AlgPlanes<double> P, dd2* partial, dd2* sums, int slot, cudaStream_t s,
-                        const ChainInfo* only, int chain) {
-    const SumRange r = sum_range(g, only, chain);
-    k_kinetic_partials<<<r.nblocks, kBlock, 0, s>>>(g, P, r.block0, partial);
-    k_finalize<<<r.nchains, kBlock, 0, s>>>(g, partial, r.chain0, 1, sums, slot, 0.5);
+                        const OneChain* only) {
+    const SumRange r = sum_range(g, kBlock, only);
+    k_kinetic_partials<<<r.count, kBlock, 0, s>>>(g, P, r.first, partial);
+    finalize(g, r, partial, 1, sums, slot, slot, 0.5, s);
 }
 
 void launch_accept(const DevGeom& g, const AcceptArgs& a, dd2* sums, ChainState* st,

@@ -214,11 +214,12 @@ int mag_action(mag_ctx* ctx, int chain, double* plaq, double* rect, double* acti
     if (!ctx) return MAG_ERR_ARG;
     MAG_TRY(ctx->chain_ok(chain));
     LinkPlanes<double> top = ctx->smear64();
-    launch_action_sums<double>(ctx->geom, top, true, ctx->partial, ctx->sums, SLOT_PLAQ_THIN, SLOT_RECT_THIN,
-                               ctx->stream, &ctx->hc[chain], chain);
+    const OneChain one = ctx->one_chain(chain);
+    launch_action_sums(ctx->geom, top, true, ctx->partial, ctx->sums, SLOT_PLAQ_THIN, SLOT_RECT_THIN, ctx->stream,
+                       &one);
     MAG_TRY(ctx->check("mag_action"));
-    dd2 s[NUM_SLOTS];
-    MAG_TRY(ctx->read_sums(chain, s));
+    MAG_TRY(ctx->sync("sums"));
+    const dd2* s = one.host;
     const dd2 pl = s[SLOT_PLAQ_THIN], re = s[SLOT_RECT_THIN];
     if (plaq) *plaq = pl.hi + pl.lo;
     if (rect) *rect = re.hi + re.lo;
@@ -230,11 +231,12 @@ int mag_action(mag_ctx* ctx, int chain, double* plaq, double* rect, double* acti
 int mag_plaquette(mag_ctx* ctx, int chain, double* avg) {
     if (!ctx || !avg) return MAG_ERR_ARG;
     MAG_TRY(ctx->chain_ok(chain));
-    launch_action_sums<double>(ctx->geom, ctx->U, false, ctx->partial, ctx->sums, SLOT_SCRATCH, SLOT_SCRATCH,
-                               ctx->stream, &ctx->hc[chain], chain);
+    const OneChain one = ctx->one_chain(chain);
+    launch_action_sums(ctx->geom, ctx->U, false, ctx->partial, ctx->sums, SLOT_SCRATCH, SLOT_SCRATCH, ctx->stream,
+                       &one);
     MAG_TRY(ctx->check("mag_plaquette"));
-    dd2 s[NUM_SLOTS];
-    MAG_TRY(ctx->read_sums(chain, s));
+    MAG_TRY(ctx->sync("sums"));
+    const dd2* s = one.host;
     const dd2 pl = s[SLOT_SCRATCH];
     *avg = (pl.hi + pl.lo) / (18.0 * ctx->hc[chain].V);
     return MAG_OK;
@@ -243,11 +245,11 @@ int mag_plaquette(mag_ctx* ctx, int chain, double* avg) {
 int mag_kinetic(mag_ctx* ctx, int chain, double* kin) {
     if (!ctx || !kin) return MAG_ERR_ARG;
     MAG_TRY(ctx->chain_ok(chain));
-    launch_kinetic_sum(ctx->geom, ctx->P, ctx->partial, ctx->sums, SLOT_SCRATCH, ctx->stream, &ctx->hc[chain],
-                       chain);
+    const OneChain one = ctx->one_chain(chain);
+    launch_kinetic_sum(ctx->geom, ctx->P, ctx->partial, ctx->sums, SLOT_SCRATCH, ctx->stream, &one);
     MAG_TRY(ctx->check("mag_kinetic"));
-    dd2 s[NUM_SLOTS];
-    MAG_TRY(ctx->read_sums(chain, s));
+    MAG_TRY(ctx->sync("sums"));
+    const dd2* s = one.host;
     const dd2 k = s[SLOT_SCRATCH];
     *kin = k.hi + k.lo;
     return MAG_OK;
@@ -638,7 +640,7 @@ int mag_time_kernel(mag_ctx* ctx, const char* which, int reps, double* ms) {
             fn = [&]() { launch_links_to_payload(ctx->U, 0, c0.off, c0.V, ctx->staging, s); };
         } else if (w == "nersc_plaq") {  // the plaquette and link-trace sums of the import check
             fn = [&]() {
-                launch_action_sums<double>(g, ctx->U, false, ctx->partial, ctx->sums, SLOT_SCRATCH, SLOT_SCRATCH, s);
+                launch_action_sums(g, ctx->U, false, ctx->partial, ctx->sums, SLOT_SCRATCH, SLOT_SCRATCH, s);
                 launch_link_trace_sum(g, ctx->U, ctx->partial, ctx->sums, SLOT_SCRATCH2, s);
             };
         } else {
@@ -663,7 +665,7 @@ int mag_time_kernel(mag_ctx* ctx, const char* which, int reps, double* ms) {
         };
     } else if (w == "action") {
         fn = [&]() {
-            launch_action_sums<double>(g, ctx->U, true, ctx->partial, ctx->sums, SLOT_SCRATCH, SLOT_SCRATCH, s);
+            launch_action_sums(g, ctx->U, true, ctx->partial, ctx->sums, SLOT_SCRATCH, SLOT_SCRATCH, s);
         };
     } else {
         return fail(MAG_ERR_ARG, "mag_time_kernel: unknown kernel '" + w + "'");

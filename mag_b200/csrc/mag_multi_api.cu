@@ -70,7 +70,7 @@ struct mag_multi {
     int hamiltonian(hdd parts[3]) {
         launch_kinetic_sum(f->geom, f->P, f->partial, f->sums, SLOT_KIN_OLD, s());
         launch_kinetic_sum(c->geom, c->P, c->partial, c->sums, SLOT_KIN_OLD, s());
-        launch_action_sums<double>(f->geom, f->U, f->iwasaki, f->partial, f->sums, SLOT_PLAQ_OLD, SLOT_RECT_OLD, s());
+        launch_action_sums(f->geom, f->U, f->iwasaki, f->partial, f->sums, SLOT_PLAQ_OLD, SLOT_RECT_OLD, s());
         launch_multi_coarse(cf(), cc(), f->U, c->U, rho, eta_sqr, AlgPlanes<double>{nullptr, 0},
                             AlgPlanes<double>{nullptr, 0}, LinkPlanes<double>{nullptr, 0}, partial, energy, s());
         std::vector<dd2> sf(NUM_SLOTS), sc(NUM_SLOTS);

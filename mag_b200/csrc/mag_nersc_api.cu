@@ -66,8 +66,7 @@ namespace {
 
 // avg_plaquette (field-matrix.h:387-389) and avg_real_trace (:391-405) of one chain
 int plaq_and_trace(mag_ctx* ctx, int chain, double* plaq, double* trace) {
-    launch_action_sums<double>(ctx->geom, ctx->U, false, ctx->partial, ctx->sums, SLOT_SCRATCH, SLOT_SCRATCH,
-                               ctx->stream, &ctx->hc[chain], chain);
+    launch_action_sums(ctx->geom, ctx->U, false, ctx->partial, ctx->sums, SLOT_SCRATCH, SLOT_SCRATCH, ctx->stream);
     launch_link_trace_sum(ctx->geom, ctx->U, ctx->partial, ctx->sums, SLOT_SCRATCH2, ctx->stream);
     MAG_TRY(ctx->check("NERSC plaquette"));
     dd2 s[NUM_SLOTS];
