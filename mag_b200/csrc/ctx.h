@@ -431,9 +431,14 @@ struct mag_ctx {
     // Smeared links: the top level's force is the derivative with respect to the top
     // links in the Lie algebra (the force kernel, beta/3 included; everything after it
     // is linear), and each level maps it to the level below (kernels_smear.cu).
+    // With a kick the force goes straight into the momenta (Fout is scratch then).
     template <typename T>
-    void force_eval(LinkPlanes<T> Uin, AlgPlanes<T> Fout, StoutBufs<T>& b) {
-        if (gather[sizeof(T) == 8 ? 0 : 1]) return force_eval_gather(Uin, Fout, b);
+    void force_eval(LinkPlanes<T> Uin, AlgPlanes<T> Fout, StoutBufs<T>& b, const Kick* kick = nullptr) {
+        if (gather[sizeof(T) == 8 ? 0 : 1]) {
+            force_eval_gather(Uin, Fout, b);
+            if (kick) launch_kick<T>(geom, kick->P, Fout, kick->eps, stream);
+            return;
+        }
         const int L = p.n_stout;
         hx(Uin);
         LinkPlanes<T> cur = Uin;
@@ -442,21 +447,25 @@ struct mag_ctx {
             cur = b.lv[k];
             hx(cur);
         }
-        const AlgPlanes<T>* qtop = L ? &b.Q[L - 1] : nullptr;
         if (iwasaki) {
             launch_plaq_rect<T>(geom, cur, plaq_buf<T>(), b.loc, b.rem, stream);
-            launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, true, qtop, L ? b.lam : Fout, stream);
+            if (L) launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, true, b.Q[L - 1], b.lam, stream);
+            else launch_force_gather<T>(geom, Uin, b.loc, b.rem, b.dir, true, Fout, kick, stream);
         } else {
             launch_wilson_force<T>(geom, cur, b.rem, Fout, stream);
-            if (L) launch_lambda<T>(geom, *qtop, Fout, b.lam, b.dir, stream);
+            if (L) {
+                launch_lambda<T>(geom, b.Q[L - 1], Fout, b.lam, b.dir, stream);
+            } else {
+                if (any_mag) launch_constraint_fixup<T>(geom, Uin, Fout, stream);
+                if (kick) launch_kick<T>(geom, kick->P, Fout, kick->eps, stream);
+            }
         }
         for (int k = L - 1; k >= 0; k--) {
             hx(b.lam);
             launch_plaq_chain<T>(geom, k == 0 ? Uin : b.lv[k - 1], b.lam, b.loc, b.rem, stream);
-            launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, false, k ? &b.Q[k - 1] : nullptr, k ? b.lam : Fout,
-                                   stream);
+            if (k) launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, false, b.Q[k - 1], b.lam, stream);
+            else launch_force_gather<T>(geom, Uin, b.loc, b.rem, b.dir, false, Fout, kick, stream);
         }
-        if (any_mag) launch_constraint_fixup<T>(geom, Uin, Fout, stream);
     }
     // Smearing level k of `cur`.  FP64: over plaquettes (0.64 against 0.80 ms at 32^4 for the
     // one-thread-per-link kernel at its best shape).  FP32: one thread per link at 102
@@ -549,7 +558,7 @@ struct mag_ctx {
         if (w == "stout_level") forward_level(Uin, b, 0);
         else if (w == "lambda") launch_lambda<T>(geom, b.Q[0], Fo, b.lam, b.dir, stream);
         else if (w == "plaq_chain") launch_plaq_chain<T>(geom, Uin, b.lam, b.loc, b.rem, stream);
-        else if (w == "chain_gather") launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, false, &b.Q[0], b.lam, stream);
+        else if (w == "chain_gather") launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, false, b.Q[0], b.lam, stream);
         else if (iwasaki) launch_plaq_rect<T>(geom, Uin, plaq_buf<T>(), b.loc, b.rem, stream);
         else launch_wilson_force<T>(geom, Uin, b.rem, Fo, stream);
     }
@@ -667,8 +676,8 @@ struct mag_ctx {
         if (p.integrator == MAG_INT_LEAPFROG) {
             master(dt / 2.);
             for (int i = 0; i < p.n_steps; i++) {
-                force_eval<T>(Ut, Fw, b);
-                launch_kick<T>(geom, P, Fw, dt, stream);
+                const Kick kick{P, dt};
+                force_eval<T>(Ut, Fw, b, &kick);
                 master(i < p.n_steps - 1 ? dt : dt / 2.);
             }
             return;
@@ -679,8 +688,8 @@ struct mag_ctx {
         auto fg_kick = [&]() {
             force_eval<T>(Ut, Fw, b);
             launch_evolve<T, T>(geom, Ut, Ua, Fw, gamma, LinkPlanes<float>{nullptr, 0}, stream);
-            force_eval<T>(Ua, Fw, b);
-            launch_kick<T>(geom, P, Fw, 0.5 * dt, stream);
+            const Kick kick{P, 0.5 * dt};
+            force_eval<T>(Ua, Fw, b, &kick);
         };
         master(alpha);
         for (int i = 0; i < p.n_steps; i++) {

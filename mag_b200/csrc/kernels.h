@@ -111,11 +111,20 @@ void launch_lambda(const DevGeom& g, AlgPlanes<T> Q, AlgPlanes<T> X, AlgPlanes<T
 template <typename T>
 void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
                        cudaStream_t s);
-// x = Dir + Loc + the Rem terms that belong to a link (top: without Dir, times beta/3): Out = Lambda and Dir of the
-// level below with exponents *Q, or Out = x itself when Q is null (the thin links)
+// x = Dir + Loc + the Rem terms that belong to a link (top: without Dir, times beta/3): Lambda and Dir of
+// the level below, whose exponents are Q
 template <typename T>
 void launch_chain_gather(const DevGeom& g, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir, bool top,
-                         const AlgPlanes<T>* Q, AlgPlanes<T> Out, cudaStream_t s);
+                         AlgPlanes<T> Q, AlgPlanes<T> Lam, cudaStream_t s);
+// the same sum as the force of the thin links U, constrained segments included: into F, or, with a kick,
+// P += eps times it (F is then not written)
+struct Kick {
+    AlgPlanes<double> P;
+    double eps;
+};
+template <typename T>
+void launch_force_gather(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir,
+                         bool top, AlgPlanes<T> F, const Kick* kick, cudaStream_t s);
 // the plaquettes of U into Pl, then the Iwasaki force's plaquette and rectangle terms (without beta/3)
 // into Loc and Rem as launch_plaq_chain leaves them
 template <typename T>

@@ -308,16 +308,11 @@ __global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_chain(DevGeom g, Link
     if (ok) sm.sum_links(Loc, st.g, w, lane);
 }
 
-// x = Loc(x) + sum_nu Rem(x - nu), and Dir unless TOP: the derivative with respect to
-// a level's links (TOP: the gauge force of the top links, beta/3 times the sum); then Lambda and Dir of the
-// level below, or (LAST) the force itself
-template <typename T, bool TOP, bool LAST>
-__global__ void __launch_bounds__(kLinkBlock) k_chain_gather(DevGeom g, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
-                                                             AlgPlanes<T> Dir, AlgPlanes<T> Q, AlgPlanes<T> Out) {
-    ChainInfo ci;
-    Site st;
-    if (!locate_tile(g, ci, st)) return;
-    const int mu = threadIdx.x >> 5;
+// Loc(x) + sum_nu Rem(x - nu) (+ Dir unless TOP, times beta/3 if TOP): the derivative
+// with respect to a level's link (TOP: the gauge force of the top links)
+template <typename T, bool TOP>
+__device__ __forceinline__ herm8<T> gathered(const AlgPlanes<T>& Loc, const AlgPlanes<T>& Rem, const AlgPlanes<T>& Dir,
+                                             const ChainInfo& ci, const Site& st, int mu) {
     herm8<T> x = Loc.load(mu, st.g);
     if (!TOP) herm_add(x, Dir.load(mu, st.g));
     herm8<T> r[3];
@@ -329,13 +324,57 @@ __global__ void __launch_bounds__(kLinkBlock) k_chain_gather(DevGeom g, AlgPlane
 #pragma unroll
     for (int i = 0; i < 3; i++) herm_add(x, r[i]);
     if (TOP) x = scaled(x, (T)(ci.beta / 3.0));
-    if (LAST) {
-        Out.store(mu, st.g, x);
+    return x;
+}
+
+// Lambda and Dir of the level below from the gathered derivative
+template <typename T, bool TOP>
+__global__ void __launch_bounds__(kLinkBlock) k_chain_gather(DevGeom g, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
+                                                             AlgPlanes<T> Dir, AlgPlanes<T> Q, AlgPlanes<T> Lam) {
+    ChainInfo ci;
+    Site st;
+    if (!locate_tile(g, ci, st)) return;
+    const int mu = threadIdx.x >> 5;
+    const herm8<T> x = gathered<T, TOP>(Loc, Rem, Dir, ci, st, mu);
+    herm8<T> lam, dir;
+    lambda_adjoint(Q.load(mu, st.g), x, lam, dir);
+    Lam.store(mu, st.g, lam);
+    Dir.store(mu, st.g, dir);
+}
+
+// The force of the thin links.  Constrained segments (field-hmc.h:399-407): the last
+// link's force is zero, every other link's is F(x + mu) - U^dag F(x) U of the free-link
+// forces (the next link's is gathered again).  KICK: P += eps F (field-hmc.h:427-440)
+// without storing F.
+template <typename T, bool TOP, bool KICK>
+__global__ void __launch_bounds__(kLinkBlock) k_force_gather(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> Loc,
+                                                             AlgPlanes<T> Rem, AlgPlanes<T> Dir, AlgPlanes<T> F,
+                                                             AlgPlanes<double> P, double eps) {
+    ChainInfo ci;
+    Site st;
+    if (!locate_tile(g, ci, st)) return;
+    const int mu = threadIdx.x >> 5;
+    herm8<T> x = gathered<T, TOP>(Loc, Rem, Dir, ci, st, mu);
+    const int cc = constraint_case(ci, st, mu);
+    if (cc == 100) {
+        x = herm_zero<T>();
+    } else if (cc != 0) {
+        Site next = st;
+        next.g = nb_sel(ci, st, mu, 1);
+#pragma unroll
+        for (int d = 0; d < 4; d++)
+            if (d == mu) next.x[d] = st.x[d] + 1 < ci.L[d] ? st.x[d] + 1 : 0;
+        herm8<T> y = gathered<T, TOP>(Loc, Rem, Dir, ci, next, mu);
+        herm_sub(y, transport_dn(U.load(mu, st.g), x));
+        x = y;
+    }
+    if (KICK) {
+        herm8<double> p = P.load(mu, st.g);
+#pragma unroll
+        for (int k = 0; k < 8; k++) p.h[k] += (double)x.h[k] * eps;
+        P.store(mu, st.g, p);
     } else {
-        herm8<T> lam, dir;
-        lambda_adjoint(Q.load(mu, st.g), x, lam, dir);
-        Out.store(mu, st.g, lam);
-        Dir.store(mu, st.g, dir);
+        F.store(mu, st.g, x);
     }
 }
 
@@ -363,13 +402,20 @@ void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgP
 }
 template <typename T>
 void launch_chain_gather(const DevGeom& g, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir, bool top,
-                         const AlgPlanes<T>* Q, AlgPlanes<T> Out, cudaStream_t s) {
-    const AlgPlanes<T> q = Q ? *Q : AlgPlanes<T>{nullptr, 0};
-#define L_(TOP, LAST) k_chain_gather<T, TOP, LAST><<<tiles(g), kLinkBlock, 0, s>>>(g, Loc, Rem, Dir, q, Out)
-    if (top && Q) L_(true, false);
-    else if (top) L_(true, true);
-    else if (Q) L_(false, false);
-    else L_(false, true);
+                         AlgPlanes<T> Q, AlgPlanes<T> Lam, cudaStream_t s) {
+    if (top) k_chain_gather<T, true><<<tiles(g), kLinkBlock, 0, s>>>(g, Loc, Rem, Dir, Q, Lam);
+    else k_chain_gather<T, false><<<tiles(g), kLinkBlock, 0, s>>>(g, Loc, Rem, Dir, Q, Lam);
+}
+template <typename T>
+void launch_force_gather(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir,
+                         bool top, AlgPlanes<T> F, const Kick* kick, cudaStream_t s) {
+    const AlgPlanes<double> P = kick ? kick->P : AlgPlanes<double>{nullptr, 0};
+    const double eps = kick ? kick->eps : 0.0;
+#define L_(TOP, KICK) k_force_gather<T, TOP, KICK><<<tiles(g), kLinkBlock, 0, s>>>(g, U, Loc, Rem, Dir, F, P, eps)
+    if (top && kick) L_(true, true);
+    else if (top) L_(true, false);
+    else if (kick) L_(false, true);
+    else L_(false, false);
 #undef L_
 }
 template <typename T>
@@ -394,7 +440,9 @@ void launch_wilson_force(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> S, AlgP
     template void launch_plaq_chain<T>(const DevGeom&, LinkPlanes<T>, AlgPlanes<T>, AlgPlanes<T>, AlgPlanes<T>,     \
                                        cudaStream_t);                                                               \
     template void launch_chain_gather<T>(const DevGeom&, AlgPlanes<T>, AlgPlanes<T>, AlgPlanes<T>, bool,            \
-                                         const AlgPlanes<T>*, AlgPlanes<T>, cudaStream_t);                          \
+                                         AlgPlanes<T>, AlgPlanes<T>, cudaStream_t);                                 \
+    template void launch_force_gather<T>(const DevGeom&, LinkPlanes<T>, AlgPlanes<T>, AlgPlanes<T>, AlgPlanes<T>,   \
+                                         bool, AlgPlanes<T>, const Kick*, cudaStream_t);                            \
     template void launch_plaq_rect<T>(const DevGeom&, LinkPlanes<T>, RowPlanes<T>, AlgPlanes<T>, AlgPlanes<T>,      \
                                       cudaStream_t);                                                                \
     template void launch_wilson_force<T>(const DevGeom&, LinkPlanes<T>, AlgPlanes<T>, AlgPlanes<T>, cudaStream_t);

@@ -305,13 +305,9 @@ int mag_stout_force(mag_ctx* ctx, int chain, double* host_force_aos) {
 
 int mag_evolve_momentum(mag_ctx* ctx, double eps) {
     if (!ctx) return MAG_ERR_ARG;
-    if (ctx->mixed) {
-        ctx->force_eval<float>(ctx->U32, ctx->F32, ctx->st32);
-        launch_kick<float>(ctx->geom, ctx->P, ctx->F32, eps, ctx->stream);
-    } else {
-        ctx->force_eval<double>(ctx->U, ctx->F, ctx->st64);
-        launch_kick<double>(ctx->geom, ctx->P, ctx->F, eps, ctx->stream);
-    }
+    const Kick kick{ctx->P, eps};
+    if (ctx->mixed) ctx->force_eval<float>(ctx->U32, ctx->F32, ctx->st32, &kick);
+    else ctx->force_eval<double>(ctx->U, ctx->F, ctx->st64, &kick);
     return ctx->sync("mag_evolve_momentum");
 }
 
