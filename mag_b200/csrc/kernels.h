@@ -4,9 +4,45 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "lattice.cuh"
 
 namespace magb {
+
+// Launch of a kernel that begins with after_previous(): its blocks may be scheduled
+// while the kernel before it on the stream drains (programmatic stream serialisation),
+// which hides launch latency and block start-up; the data dependence is kept by the
+// wait in after_previous().  A kernel launched this way must call it in every block
+// before it touches memory, so that its completion implies its predecessors'.  A force
+// with three levels: 12^4 0.192 -> 0.161 ms, 16^3 x 32 0.866 -> 0.842, 24^4 and larger
+// unchanged.  Not while the stream is being captured: as graph edges the same
+// dependences made an 8^4 trajectory slower (0.82 -> 0.97 ms).
+template <typename... P, typename... A>
+inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(s, &capture);
+    at.val.programmaticStreamSerializationAllowed = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+}
+#if defined(__CUDACC__)
+// lets the next kernel's blocks in, then waits for the previous kernel and its writes
+__device__ __forceinline__ void after_previous() {
+#if defined(__CUDA_ARCH__)
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+#endif
+}
+#endif
 
 struct dd2 {
     double hi, lo;

@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(kForceBlock, MINB) k_staple_dagger(DevGeom g, 
 // One thread per coarse site handles the four directions.
 template <typename T>
 __global__ void k_constraint_fixup(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> F) {
+    after_previous();
     const int gs = blockIdx.x * blockDim.x + threadIdx.x;
     if (gs >= g.vpad) return;
     const ChainInfo ci = g.chains[g.c2c[gs / MAG_CHUNK]];
@@ -128,6 +129,7 @@ __global__ void k_constraint_fixup(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> F) {
 template <typename T, int MINB>
 __global__ void __launch_bounds__(kForceBlock, MINB) k_stout_forward(DevGeom g, LinkPlanes<T> Uin,
                                                                    LinkPlanes<T> Uout, AlgPlanes<T> Q) {
+    after_previous();
     ChainInfo ci;
     Site st;
     int mu;
@@ -391,12 +393,12 @@ void launch_staple_dagger(const DevGeom& g, LinkPlanes<T> U, LinkPlanes<T> W, Li
 }
 template <typename T>
 void launch_constraint_fixup(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> F, cudaStream_t s) {
-    k_constraint_fixup<T><<<(unsigned)((g.vpad + 255) / 256), 256, 0, s>>>(g, U, F);
+    launch_after(k_constraint_fixup<T>, (unsigned)((g.vpad + 255) / 256), 256, 0, s, g, U, F);
 }
 template <typename T>
 void launch_stout_forward(const DevGeom& g, LinkPlanes<T> Uin, LinkPlanes<T> Uout, AlgPlanes<T> Q, int v,
                           cudaStream_t s) {
-#define L_(M) k_stout_forward<T, M><<<link_blocks(g), kForceBlock, 0, s>>>(g, Uin, Uout, Q);
+#define L_(M) launch_after(k_stout_forward<T, M>, link_blocks(g), kForceBlock, 0, s, g, Uin, Uout, Q);
     MAG_BY_VARIANT(v, L_)
 #undef L_
 }

@@ -79,6 +79,7 @@ struct site_terms {
 // S = (P - P^dag) / 2i of every plaquette (plane fields 0..5 of S)
 template <typename T>
 __global__ void __launch_bounds__(kPlaqBlock, 4) k_plaq_sin(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S) {
+    after_previous();
     ChainInfo ci;
     Site st;
     if (!locate_tile(g, ci, st)) return;
@@ -112,6 +113,7 @@ __device__ __forceinline__ herm8<T> staple_angle(const LinkPlanes<T>& U, const A
 template <typename T>
 __global__ void __launch_bounds__(kLinkBlock, 5) k_stout_apply(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S,
                                                             LinkPlanes<T> Uout, AlgPlanes<T> Q) {
+    after_previous();
     ChainInfo ci;
     Site st;
     if (!locate_tile(g, ci, st)) return;
@@ -125,6 +127,7 @@ __global__ void __launch_bounds__(kLinkBlock, 5) k_stout_apply(DevGeom g, LinkPl
 template <typename T>
 __global__ void __launch_bounds__(kLinkBlock) k_wilson_force(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S,
                                                              AlgPlanes<T> F) {
+    after_previous();
     ChainInfo ci;
     Site st;
     if (!locate_tile(g, ci, st)) return;
@@ -135,6 +138,7 @@ __global__ void __launch_bounds__(kLinkBlock) k_wilson_force(DevGeom g, LinkPlan
 // rows 0, 1 of every plaquette (plane fields 0..5 of Pl)
 template <typename T>
 __global__ void __launch_bounds__(kPlaqBlock, sizeof(T) == 8 ? 2 : 4) k_plaq(DevGeom g, LinkPlanes<T> U, RowPlanes<T> Pl) {
+    after_previous();
     ChainInfo ci;
     Site st;
     if (!locate_tile(g, ci, st)) return;
@@ -165,6 +169,7 @@ __global__ void __launch_bounds__(kPlaqBlock, sizeof(T) == 8 ? 2 : 4) k_plaq(Dev
 template <typename T, int MINB>
 __global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_rect(DevGeom g, LinkPlanes<T> U, RowPlanes<T> Pl,
                                                                 AlgPlanes<T> Loc, AlgPlanes<T> Rem) {
+    after_previous();
     __shared__ site_terms<T> sm;
     ChainInfo ci;
     Site st;
@@ -236,6 +241,7 @@ __global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_rect(DevGeom g, LinkP
 template <typename T>
 __global__ void __launch_bounds__(kLinkBlock) k_lambda(DevGeom g, AlgPlanes<T> Q, AlgPlanes<T> X, AlgPlanes<T> Lam,
                                                        AlgPlanes<T> Dir) {
+    after_previous();
     ChainInfo ci;
     Site st;
     if (!locate_tile(g, ci, st)) return;
@@ -258,6 +264,7 @@ __global__ void __launch_bounds__(kLinkBlock) k_lambda(DevGeom g, AlgPlanes<T> Q
 template <typename T, int MINB>
 __global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_chain(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> Lam,
                                                                  AlgPlanes<T> Loc, AlgPlanes<T> Rem) {
+    after_previous();
     __shared__ site_terms<T> sm;
     ChainInfo ci;
     Site st;
@@ -331,6 +338,7 @@ __device__ __forceinline__ herm8<T> gathered(const AlgPlanes<T>& Loc, const AlgP
 template <typename T, bool TOP>
 __global__ void __launch_bounds__(kLinkBlock) k_chain_gather(DevGeom g, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
                                                              AlgPlanes<T> Dir, AlgPlanes<T> Q, AlgPlanes<T> Lam) {
+    after_previous();
     ChainInfo ci;
     Site st;
     if (!locate_tile(g, ci, st)) return;
@@ -350,6 +358,7 @@ template <typename T, bool TOP, bool KICK>
 __global__ void __launch_bounds__(kLinkBlock) k_force_gather(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> Loc,
                                                              AlgPlanes<T> Rem, AlgPlanes<T> Dir, AlgPlanes<T> F,
                                                              AlgPlanes<double> P, double eps) {
+    after_previous();
     ChainInfo ci;
     Site st;
     if (!locate_tile(g, ci, st)) return;
@@ -385,33 +394,33 @@ unsigned tiles(const DevGeom& g) { return (unsigned)(g.vpad / MAG_TILE); }
 template <typename T>
 void launch_stout_level(const DevGeom& g, LinkPlanes<T> U, LinkPlanes<T> Uout, AlgPlanes<T> Q, AlgPlanes<T> S,
                         cudaStream_t s) {
-    k_plaq_sin<T><<<tiles(g), kPlaqBlock, 0, s>>>(g, U, S);
-    k_stout_apply<T><<<tiles(g), kLinkBlock, 0, s>>>(g, U, S, Uout, Q);
+    launch_after(k_plaq_sin<T>, tiles(g), kPlaqBlock, 0, s, g, U, S);
+    launch_after(k_stout_apply<T>, tiles(g), kLinkBlock, 0, s, g, U, S, Uout, Q);
 }
 template <typename T>
 void launch_lambda(const DevGeom& g, AlgPlanes<T> Q, AlgPlanes<T> X, AlgPlanes<T> Lam, AlgPlanes<T> Dir,
                    cudaStream_t s) {
-    k_lambda<T><<<tiles(g), kLinkBlock, 0, s>>>(g, Q, X, Lam, Dir);
+    launch_after(k_lambda<T>, tiles(g), kLinkBlock, 0, s, g, Q, X, Lam, Dir);
 }
 template <typename T>
 void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
                        cudaStream_t s) {
     // blocks of six warps per SM: two of FP64 (168 registers, no spills; three would spill 1 KB:
     // 1.47 against 0.83 ms at 32^4), three of FP32 (96 registers; 0.369 against 0.431 ms)
-    k_plaq_chain<T, sizeof(T) == 8 ? 2 : 3><<<tiles(g), kPlaqBlock, 0, s>>>(g, U, Lam, Loc, Rem);
+    launch_after(k_plaq_chain<T, sizeof(T) == 8 ? 2 : 3>, tiles(g), kPlaqBlock, 0, s, g, U, Lam, Loc, Rem);
 }
 template <typename T>
 void launch_chain_gather(const DevGeom& g, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir, bool top,
                          AlgPlanes<T> Q, AlgPlanes<T> Lam, cudaStream_t s) {
-    if (top) k_chain_gather<T, true><<<tiles(g), kLinkBlock, 0, s>>>(g, Loc, Rem, Dir, Q, Lam);
-    else k_chain_gather<T, false><<<tiles(g), kLinkBlock, 0, s>>>(g, Loc, Rem, Dir, Q, Lam);
+    if (top) launch_after(k_chain_gather<T, true>, tiles(g), kLinkBlock, 0, s, g, Loc, Rem, Dir, Q, Lam);
+    else launch_after(k_chain_gather<T, false>, tiles(g), kLinkBlock, 0, s, g, Loc, Rem, Dir, Q, Lam);
 }
 template <typename T>
 void launch_force_gather(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir,
                          bool top, AlgPlanes<T> F, const Kick* kick, cudaStream_t s) {
     const AlgPlanes<double> P = kick ? kick->P : AlgPlanes<double>{nullptr, 0};
     const double eps = kick ? kick->eps : 0.0;
-#define L_(TOP, KICK) k_force_gather<T, TOP, KICK><<<tiles(g), kLinkBlock, 0, s>>>(g, U, Loc, Rem, Dir, F, P, eps)
+#define L_(TOP, KICK) launch_after(k_force_gather<T, TOP, KICK>, tiles(g), kLinkBlock, 0, s, g, U, Loc, Rem, Dir, F, P, eps)
     if (top && kick) L_(true, true);
     else if (top) L_(true, false);
     else if (kick) L_(false, true);
@@ -421,15 +430,15 @@ void launch_force_gather(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Loc, Al
 template <typename T>
 void launch_plaq_rect(const DevGeom& g, LinkPlanes<T> U, RowPlanes<T> Pl, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
                       cudaStream_t s) {
-    k_plaq<T><<<tiles(g), kPlaqBlock, 0, s>>>(g, U, Pl);
+    launch_after(k_plaq<T>, tiles(g), kPlaqBlock, 0, s, g, U, Pl);
     // two blocks of six warps per SM in both precisions (three: 0.81 against 0.75 ms FP32 at 32^4,
     // twice as slow in FP64, from spills)
-    k_plaq_rect<T, 2><<<tiles(g), kPlaqBlock, 0, s>>>(g, U, Pl, Loc, Rem);
+    launch_after(k_plaq_rect<T, 2>, tiles(g), kPlaqBlock, 0, s, g, U, Pl, Loc, Rem);
 }
 template <typename T>
 void launch_wilson_force(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> S, AlgPlanes<T> F, cudaStream_t s) {
-    k_plaq_sin<T><<<tiles(g), kPlaqBlock, 0, s>>>(g, U, S);
-    k_wilson_force<T><<<tiles(g), kLinkBlock, 0, s>>>(g, U, S, F);
+    launch_after(k_plaq_sin<T>, tiles(g), kPlaqBlock, 0, s, g, U, S);
+    launch_after(k_wilson_force<T>, tiles(g), kLinkBlock, 0, s, g, U, S, F);
 }
 
 #define MAG_INSTANTIATE(T)                                                                                          \

@@ -78,6 +78,7 @@ template <typename TU, typename TX>
 __global__ void __launch_bounds__(kBlock, 2) k_evolve(DevGeom g, LinkPlanes<TU> Uin, LinkPlanes<TU> Uout,
                                                       AlgPlanes<TX> X, double eps,
                          LinkPlanes<float> Ucopy) {
+    after_previous();
     ChainInfo ci;
     Site st;
     if (!locate(g, blockIdx.x * blockDim.x + threadIdx.x, ci, st)) return;
@@ -92,6 +93,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_evolve(DevGeom g, LinkPlanes<TU> 
 // P += eps F  (field-hmc.h:427-440)
 template <typename TF>
 __global__ void k_kick(DevGeom g, AlgPlanes<double> P, AlgPlanes<TF> F, double eps) {
+    after_previous();
     ChainInfo ci;
     Site st;
     if (!locate(g, blockIdx.x * blockDim.x + threadIdx.x, ci, st)) return;
@@ -188,6 +190,7 @@ constexpr int kPlaneBlock = 6 * MAG_TILE;
 template <bool RECT>
 __global__ void __launch_bounds__(kPlaneBlock, 2) k_action_partials(DevGeom g, LinkPlanes<double> U, int tile0,
                                                                     dd2* partial) {
+    after_previous();
     __shared__ double sm[RECT ? 2 : 1][6][MAG_TILE];
     __shared__ cplx<double> keep[RECT ? 6 : 1][9][MAG_TILE];
     ChainInfo ci;
@@ -232,6 +235,7 @@ __global__ void __launch_bounds__(kPlaneBlock, 2) k_action_partials(DevGeom g, L
 template <bool RECT>
 __global__ void __launch_bounds__(128, 3) k_action_sites(DevGeom g, LinkPlanes<double> U, int tile0, int ntile,
                                                          dd2* partial) {
+    after_previous();
     __shared__ cplx<double> keep[RECT ? 9 : 1][128];
     ChainInfo ci;
     Site st;
@@ -280,6 +284,7 @@ __global__ void __launch_bounds__(128, 3) k_action_sites(DevGeom g, LinkPlanes<d
 
 // kinetic energy sum of Re Tr(P^2), constrained-last links excluded (field-hmc.h:605-620)
 __global__ void k_kinetic_partials(DevGeom g, AlgPlanes<double> P, int block0, dd2* partial) {
+    after_previous();
     ChainInfo ci;
     Site st;
     dd2 k = {0.0, 0.0};
@@ -315,6 +320,7 @@ __global__ void k_link_trace_partials(DevGeom g, LinkPlanes<double> U, dd2* part
 // `unit` sites, q = blockIdx.y going to slot0 or slot1), also to host[slot] when given
 __global__ void k_finalize(DevGeom g, const dd2* partial, int unit, int chain0, dd2* sums, int slot0, int slot1,
                            double scale, dd2* host) {
+    after_previous();
     const int c = chain0 + blockIdx.x, q = blockIdx.y;
     const ChainInfo ci = g.chains[c];
     const int b0 = ci.off / unit, b1 = (ci.off + ci.V + unit - 1) / unit;
@@ -586,7 +592,7 @@ template void launch_fma_probe<double>(double*, int, int, cudaStream_t);
 template <typename TU, typename TX>
 void launch_evolve(const DevGeom& g, LinkPlanes<TU> Uin, LinkPlanes<TU> Uout, AlgPlanes<TX> X, double eps,
                    LinkPlanes<float> Ucopy, cudaStream_t s) {
-    k_evolve<TU, TX><<<dim3(blocks(g), 4), kBlock, 0, s>>>(g, Uin, Uout, X, eps, Ucopy);
+    launch_after(k_evolve<TU, TX>, dim3(blocks(g), 4), kBlock, 0, s, g, Uin, Uout, X, eps, Ucopy);
 }
 template void launch_evolve<double, double>(const DevGeom&, LinkPlanes<double>, LinkPlanes<double>,
                                             AlgPlanes<double>, double, LinkPlanes<float>, cudaStream_t);
@@ -597,7 +603,7 @@ template void launch_evolve<double, float>(const DevGeom&, LinkPlanes<double>, L
 
 template <typename TF>
 void launch_kick(const DevGeom& g, AlgPlanes<double> P, AlgPlanes<TF> F, double eps, cudaStream_t s) {
-    k_kick<TF><<<dim3(blocks(g), 4), kBlock, 0, s>>>(g, P, F, eps);
+    launch_after(k_kick<TF>, dim3(blocks(g), 4), kBlock, 0, s, g, P, F, eps);
 }
 template void launch_kick<double>(const DevGeom&, AlgPlanes<double>, AlgPlanes<double>, double, cudaStream_t);
 template void launch_kick<float>(const DevGeom&, AlgPlanes<double>, AlgPlanes<float>, double, cudaStream_t);
@@ -632,8 +638,8 @@ SumRange sum_range(const DevGeom& g, int unit, const OneChain* only) {
 void finalize(const DevGeom& g, const SumRange& r, const dd2* partial, int nq, dd2* sums, int slot0, int slot1,
               double scale, cudaStream_t s) {
     // enough threads that each adds a few tens of partials
-    k_finalize<<<dim3(r.nchains, nq), r.count > 4096 ? 1024 : kBlock, 0, s>>>(g, partial, r.unit, r.chain0, sums, slot0,
-                                                                             slot1, scale, r.host);
+    launch_after(k_finalize, dim3(r.nchains, nq), r.count > 4096 ? 1024 : kBlock, 0, s, g, partial, r.unit, r.chain0,
+                 sums, slot0, slot1, scale, r.host);
 }
 }  // namespace
 
@@ -644,10 +650,10 @@ void launch_action_sums(const DevGeom& g, LinkPlanes<double> U, bool with_rect, 
     // rectangles and 16^4 0.037 against 0.040 without, 32^4 0.69 against 0.80 and 0.27 against 0.35;
     // below, a warp per plane: 16^4 0.055 against 0.062, 8^4 0.0126 against 0.026
     if (r.count >= (with_rect ? 3072 : 1536)) {
-        if (with_rect) k_action_sites<true><<<(r.count + 3) / 4, 128, 0, s>>>(g, U, r.first, r.count, partial);
-        else k_action_sites<false><<<(r.count + 3) / 4, 128, 0, s>>>(g, U, r.first, r.count, partial);
-    } else if (with_rect) k_action_partials<true><<<r.count, kPlaneBlock, 0, s>>>(g, U, r.first, partial);
-    else k_action_partials<false><<<r.count, kPlaneBlock, 0, s>>>(g, U, r.first, partial);
+        if (with_rect) launch_after(k_action_sites<true>, (r.count + 3) / 4, 128, 0, s, g, U, r.first, r.count, partial);
+        else launch_after(k_action_sites<false>, (r.count + 3) / 4, 128, 0, s, g, U, r.first, r.count, partial);
+    } else if (with_rect) launch_after(k_action_partials<true>, r.count, kPlaneBlock, 0, s, g, U, r.first, partial);
+    else launch_after(k_action_partials<false>, r.count, kPlaneBlock, 0, s, g, U, r.first, partial);
     finalize(g, r, partial, with_rect ? 2 : 1, sums, slot_plaq, slot_rect, 1.0, s);
 }
 
@@ -659,7 +665,7 @@ void launch_link_trace_sum(const DevGeom& g, LinkPlanes<double> U, dd2* partial,
 void launch_kinetic_sum(const DevGeom& g, AlgPlanes<double> P, dd2* partial, dd2* sums, int slot, cudaStream_t s,
                         const OneChain* only) {
     const SumRange r = sum_range(g, kBlock, only);
-    k_kinetic_partials<<<r.count, kBlock, 0, s>>>(g, P, r.first, partial);
+    launch_after(k_kinetic_partials, r.count, kBlock, 0, s, g, P, r.first, partial);
     finalize(g, r, partial, 1, sums, slot, slot, 0.5, s);
 }
 

@@ -210,6 +210,7 @@ constexpr int kGaugeBlock = 64;
 __global__ void __launch_bounds__(kGaugeBlock) k_temporal_gauge(ChainInfo ci, LinkPlanes<double> U,
                                                                 LinkPlanes<double> G, LinkPlanes<double> P,
                                                                 int* bad) {
+    after_previous();
     const int vs = ci.L[0] * ci.L[1] * ci.L[2];
     const int x = blockIdx.x * kGaugeBlock + threadIdx.x;
     if (x >= vs) return;
@@ -230,6 +231,7 @@ __global__ void __launch_bounds__(kGaugeBlock) k_temporal_gauge(ChainInfo ci, Li
 // V_i(x) = G(x) U_i(x) G(x + i)^dag, the three spatial directions
 __global__ void __launch_bounds__(kBlock) k_gauge_links(ChainInfo ci, LinkPlanes<double> U, LinkPlanes<double> G,
                                                         LinkPlanes<double> V, int* bad) {
+    after_previous();
     const int s = blockIdx.x * kBlock + threadIdx.x, i = blockIdx.y;
     if (s >= ci.V) return;
     Site st;
@@ -254,6 +256,7 @@ constexpr int kGaugedBlocks = 592;  // per direction at most: four per SM
 template <int NX>
 __global__ void __maxnreg__(168) k_wloop_gauged(ChainInfo ci, LinkPlanes<double> V, LinkPlanes<double> P,
                                                       int Rmax, int Tmax, dd2* part) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char wsm[];
     cplx<double>* S = reinterpret_cast<cplx<double>*>(wsm);  // [Lt + Tmax][9][NX]
     __shared__ double red[8][kTChunk];
@@ -344,6 +347,7 @@ __global__ void __maxnreg__(168) k_wloop_gauged(ChainInfo ci, LinkPlanes<double>
 
 // out[(R-1) Tmax + T-1] = the sum over directions and blocks
 __global__ void k_wloop_gauged_sum(int nblk, int RT, const dd2* part, dd2* out) {
+    after_previous();
     dd2 v{0.0, 0.0};
     for (int i = 0; i < 3; i++)
         for (int b = threadIdx.x; b < nblk; b += blockDim.x)
@@ -384,7 +388,7 @@ static cudaError_t wloop_gauged(const ChainInfo& ci, LinkPlanes<double> V, LinkP
     const cudaError_t e =
         cudaFuncSetAttribute(k_wloop_gauged<NX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024);
     if (e != cudaSuccess) return e;
-    k_wloop_gauged<NX><<<dim3(gauged_blocks(ci, NX), 3), threads, smem, s>>>(ci, V, P, Rmax, Tmax, part);
+    launch_after(k_wloop_gauged<NX>, dim3(gauged_blocks(ci, NX), 3), threads, smem, s, ci, V, P, Rmax, Tmax, part);
     return cudaGetLastError();
 }
 
@@ -396,8 +400,8 @@ cudaError_t launch_wilson_gauged(const ChainInfo& ci, LinkPlanes<double> U, int 
                                  LinkPlanes<double> V, LinkPlanes<double> P, dd2* part, dd2* out, int* bad,
                                  cudaStream_t s) {
     const int nx = wilson_gauged_sites(ci, Tmax), vs = ci.L[0] * ci.L[1] * ci.L[2];
-    k_temporal_gauge<<<(vs + kGaugeBlock - 1) / kGaugeBlock, kGaugeBlock, 0, s>>>(ci, U, G, P, bad);
-    k_gauge_links<<<dim3((ci.V + kBlock - 1) / kBlock, 3), kBlock, 0, s>>>(ci, U, G, V, bad);
+    launch_after(k_temporal_gauge, (vs + kGaugeBlock - 1) / kGaugeBlock, kGaugeBlock, 0, s, ci, U, G, P, bad);
+    launch_after(k_gauge_links, dim3((ci.V + kBlock - 1) / kBlock, 3), kBlock, 0, s, ci, U, G, V, bad);
     cudaError_t e = cudaErrorInvalidValue;
     switch (nx) {
         case 32: e = wloop_gauged<32>(ci, V, P, Rmax, Tmax, part, s); break;
@@ -409,7 +413,7 @@ cudaError_t launch_wilson_gauged(const ChainInfo& ci, LinkPlanes<double> U, int 
         default: return e;
     }
     if (e != cudaSuccess) return e;
-    k_wloop_gauged_sum<<<Rmax * Tmax, kBlock, 0, s>>>(gauged_blocks(ci, nx), Rmax * Tmax, part, out);
+    launch_after(k_wloop_gauged_sum, Rmax * Tmax, kBlock, 0, s, gauged_blocks(ci, nx), Rmax * Tmax, part, out);
     return cudaGetLastError();
 }
 
