@@ -219,7 +219,19 @@ struct mag_ctx {
         stream = nullptr;
     }
 
+    // Fields that live as long as the context are carved out of one allocation (a cudaMalloc
+    // and its cudaFree cost 0.1-0.2 ms each): while `carve` is set, alloc() hands out
+    // pieces of arena (or only counts them, arena = null).
+    bool carve = false;
+    char* arena = nullptr;
+    size_t arena_used = 0;
+
     int alloc(void** ptr, size_t n) {
+        if (carve) {
+            *ptr = arena ? arena + arena_used : nullptr;
+            arena_used += (n + 255) / 256 * 256;
+            return MAG_OK;
+        }
         cudaError_t e = cudaMalloc(ptr, n);
         if (e != cudaSuccess) {
             cudaGetLastError();
@@ -247,20 +259,13 @@ struct mag_ctx {
             MAG_TRY(alloc_links(b.lv[k]));
             MAG_TRY(alloc_alg(b.Q[k]));
         }
-        // the algebra fields of the force in one allocation; a forward-only set needs the six
-        // plane fields of the smearing (in rem) and nothing else
-        AlgPlanes<T> all{nullptr, 0};
-        const int nlam = backward && p.n_stout > 0 ? 8 : 0;
-        const int planes = backward ? 16 + nlam : p.n_stout > 0 ? 6 : 0;
-        if (!planes) return MAG_OK;
-        MAG_TRY(alloc_alg(all, planes));
-        const size_t plane = 8 * (size_t)vpad;
-        b.rem = AlgPlanes<T>{all.p, vpad};
+        // a forward-only set needs the six plane fields of the smearing (in rem) and nothing else
+        if (backward || p.n_stout > 0) MAG_TRY(alloc_alg(b.rem, backward ? 12 : 6));
         if (!backward) return MAG_OK;
-        b.loc = AlgPlanes<T>{all.p + 12 * plane, vpad};
-        if (nlam) {
-            b.lam = AlgPlanes<T>{all.p + 16 * plane, vpad};
-            b.dir = AlgPlanes<T>{all.p + 20 * plane, vpad};
+        MAG_TRY(alloc_alg(b.loc));
+        if (p.n_stout > 0) {
+            MAG_TRY(alloc_alg(b.lam));
+            MAG_TRY(alloc_alg(b.dir));
         }
         return MAG_OK;
     }
@@ -274,6 +279,40 @@ struct mag_ctx {
         cudaError_t e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return fail(MAG_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
         return check(what);
+    }
+
+    int alloc_fields(int n, long nchunk) {
+        MAG_TRY(alloc((void**)&d_chains, sizeof(ChainInfo) * n));
+        MAG_TRY(alloc((void**)&d_c2c, sizeof(uint16_t) * nchunk));
+        MAG_TRY(alloc((void**)&d_stream_index, sizeof(unsigned long long) * n));
+        MAG_TRY(alloc_links(U));
+        MAG_TRY(alloc_links(Ubak));
+        MAG_TRY(alloc_alg(P));
+        if (mixed) {
+            MAG_TRY(alloc_links(U32));
+            MAG_TRY(alloc_links(Uaux32));
+            MAG_TRY(alloc_alg(F32));
+            MAG_TRY(alloc_stout(st32, true));
+            MAG_TRY(alloc_stout(st64, false));  // FP64 forward smearing for the Hamiltonian
+            if (iwasaki) MAG_TRY(alloc_links(W32));
+        } else {
+            MAG_TRY(alloc_links(Uaux));
+            MAG_TRY(alloc_alg(F));
+            MAG_TRY(alloc_stout(st64, true));
+            if (iwasaki) MAG_TRY(alloc_links(W64));
+        }
+        MAG_TRY(alloc((void**)&partial, sizeof(dd2) * 2 * (vpad / MAG_TILE)));
+        MAG_TRY(alloc((void**)&sums, sizeof(dd2) * NUM_SLOTS * n));
+        MAG_TRY(alloc((void**)&cstate, sizeof(ChainState) * n));
+        MAG_TRY(alloc((void**)&reunit, sizeof(unsigned long long) * n));
+        MAG_TRY(alloc((void**)&rec, sizeof(TrajRecord) * n));
+        MAG_TRY(alloc((void**)&hist, sizeof(TrajRecord) * n * kHistCap));
+        MAG_TRY(alloc((void**)&hist_base, sizeof(long long)));
+        MAG_TRY(alloc((void**)&traj_counter, sizeof(long long)));
+        MAG_TRY(alloc((void**)&tmp_counter, sizeof(long long)));
+        MAG_TRY(alloc((void**)&d_uniform, sizeof(double) * n));
+        MAG_TRY(alloc((void**)&staging, sizeof(double) * 72 * (size_t)max_v));
+        return MAG_OK;
     }
 
     // shard != nullptr: {nshards, rank, halo} of a lattice split along x3 (n == 1)
@@ -339,9 +378,15 @@ struct mag_ctx {
         MAG_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         MAG_CUDA(cudaEventCreate(&ev0));
         MAG_CUDA(cudaEventCreate(&ev1));
-        MAG_TRY(alloc((void**)&d_chains, sizeof(ChainInfo) * n));
         const long nchunk = vpad / MAG_CHUNK;
-        MAG_TRY(alloc((void**)&d_c2c, sizeof(uint16_t) * nchunk));
+        carve = true;
+        MAG_TRY(alloc_fields(n, nchunk));  // counts
+        carve = false;
+        MAG_TRY(alloc((void**)&arena, arena_used));
+        arena_used = 0;
+        carve = true;
+        MAG_TRY(alloc_fields(n, nchunk));
+        carve = false;
         std::vector<uint16_t> c2c(nchunk, 0);
         for (int c = 0; c < n; c++)
             for (long k = hc[c].off / MAG_CHUNK; k < (hc[c].off + hc[c].V + MAG_CHUNK - 1) / MAG_CHUNK; k++)
@@ -350,7 +395,6 @@ struct mag_ctx {
         // non-blocking stream would not wait for it); the sync at the end of init covers them
         MAG_CUDA(cudaMemcpyAsync(d_chains, hc.data(), sizeof(ChainInfo) * n, cudaMemcpyHostToDevice, stream));
         MAG_CUDA(cudaMemcpyAsync(d_c2c, c2c.data(), sizeof(uint16_t) * nchunk, cudaMemcpyHostToDevice, stream));
-        MAG_TRY(alloc((void**)&d_stream_index, sizeof(unsigned long long) * n));
         std::vector<unsigned long long> sidx(n);
         for (int c = 0; c < n; c++) sidx[c] = (unsigned long long)c;
         MAG_CUDA(cudaMemcpyAsync(d_stream_index, sidx.data(), sizeof(unsigned long long) * n,
@@ -358,35 +402,6 @@ struct mag_ctx {
         h_stream_index = sidx;
         geom = DevGeom{d_chains, d_c2c, vpad, n, d_stream_index, 0, 0, 0};
 
-        MAG_TRY(alloc_links(U));
-        MAG_TRY(alloc_links(Ubak));
-        MAG_TRY(alloc_alg(P));
-        if (mixed) {
-            MAG_TRY(alloc_links(U32));
-            MAG_TRY(alloc_links(Uaux32));
-            MAG_TRY(alloc_alg(F32));
-            MAG_TRY(alloc_stout(st32, true));
-            MAG_TRY(alloc_stout(st64, false));  // FP64 forward smearing for the Hamiltonian
-            MAG_TRY(alloc_alg(F));              // FP64 force for single-call API use
-            if (iwasaki) MAG_TRY(alloc_links(W32));
-        } else {
-            MAG_TRY(alloc_links(Uaux));
-            MAG_TRY(alloc_alg(F));
-            MAG_TRY(alloc_stout(st64, true));
-            if (iwasaki) MAG_TRY(alloc_links(W64));
-        }
-        MAG_TRY(alloc((void**)&partial, sizeof(dd2) * 2 * (vpad / MAG_TILE)));
-        MAG_CUDA(cudaHostAlloc((void**)&h_sums, sizeof(dd2) * NUM_SLOTS, cudaHostAllocMapped));
-        MAG_TRY(alloc((void**)&sums, sizeof(dd2) * NUM_SLOTS * n));
-        MAG_TRY(alloc((void**)&cstate, sizeof(ChainState) * n));
-        MAG_TRY(alloc((void**)&reunit, sizeof(unsigned long long) * n));
-        MAG_TRY(alloc((void**)&rec, sizeof(TrajRecord) * n));
-        MAG_TRY(alloc((void**)&hist, sizeof(TrajRecord) * n * kHistCap));
-        MAG_TRY(alloc((void**)&hist_base, sizeof(long long)));
-        MAG_TRY(alloc((void**)&traj_counter, sizeof(long long)));
-        MAG_TRY(alloc((void**)&tmp_counter, sizeof(long long)));
-        MAG_TRY(alloc((void**)&d_uniform, sizeof(double) * n));
-        MAG_TRY(alloc((void**)&staging, sizeof(double) * 72 * (size_t)max_v));
         MAG_CUDA(cudaMemsetAsync(cstate, 0, sizeof(ChainState) * n, stream));
         MAG_CUDA(cudaMemsetAsync(reunit, 0, sizeof(unsigned long long) * n, stream));
         MAG_CUDA(cudaMemsetAsync(traj_counter, 0, sizeof(long long), stream));
@@ -848,6 +863,10 @@ struct mag_ctx {
         return MAG_OK;
     }
 
+    int ensure_h_sums() {
+        if (!h_sums) MAG_CUDA(cudaHostAlloc((void**)&h_sums, sizeof(dd2) * NUM_SLOTS, cudaHostAllocMapped));
+        return MAG_OK;
+    }
     OneChain one_chain(int c) const { return OneChain{&hc[c], c, h_sums}; }
     // read a chain's double-double sums back to the host
     int read_sums(int chain, dd2 out[NUM_SLOTS]) {
