@@ -400,7 +400,7 @@ struct mag_ctx {
         MAG_CUDA(cudaMemcpyAsync(d_stream_index, sidx.data(), sizeof(unsigned long long) * n,
                                  cudaMemcpyHostToDevice, stream));
         h_stream_index = sidx;
-        geom = DevGeom{d_chains, d_c2c, vpad, n, d_stream_index, 0, 0, 0};
+        geom = DevGeom{d_chains, d_c2c, vpad, n, d_stream_index, 0, 0, 0, hc[0]};
 
         MAG_CUDA(cudaMemsetAsync(cstate, 0, sizeof(ChainState) * n, stream));
         MAG_CUDA(cudaMemsetAsync(reunit, 0, sizeof(unsigned long long) * n, stream));

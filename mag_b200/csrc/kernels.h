@@ -63,6 +63,7 @@ struct DevGeom {
     // tiles, rows of `gpr` blocks (x0 x1 = 128 gpr sites), L2 rows along x2.
     // Only the order changes: every link is computed as in raster order.
     int tile, gpr, L2;
+    ChainInfo one;             // the chain of a single lattice (kernel parameters: no dependent loads)
 };
 
 // Per-trajectory record kept on the device, one per chain per trajectory.

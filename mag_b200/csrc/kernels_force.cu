@@ -37,7 +37,7 @@ __device__ __forceinline__ bool locate_link(const DevGeom& g, ChainInfo& ci, Sit
     mu = blockIdx.x & 3;
     const int gs = block_site(g, blockIdx.x >> 2) + threadIdx.x;
     if (gs >= g.vpad) return false;
-    ci = g.chains[g.c2c[gs / MAG_CHUNK]];
+    ci = g.nchain == 1 ? g.one : g.chains[g.c2c[gs / MAG_CHUNK]];
     const int s = gs - ci.off;
     if (s >= ci.V) return false;
     decode(ci, s, st);

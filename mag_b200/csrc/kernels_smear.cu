@@ -35,7 +35,7 @@ __device__ __forceinline__ int plane_index(int i, int j) {
 
 __device__ __forceinline__ bool locate_tile(const DevGeom& g, ChainInfo& ci, Site& st) {
     const int gs = blockIdx.x * MAG_TILE + (threadIdx.x & 31);
-    ci = g.chains[g.c2c[gs / MAG_CHUNK]];
+    ci = g.nchain == 1 ? g.one : g.chains[g.c2c[gs / MAG_CHUNK]];
     const int s = gs - ci.off;
     if (s >= ci.V) return false;
     decode(ci, s, st);

@@ -14,7 +14,7 @@ constexpr int kBlock = 256;  // == MAG_CHUNK: a block never spans two chains
 
 __device__ __forceinline__ bool locate(const DevGeom& g, int gs, ChainInfo& ci, Site& st) {
     if (gs >= g.vpad) return false;
-    ci = g.chains[g.c2c[gs / MAG_CHUNK]];
+    ci = g.nchain == 1 ? g.one : g.chains[g.c2c[gs / MAG_CHUNK]];
     const int s = gs - ci.off;
     if (s >= ci.V) return false;
     decode(ci, s, st);
