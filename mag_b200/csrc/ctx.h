@@ -446,12 +446,22 @@ struct mag_ctx {
     // Smeared links: the top level's force is the derivative with respect to the top
     // links in the Lie algebra (the force kernel, beta/3 included; everything after it
     // is linear), and each level maps it to the level below (kernels_smear.cu).
-    // With a kick the force goes straight into the momenta (Fout is scratch then).
     template <typename T>
-    void force_eval(LinkPlanes<T> Uin, AlgPlanes<T> Fout, StoutBufs<T>& b, const Kick* kick = nullptr) {
+    void force_eval(LinkPlanes<T> Uin, AlgPlanes<T> Fout, StoutBufs<T>& b) {
+        force_use(Uin, ForceUse<T>::store(Fout), b);
+    }
+    // a stored force's use
+    template <typename T>
+    void apply_use(LinkPlanes<T> Uin, const ForceUse<T>& use) {
+        if (use.kind == ForceUse<T>::kKick) launch_kick<T>(geom, use.P, use.F, use.eps, stream);
+        else if (use.kind == ForceUse<T>::kEvolve)
+            launch_evolve<T, T>(geom, Uin, use.Uout, use.F, use.eps, LinkPlanes<float>{nullptr, 0}, stream);
+    }
+    template <typename T>
+    void force_use(LinkPlanes<T> Uin, const ForceUse<T>& use, StoutBufs<T>& b) {
         if (gather[sizeof(T) == 8 ? 0 : 1]) {
-            force_eval_gather(Uin, Fout, b);
-            if (kick) launch_kick<T>(geom, kick->P, Fout, kick->eps, stream);
+            force_eval_gather(Uin, use.F, b);
+            apply_use(Uin, use);
             return;
         }
         const int L = p.n_stout;
@@ -465,21 +475,21 @@ struct mag_ctx {
         if (iwasaki) {
             launch_plaq_rect<T>(geom, cur, plaq_buf<T>(), b.loc, b.rem, stream);
             if (L) launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, true, b.Q[L - 1], b.lam, stream);
-            else launch_force_gather<T>(geom, Uin, b.loc, b.rem, b.dir, true, Fout, kick, stream);
+            else launch_force_gather<T>(geom, Uin, b.loc, b.rem, b.dir, true, use, stream);
         } else {
-            launch_wilson_force<T>(geom, cur, b.rem, Fout, stream);
+            launch_wilson_force<T>(geom, cur, b.rem, use.F, stream);
             if (L) {
-                launch_lambda<T>(geom, b.Q[L - 1], Fout, b.lam, b.dir, stream);
+                launch_lambda<T>(geom, b.Q[L - 1], use.F, b.lam, b.dir, stream);
             } else {
-                if (any_mag) launch_constraint_fixup<T>(geom, Uin, Fout, stream);
-                if (kick) launch_kick<T>(geom, kick->P, Fout, kick->eps, stream);
+                if (any_mag) launch_constraint_fixup<T>(geom, Uin, use.F, stream);
+                apply_use(Uin, use);
             }
         }
         for (int k = L - 1; k >= 0; k--) {
             hx(b.lam);
             launch_plaq_chain<T>(geom, k == 0 ? Uin : b.lv[k - 1], b.lam, b.loc, b.rem, stream);
             if (k) launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, false, b.Q[k - 1], b.lam, stream);
-            else launch_force_gather<T>(geom, Uin, b.loc, b.rem, b.dir, false, Fout, kick, stream);
+            else launch_force_gather<T>(geom, Uin, b.loc, b.rem, b.dir, false, use, stream);
         }
     }
     // Smearing level k of `cur`.  FP64: over plaquettes (0.64 against 0.80 ms at 32^4 for the
@@ -691,8 +701,7 @@ struct mag_ctx {
         if (p.integrator == MAG_INT_LEAPFROG) {
             master(dt / 2.);
             for (int i = 0; i < p.n_steps; i++) {
-                const Kick kick{P, dt};
-                force_eval<T>(Ut, Fw, b, &kick);
+                force_use<T>(Ut, ForceUse<T>::kick(Fw, P, dt), b);
                 master(i < p.n_steps - 1 ? dt : dt / 2.);
             }
             return;
@@ -701,10 +710,8 @@ struct mag_ctx {
         const double beta = dt / std::sqrt(3.);
         const double gamma = (2. - std::sqrt(3.)) * dt * dt / 12.;
         auto fg_kick = [&]() {
-            force_eval<T>(Ut, Fw, b);
-            launch_evolve<T, T>(geom, Ut, Ua, Fw, gamma, LinkPlanes<float>{nullptr, 0}, stream);
-            const Kick kick{P, 0.5 * dt};
-            force_eval<T>(Ua, Fw, b, &kick);
+            force_use<T>(Ut, ForceUse<T>::evolve(Fw, gamma, Ua), b);
+            force_use<T>(Ua, ForceUse<T>::kick(Fw, P, 0.5 * dt), b);
         };
         master(alpha);
         for (int i = 0; i < p.n_steps; i++) {

@@ -307,17 +307,17 @@ MAG_HD void stout_lambda(const herm8<T>& q, const mat3<T>& Z, const mat3<T>& Ul,
 // force and step eps:  0: e^{i eps X(x)} U;  1: e^{i eps X(x-mu)} U e^{-i eps X(x)};
 // 10: U e^{-i eps X(x)};  100: e^{i eps X(x-mu)} U.  One exponential per link
 // (two for the interior links of a segment, case 1, which only mag >= 3 has),
-// evaluated at one call site in a loop so that it is inlined once.
-template <typename TU, typename TX>
-MAG_HD mat3<TU> evolve_link(const mat3<TU>& u, const AlgPlanes<TX>& X, double eps, int ccase, int g, int gm, int mu) {
+// evaluated at one call site in a loop so that it is inlined once.  X(previous): the
+// exponent of the link itself or of the one before it in its segment.
+template <typename TX, typename TU, typename F>
+MAG_HD mat3<TU> evolve_link(const mat3<TU>& u, double eps, int ccase, F X) {
     mat3<TU> r = u;
     const int nexp = ccase == 1 ? 2 : 1;
 #pragma unroll 1
     for (int k = 0; k < nexp; k++) {
         // left factor e^{i eps X(y)} (cases 0, 100, and 1 first) or right factor e^{-i eps X(x)} (10, 1 second)
         const bool right = ccase == 10 || k == 1;
-        const int y = (ccase == 100 || (ccase == 1 && k == 0)) ? gm : g;
-        const herm8<TX> xl = X.load(mu, y);
+        const herm8<TX> xl = X(ccase == 100 || (ccase == 1 && k == 0));
         const TU s = (TU)(right ? -eps : eps);
         herm8<TU> q;
 #pragma unroll

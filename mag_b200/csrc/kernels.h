@@ -153,15 +153,26 @@ void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgP
 template <typename T>
 void launch_chain_gather(const DevGeom& g, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir, bool top,
                          AlgPlanes<T> Q, AlgPlanes<T> Lam, cudaStream_t s);
-// the same sum as the force of the thin links U, constrained segments included: into F, or, with a kick,
-// P += eps times it (F is then not written)
-struct Kick {
+// What is done with the force of the thin links: stored in F, added to the momenta (P += eps F,
+// field-hmc.h:427-440) or the links moved by it (Uout = e^{i eps F} U with the constraint rules,
+// :497-503); F is scratch in the last two.
+template <typename T>
+struct ForceUse {
+    enum Kind { kStore, kKick, kEvolve } kind;
+    AlgPlanes<T> F;
     AlgPlanes<double> P;
     double eps;
+    LinkPlanes<T> Uout;
+    static ForceUse store(AlgPlanes<T> F) { return {kStore, F, {nullptr, 0}, 0.0, {nullptr, 0}}; }
+    static ForceUse kick(AlgPlanes<T> F, AlgPlanes<double> P, double eps) { return {kKick, F, P, eps, {nullptr, 0}}; }
+    static ForceUse evolve(AlgPlanes<T> F, double eps, LinkPlanes<T> Uout) {
+        return {kEvolve, F, {nullptr, 0}, eps, Uout};
+    }
 };
+// the same sum as the force of the thin links U, constrained segments included
 template <typename T>
 void launch_force_gather(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir,
-                         bool top, AlgPlanes<T> F, const Kick* kick, cudaStream_t s);
+                         bool top, const ForceUse<T>& use, cudaStream_t s);
 // the plaquettes of U into Pl, then the Iwasaki force's plaquette and rectangle terms (without beta/3)
 // into Loc and Rem as launch_plaq_chain leaves them
 template <typename T>

@@ -85,7 +85,8 @@ __global__ void __launch_bounds__(kBlock, 2) k_evolve(DevGeom g, LinkPlanes<TU> 
     const int mu = blockIdx.y;
     const int cc = constraint_case(ci, st, mu);
     const int gm = nb_sel(ci, st, mu, -1);
-    const mat3<TU> r = evolve_link<TU, TX>(Uin.load(mu, st.g), X, eps, cc, st.g, gm, mu);
+    const mat3<TU> r = evolve_link<TX>(Uin.load(mu, st.g), eps, cc,
+                                       [&](bool previous) { return X.load(mu, previous ? gm : st.g); });
     Uout.store(mu, st.g, r);
     if (Ucopy.p) Ucopy.store(mu, st.g, convert<float>(r));
 }

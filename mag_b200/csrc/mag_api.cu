@@ -308,9 +308,8 @@ int mag_stout_force(mag_ctx* ctx, int chain, double* host_force_aos) {
 
 int mag_evolve_momentum(mag_ctx* ctx, double eps) {
     if (!ctx) return MAG_ERR_ARG;
-    const Kick kick{ctx->P, eps};
-    if (ctx->mixed) ctx->force_eval<float>(ctx->U32, ctx->F32, ctx->st32, &kick);
-    else ctx->force_eval<double>(ctx->U, ctx->F, ctx->st64, &kick);
+    if (ctx->mixed) ctx->force_use<float>(ctx->U32, ForceUse<float>::kick(ctx->F32, ctx->P, eps), ctx->st32);
+    else ctx->force_use<double>(ctx->U, ForceUse<double>::kick(ctx->F, ctx->P, eps), ctx->st64);
     return ctx->sync("mag_evolve_momentum");
 }
 
