@@ -180,8 +180,11 @@ __global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_rect(DevGeom g, LinkP
         plane_of(w, p, q);
         const int ip = 3 * p + q - 1, iq = 3 * q + p;
         const T k0 = (T)ci.c0, k1 = (T)ci.c1;
-        // operands are loaded again for each use (L1) instead of staying in registers
-        auto fresh = []() { asm volatile("" ::: "memory"); };
+        // operands are loaded again for each use (L1) instead of staying in registers, unless
+        // the block has an SM's registers to itself
+        auto fresh = []() {
+            if (MINB > 1) asm volatile("" ::: "memory");
+        };
         herm8<T> lb, lc, t;
         {
             const int gm = nb_sel(ci, st, q, -1);
@@ -276,9 +279,10 @@ __global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_chain(DevGeom g, Link
         const int gp = nb_sel(ci, st, p, 1), gq = nb_sel(ci, st, q, 1);
         const int ip = 3 * p + q - 1, iq = 3 * q + p;
         // the thread's two slots hold A and D until y_a and y_d replace them
-        // a and d are loaded again (L1) for each use instead of staying in registers
+        // a and d are loaded again (L1) for each use instead of staying in registers, unless
+        // the block has an SM's registers to itself
         auto link = [&](int d) {
-            asm volatile("" ::: "memory");
+            if (MINB > 1) asm volatile("" ::: "memory");
             return U.load(d, st.g);
         };
         const mat3<T> P =
@@ -424,6 +428,10 @@ __global__ void __launch_bounds__(kLinkBlock, sizeof(T) == 8 ? 2 : 4) k_force_ev
                }));
 }
 
+// Up to one block per SM the FP64 plaquette kernels take the registers of two (the same
+// arithmetic; no reloads, no spills): 8^4 force with one level 0.042 -> 0.035 ms; with
+// more tiles than SMs two blocks per SM are faster (10 x 8^3: 0.0151 against 0.0158 ms).
+constexpr unsigned kSoloTiles = 148;
 unsigned tiles(const DevGeom& g) { return (unsigned)(g.vpad / MAG_TILE); }
 
 }  // namespace
@@ -444,7 +452,9 @@ void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgP
                        cudaStream_t s) {
     // blocks of six warps per SM: two of FP64 (168 registers, no spills; three would spill 1 KB:
     // 1.47 against 0.83 ms at 32^4), three of FP32 (96 registers; 0.369 against 0.431 ms)
-    launch_after(k_plaq_chain<T, sizeof(T) == 8 ? 2 : 3>, tiles(g), kPlaqBlock, 0, s, g, U, Lam, Loc, Rem);
+    if (sizeof(T) == 8 && tiles(g) <= kSoloTiles)
+        launch_after(k_plaq_chain<T, 1>, tiles(g), kPlaqBlock, 0, s, g, U, Lam, Loc, Rem);
+    else launch_after(k_plaq_chain<T, sizeof(T) == 8 ? 2 : 3>, tiles(g), kPlaqBlock, 0, s, g, U, Lam, Loc, Rem);
 }
 template <typename T>
 void launch_chain_gather(const DevGeom& g, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir, bool top,
@@ -475,7 +485,9 @@ void launch_plaq_rect(const DevGeom& g, LinkPlanes<T> U, RowPlanes<T> Pl, AlgPla
     launch_after(k_plaq<T>, tiles(g), kPlaqBlock, 0, s, g, U, Pl);
     // two blocks of six warps per SM in both precisions (three: 0.81 against 0.75 ms FP32 at 32^4,
     // twice as slow in FP64, from spills)
-    launch_after(k_plaq_rect<T, 2>, tiles(g), kPlaqBlock, 0, s, g, U, Pl, Loc, Rem);
+    if (sizeof(T) == 8 && tiles(g) <= kSoloTiles)
+        launch_after(k_plaq_rect<T, 1>, tiles(g), kPlaqBlock, 0, s, g, U, Pl, Loc, Rem);
+    else launch_after(k_plaq_rect<T, 2>, tiles(g), kPlaqBlock, 0, s, g, U, Pl, Loc, Rem);
 }
 template <typename T>
 void launch_wilson_force(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> S, AlgPlanes<T> F, cudaStream_t s) {

@@ -37,3 +37,16 @@ def test_zero_exponents_give_zero_lambda():
     U[:] = np.eye(3)
     U[37, 2] = O.gen_hot(dims, 5)[0, 0]
     _check(dims, U, "fp64", 1e-11, mag=0, n_stout=2, rho=0.1)
+
+
+@pytest.mark.parametrize("n_stout", [0, 2])
+def test_force_is_the_same_bits_alone_and_beside_a_larger_chain(n_stout):
+    """Up to 148 tiles (4736 sites) the FP64 plaquette kernels run one block per SM with more
+    registers: the same bits as in a larger context."""
+    dims = (8, 8, 8, 8)
+    U = O.gen_hot(dims, 13)
+    with M.Chmc(dims, mag=2, n_stout=n_stout) as s, \
+            M.Chmc(chains=[dict(dims=dims), dict(dims=(6, 6, 6, 4))], mag=2, n_stout=n_stout) as e:
+        s.set_gauge(U)
+        e.set_gauge(U, chain=0)
+        assert np.array_equal(s.get_force(), e.get_force(0))
