@@ -265,7 +265,7 @@ void launch_compute_lambda(const double* q, const double* sigma, const double* u
 
 // ---- per-link demon sweep (kernels_demon.cu)
 constexpr int kDemonPaths = 168;   // staple paths per link: 6 plaquette, 18 rectangle, 72 chair, 72 twist
-constexpr int kDemonWindow = 384;  // capacity of the per-site link window (353 used)
+constexpr int kDemonWindow = 384;  // capacity of the per-site link window (353 links)
 struct DemonState {
     double E[4];  // plaquette, rectangle, chair, twist demons
     long long accept, reject;
@@ -273,12 +273,20 @@ struct DemonState {
 // The staple paths of the four links of a site as steps through a window of links around the
 // site: packed[n] = site offset of slot n (4 bits per coordinate, biased by 4) | direction << 16
 // (direction 4: the unit matrix that pads the three-link plaquette paths); step i of path p of
-// the link in direction mu reads slot[mu][p][i], as the link (fwd = 1) or its adjoint (fwd = 0)
+// the link in direction mu reads slot[mu][p][i], as the link (fwd = 1) or its adjoint (fwd = 0).
+// late[mu][p] >= 0 counts the paths that contain the link updated just before; their steps up to
+// that link are replaced by the unit matrix, and first[mu][k] .. first[mu][k + 1] are those of
+// staple kind k.  The link is U_(mu-1)(x) itself for mu > 0; for mu = 0 it is the link of slot
+// uslot, after the one of lslot.
+constexpr int kDemonLate = 27;
 struct DemonTables {
-    int nslot;
+    int nslot, lslot, uslot;
+    uint8_t lfwd, ufwd;
     int packed[kDemonWindow];
     uint16_t slot[4][kDemonPaths][5];
     uint8_t fwd[4][kDemonPaths][5];
+    int8_t late[4][kDemonPaths];
+    int8_t first[4][5];
 };
 // false if the path set does not fit the window (cannot happen for the fixed path set)
 bool build_demon_tables(DemonTables* out);

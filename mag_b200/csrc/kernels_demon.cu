@@ -5,30 +5,50 @@
 // (x0 fastest, mu = 0..3 inner), each update seeing every earlier one, and four
 // global demons decide every hit: the sweep is sequential by definition.  One
 // CTA walks the links of one chain in that order (independent chains of an
-// ensemble run side by side, one CTA each) and parallelises inside a link:
+// ensemble run side by side, one CTA each).  What bounds it is the latency of
+// one link's work: the staple paths, their sums and the two hits.  The work of
+// neighbouring links overlaps as far as the order allows:
 //
-//  * window: the 353 distinct links that the 168 staple paths of the four links
-//    of a site touch are staged in shared memory, one window per site, with
-//    16-byte cp.async copies (32 consecutive pieces per instruction); the window
-//    of site s + 1 is staged in four parts while warp 0 runs the hits of site s,
-//    so the copies hide behind the hits.  The links of sites s and s - 1, which
-//    change after a window was staged, are read from three small site buffers
-//    that warp 0 keeps current;
-//  * paths: 168 threads multiply out one staple path each from the window (two
-//    rows of four products and a reconstructed third row; the three-link
-//    plaquette paths are padded with a unit slot so every thread runs the same
-//    instructions, and adjoints are formed by selects, not by a second product
-//    form);
-//  * sums: three lanes per component of each of the four staple sums;
-//  * hits: warp 0.  A proposal is an SU(2) subgroup element, so a hit's action
-//    change only needs the 2x2 block of v S on the subgroup's rows and columns,
-//    and the update only changes two rows of the link.  Lanes 0-3 evaluate the
-//    first hit for the four demons, lanes 4-11 the second hit after a rejected
-//    and after an accepted first hit, so both decisions follow one evaluation.
+//  * in stage l (one block barrier each) the path warps multiply out the 168
+//    staple paths of link l while one warp runs the hits of link l - 1, one
+//    prepares link l + 1's proposals and three stage links;
+//  * link l - 1 changes during stage l.  It enters the paths of link l only as
+//    the first step, U_(mu-1)(x) forward, of 27 paths (mu > 0) or the second
+//    step of one rectangle (mu = 0): those paths are multiplied out with the
+//    unit matrix in its place (and in place of the steps before it), and the
+//    hits of link l complete their sums with the link itself.  This holds when
+//    the offsets -2..2 are distinct sites, every extent >= 5; below that the
+//    same kernel runs the hits of l - 1 before the paths of l (8^3 x 4: 2.46 us
+//    per link, 6^4: 1.87);
+//  * a hit's action change is linear in the staple sum, ReTr(Y S) with
+//    Y = v - m v for the proposal m: the path warps contract each path with the
+//    three Y (first hit, second after a rejected or an accepted first) where
+//    they multiply it out, so that no staple sum is ever formed;
+//  * window: the 353 distinct links of the four links' paths, one window per
+//    site, staged for site s + 1 during the four stages of site s by 16-byte
+//    cp.async copies.  The links of sites s + 1, s and s - 1, which change after
+//    a window was staged, are read from small site buffers that the hits
+//    keep current;
+//  * paths: 24 threads in each of seven warps, a warp holding paths of one
+//    staple kind, so that a kind's sums end in its warps.  A thread multiplies
+//    two rows of four products and reconstructs the third; the three-link
+//    plaquette paths are padded with a unit slot and adjoints are formed by the
+//    loads' addresses, so every thread runs the same instructions.  The window's slots
+//    are numbered so that the eight threads that load together find their links
+//    in different bank groups.
+//
+// Measured, us per link: 3.21 with paths, sums and hits one after another behind
+// three barriers (6^4 and 8^3 x 4), now 1.87 and 2.46.  Of a stage's 3500 cycles
+// the products of a path take 2400 (two path warps share an SM quarter's FP64
+// pipe, 2.1 cycles per instruction), its contraction 600, the sum over eight
+// lanes 280; the hits take 2700 of them beside.  At most 12 warps: a thirteenth
+// would leave a thread 128 registers (2.1 us).
 #include <stdint.h>
 
+#include <algorithm>
 #include <cstring>
 #include <initializer_list>
+#include <utility>
 #include <vector>
 
 #include "kernels.h"
@@ -38,11 +58,17 @@ namespace magb {
 
 namespace {
 
-constexpr int kDemonThreads = 256;
+// one warp each for the proposals and the hits (the latter on the SM quarter with the
+// fewest path warps), kPathWarps of 24 threads with a path each, the rest stage links
+constexpr int kPrepareWarp = 0, kHitWarp = 1, kPathWarp0 = 2, kPathWarps = 7, kPathsPerWarp = 24;
+constexpr int kStageWarp0 = kPathWarp0 + kPathWarps, kStageWarps = 3;
+constexpr int kDemonThreads = 32 * (kStageWarp0 + kStageWarps);
 constexpr int kPaths = kDemonPaths;  // 6 + 18 + 72 + 72
+static_assert(kPaths == kPathWarps * kPathsPerWarp, "one thread per path");
 constexpr int kSteps = 5;
 constexpr size_t kLinkBytes = 144;  // 9 complex doubles
-constexpr size_t kDemonDynSmem = (2 * kDemonWindow + kPaths) * kLinkBytes;
+constexpr int kSiteLinks = 2 * kDemonWindow;  // the site buffers follow the two windows
+constexpr size_t kDemonDynSmem = (kSiteLinks + 16) * kLinkBytes;
 enum { RNG_DEMON_SU2 = 4, RNG_DEMON_SUBGROUP = 5 };
 
 __device__ __forceinline__ int wrap(int v, int L) { return v < 0 ? v + L : (v >= L ? v - L : v); }
@@ -92,25 +118,8 @@ __device__ __forceinline__ Su2 su2_of(double a0, double a1, double a2, double a3
 __device__ __forceinline__ cplx<double> pick(const cplx<double>& a, const cplx<double>& b, const cplx<double>& c, int r) {
     return r == 0 ? a : (r == 1 ? b : c);
 }
-// v <- m v when `apply`: rows i, j change
-__device__ __forceinline__ void apply_su2(mat3<double>& v, const Su2& m, bool apply) {
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        const cplx<double> vi = pick(v.e[0][c], v.e[1][c], v.e[2][c], m.i);
-        const cplx<double> vj = pick(v.e[0][c], v.e[1][c], v.e[2][c], m.j);
-        cplx<double> ni = cmul<false, false>(m.ii, vi);
-        cmac<false, false, false>(ni, m.ij, vj);
-        cplx<double> nj = cmul<false, false>(m.ji, vi);
-        cmac<false, false, false>(nj, m.jj, vj);
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-            if (apply && r == m.i) v.e[r][c] = ni;
-            if (apply && r == m.j) v.e[r][c] = nj;
-        }
-    }
-}
-// one column of v <- m v (the operations of apply_su2 on that column)
-__device__ __forceinline__ void apply_su2_col(cplx<double> col[3], const Su2& m, bool apply) {
+// one column of v <- m v: rows i, j change
+__device__ __forceinline__ void apply_su2_col(cplx<double> col[3], const Su2& m) {
     const cplx<double> vi = pick(col[0], col[1], col[2], m.i);
     const cplx<double> vj = pick(col[0], col[1], col[2], m.j);
     cplx<double> ni = cmul<false, false>(m.ii, vi);
@@ -119,59 +128,29 @@ __device__ __forceinline__ void apply_su2_col(cplx<double> col[3], const Su2& m,
     cmac<false, false, false>(nj, m.jj, vj);
 #pragma unroll
     for (int r = 0; r < 3; r++) {
-        if (apply && r == m.i) col[r] = ni;
-        if (apply && r == m.j) col[r] = nj;
+        if (r == m.i) col[r] = ni;
+        if (r == m.j) col[r] = nj;
     }
 }
-// ReTr(v S) - ReTr(m v S) (field-demon.h:75-78): only the 2x2 block of X = v S on rows and
-// columns i, j enters, the other diagonal elements of m X and X being equal
-__device__ __forceinline__ double delta_s(const mat3<double>& v, const mat3<double>& S, const Su2& m) {
-    cplx<double> vi[3], vj[3], si[3], sj[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        vi[c] = pick(v.e[0][c], v.e[1][c], v.e[2][c], m.i);
-        vj[c] = pick(v.e[0][c], v.e[1][c], v.e[2][c], m.j);
-        si[c] = pick(S.e[c][0], S.e[c][1], S.e[c][2], m.i);
-        sj[c] = pick(S.e[c][0], S.e[c][1], S.e[c][2], m.j);
-    }
-    cplx<double> xii = cmul<false, false>(vi[0], si[0]), xij = cmul<false, false>(vi[0], sj[0]);
-    cplx<double> xji = cmul<false, false>(vj[0], si[0]), xjj = cmul<false, false>(vj[0], sj[0]);
-#pragma unroll
-    for (int c = 1; c < 3; c++) {
-        cmac<false, false, false>(xii, vi[c], si[c]);
-        cmac<false, false, false>(xij, vi[c], sj[c]);
-        cmac<false, false, false>(xji, vj[c], si[c]);
-        cmac<false, false, false>(xjj, vj[c], sj[c]);
-    }
-    double d = xii.re + xjj.re;
-    d = fma(-m.ii.re, xii.re, d);
-    d = fma(m.ii.im, xii.im, d);
-    d = fma(-m.ij.re, xji.re, d);
-    d = fma(m.ij.im, xji.im, d);
-    d = fma(-m.ji.re, xij.re, d);
-    d = fma(m.ji.im, xij.im, d);
-    d = fma(-m.jj.re, xjj.re, d);
-    d = fma(m.jj.im, xjj.im, d);
-    return d;
-}
-
-// a staged link, or its adjoint (by selects: every lane runs the same product code)
+// a staged link, or its adjoint (by the addresses and signs: every lane runs the same product code)
 __device__ __forceinline__ mat3<double> load_oriented(const double2* q, bool fwd) {
-    mat3<double> m;
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-        const double2 v = q[k];
-        m.e[k / 3][k % 3] = mk(v.x, v.y);
-    }
+    const int sr = fwd ? 3 : 1, sc = fwd ? 1 : 3;
+    const long long flip = fwd ? 0 : (long long)0x8000000000000000ull;
     mat3<double> o;
 #pragma unroll
     for (int r = 0; r < 3; r++)
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            o.e[r][c].re = fwd ? m.e[r][c].re : m.e[c][r].re;
-            o.e[r][c].im = fwd ? m.e[r][c].im : -m.e[c][r].im;
+            const double2 v = q[r == c ? 4 * r : r * sr + c * sc];
+            o.e[r][c] = mk(v.x, __longlong_as_double(__double_as_longlong(v.y) ^ flip));
         }
     return o;
+}
+
+// element (r, c) of a staged link or of its adjoint
+__device__ __forceinline__ cplx<double> oriented(const double2* q, bool fwd, int r, int c) {
+    const double2 v = q[fwd ? 3 * r + c : 3 * c + r];
+    return mk(v.x, fwd ? v.y : -v.y);
 }
 
 __global__ void __launch_bounds__(kDemonThreads, 1) k_demon_sweep(const DemonJob* jobs, double2* aos,
@@ -181,38 +160,52 @@ __global__ void __launch_bounds__(kDemonThreads, 1) k_demon_sweep(const DemonJob
     double2* U = aos + jobs[blockIdx.x].aos_off;
     const unsigned long long seed = jobs[blockIdx.x].seed;
     DemonState* st = states + blockIdx.x;
-    extern __shared__ __align__(16) unsigned char dsm[];
-    double2* win = reinterpret_cast<double2*>(dsm);  // [2][kDemonWindow][9]: windows of sites s, s + 1
-    double(*prod)[18] = reinterpret_cast<double(*)[18]>(dsm + 2 * kDemonWindow * kLinkBytes);  // [kPaths][18]
-    __shared__ __align__(16) double2 sbuf[3][4][9];  // links of sites s - 1, s, s + 1 (index site % 3)
-    __shared__ double Ssum[4][18];                   // the four staple sums of the current link
-    __shared__ double hin_a[2][2][4];                // proposals of this and the next link
-    __shared__ int hin_sub[2][2];
-    __shared__ uint8_t redir[2][kDemonWindow];  // 0: window slot; 1 + d: link d of the window's site; 5 + d: of the site before
-    __shared__ uint16_t sslot[4][kPaths][kSteps];
-    __shared__ uint8_t sfwd[4][kPaths][kSteps];
+    // [2][kDemonWindow] windows of sites s and s + 1, [4][4] links of sites s - 2 .. s + 1 (site % 4)
+    extern __shared__ __align__(16) double2 links[];
+    auto site_link = [&](int s, int d) { return links + (kSiteLinks + 4 * (s & 3) + d) * 9; };
+    // by link % 3: the candidates v, m0 v, m1 v, m1 m0 v and the Y of the three action changes
+    __shared__ __align__(16) double2 cand[3][4][9];
+    __shared__ __align__(16) double2 ymat[3][3][9];
+    // by link % 2: the paths that wait for a link, the other paths' action changes by eight lanes
+    __shared__ __align__(16) double2 tail[2][kDemonLate][9];
+    __shared__ double psum[2][kPathWarps][4][3];
+    // hits: sums of the waiting paths by kind, Y times the link they wait for
+    __shared__ __align__(16) double2 late[4][9], lu[9], yu[2][3][9];
+    __shared__ double draw_a[2][4];
+    __shared__ int draw_sub[2];
+    __shared__ uint16_t loc[2][kDemonWindow];  // where a window slot's link is: index into `links`
+    // slots of the five steps, five bits of orientation, 1 + index into `tail`
+    __shared__ __align__(16) uint4 path[4][kPaths];
+    __shared__ int8_t sfirst[4][5];
     __shared__ int spk[kDemonWindow];
-    __shared__ int snslot;
-    for (int i = threadIdx.x; i < 4 * kPaths * kSteps; i += blockDim.x) {
-        (&sslot[0][0][0])[i] = (&tabs->slot[0][0][0])[i];
-        (&sfwd[0][0][0])[i] = (&tabs->fwd[0][0][0])[i];
+    for (int i = threadIdx.x; i < 4 * kPaths; i += blockDim.x) {
+        const uint16_t* sl = &tabs->slot[0][0][0] + kSteps * i;
+        const uint8_t* fw = &tabs->fwd[0][0][0] + kSteps * i;
+        uint32_t f = 0;
+        for (int k = 0; k < kSteps; k++) f |= (uint32_t)(fw[k] != 0) << k;
+        (&path[0][0])[i] = make_uint4(sl[0] | (uint32_t)sl[1] << 16, sl[2] | (uint32_t)sl[3] << 16, sl[4] | f << 16,
+                                      (uint32_t)(1 + (&tabs->late[0][0])[i]));
     }
+    if (threadIdx.x < 20) (&sfirst[0][0])[threadIdx.x] = (&tabs->first[0][0])[threadIdx.x];
     for (int i = threadIdx.x; i < kDemonWindow; i += blockDim.x) spk[i] = tabs->packed[i];
-    if (threadIdx.x == 0) snslot = tabs->nslot;
-    const int t = threadIdx.x, lane = t & 31;
-    double E[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) E[k] = st->E[k];
+    const int ns = tabs->nslot, lslot = tabs->lslot, uslot = tabs->uslot;
+    const bool lfwd = tabs->lfwd, ufwd = tabs->ufwd;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    double E = st->E[lane & 3];  // hits: demon lane % 4
     long long acc = 0, rej = 0;
     __syncthreads();
-    const int ns = snslot;
     const int nsite = ci.V;
+    // the offsets -2..2 are distinct sites: the paths of a link may run ahead of its predecessor's hits
+    const bool ahead = ci.L[0] >= 5 && ci.L[1] >= 5 && ci.L[2] >= 5 && ci.L[3] >= 5;
 
-    // Stage part `part` (0..3; -1: all) of site s's window into buffer wb with the threads
-    // [t0, t0 + nthr) (whole warps): lane k of a round forms the source of slot base + k, the
-    // round's 32 slots are then copied as 288 consecutive 16-byte pieces.  Part 0 also stages the
-    // site's own four links.  Slots holding a link of site s or of sprev are redirected.
-    auto stage_site = [&](int s, int wb, int part, int t0, int nthr, int sprev) {
+    // Stage part `part` (0..3; -1: all) of site s's window into buffer s % 2 with the nw warps from
+    // w0 on: lane k of a round forms the source of slot base + k, the round's 32 slots are then
+    // copied as 288 consecutive 16-byte pieces.  Part 0 also stages the site's own four links.
+    // Links of site s or of the two sites before it are read from the site buffers.  Each part
+    // first waits for the copies of the part before it, the last one for its own as well.
+    auto stage_site = [&](int s, int part, int w0, int nw) {
+        cp_wait_all();
+        const int wb = s & 1;
         int x[4];
         int r = s;
         x[0] = r % ci.L[0]; r /= ci.L[0];
@@ -220,20 +213,20 @@ __global__ void __launch_bounds__(kDemonThreads, 1) k_demon_sweep(const DemonJob
         x[2] = r % ci.L[2]; r /= ci.L[2];
         x[3] = r;
         const int n0 = part < 0 ? 0 : (ns * part) / 4, n1 = part < 0 ? ns : (ns * (part + 1)) / 4;
-        const int w = (t - t0) >> 5, nw = nthr >> 5;
+        const int w = warp - w0;
         if (part <= 0 && w == 0) {
-            cp16(&sbuf[s % 3][0][0] + lane, U + (size_t)s * 36 + lane);
-            if (lane < 4) cp16(&sbuf[s % 3][0][0] + 32 + lane, U + (size_t)s * 36 + 32 + lane);
+            cp16(site_link(s, 0) + lane, U + (size_t)s * 36 + lane);
+            if (lane < 4) cp16(site_link(s, 0) + 32 + lane, U + (size_t)s * 36 + 32 + lane);
         }
         for (int base = n0 + 32 * w; base < n1; base += 32 * nw) {
             const int n = base + lane;
-            long long src = -1;
+            int src = -1;  // link index; -1: nothing to copy
             if (n < n1) {
                 const int pk = spk[n];
                 const int d = pk >> 16;
+                int at = wb * kDemonWindow + n;
                 if (d >= 4) {
-                    redir[wb][n] = 0;
-                    double2* dst = win + ((size_t)wb * kDemonWindow + n) * 9;
+                    double2* dst = links + (size_t)at * 9;
 #pragma unroll
                     for (int j = 0; j < 9; j++) dst[j] = make_double2(j == 0 || j == 4 || j == 8 ? 1.0 : 0.0, 0.0);
                 } else {
@@ -241,164 +234,233 @@ __global__ void __launch_bounds__(kDemonThreads, 1) k_demon_sweep(const DemonJob
                                   wrap(x[1] + ((pk >> 4) & 15) - 4, ci.L[1]) * ci.stride[1] +
                                   wrap(x[2] + ((pk >> 8) & 15) - 4, ci.L[2]) * ci.stride[2] +
                                   wrap(x[3] + ((pk >> 12) & 15) - 4, ci.L[3]) * ci.stride[3];
-                    const int code = g == s ? 1 + d : (g == sprev ? 5 + d : 0);
-                    redir[wb][n] = (uint8_t)code;
-                    if (!code) src = ((long long)g * 4 + d) * 9;
+                    const int back = s - g;
+                    if (back >= 0 && back <= 2)
+                        at = kSiteLinks + 4 * (g & 3) + d;
+                    else
+                        src = g * 4 + d;
                 }
+                loc[wb][n] = (uint16_t)at;
             }
-            double2* dst0 = win + ((size_t)wb * kDemonWindow + base) * 9;
+            double2* dst0 = links + ((size_t)wb * kDemonWindow + base) * 9;
 #pragma unroll
             for (int rr = 0; rr < 9; rr++) {
                 const int f = rr * 32 + lane;
                 const int q = f / 9, j = f - 9 * q;
-                const long long a = __shfl_sync(0xffffffffu, src, q);
-                if (base + q < n1 && a >= 0) cp16(dst0 + f, U + a + j);
+                const int a = __shfl_sync(0xffffffffu, src, q);
+                if (a >= 0) cp16(dst0 + f, U + (size_t)a * 9 + j);
             }
         }
-        cp_wait_all();
+        if (part < 0 || part == 3) cp_wait_all();
     };
-
-    stage_site(0, 0, -1, 0, kDemonThreads, -1);
-    if (t < 2) {
-        double a[4];
-        int sub;
-        su2_draw(seed, 0u, (uint32_t)sweep, (uint32_t)t, a, sub);
-        for (int k = 0; k < 4; k++) hin_a[0][t][k] = a[k];
-        hin_sub[0][t] = sub;
-    }
-    __syncthreads();
-    const long nlink = 4L * ci.V;
-    for (long l = 0; l < nlink; l++) {
-        const int s = (int)(l >> 2), mu = (int)(l & 3);
-        const int wb = s & 1, hb = (int)(l & 1);
-        const int cs = s % 3, ps = (s + 2) % 3;
-        // 1. the 168 path products from the window; the last warp draws the next link's proposals
-        if (t < kPaths) {
-            const uint16_t* sl = sslot[mu][t];
-            const uint8_t* fw = sfwd[mu][t];
-            auto src = [&](int i) -> const double2* {
-                const int slot = sl[i];
-                const int code = redir[wb][slot];
-                if (code == 0) return win + ((size_t)wb * kDemonWindow + slot) * 9;
-                return &sbuf[code < 5 ? cs : ps][(code - 1) & 3][0];
-            };
-            mat3<double> m = load_oriented(src(0), fw[0]);
-#pragma unroll
-            for (int i = 1; i < kSteps; i++) m = mul_2r(m, load_oriented(src(i), fw[i]));
-            reconstruct_row2(m);
-#pragma unroll
-            for (int k = 0; k < 9; k++) {
-                prod[t][2 * k] = m.e[k / 3][k % 3].re;
-                prod[t][2 * k + 1] = m.e[k / 3][k % 3].im;
-            }
-        } else if (t >= kDemonThreads - 32 && lane < 2 && l + 1 < nlink) {
+    // proposals of link l (one warp): the two draws, the candidate links and Y = v - m0 v,
+    // v - m1 v, m0 v - m1 m0 v; v does not change before its own hits
+    auto prepare = [&](int l) {
+        if (lane < 2) {
             double a[4];
             int sub;
-            su2_draw(seed, (uint32_t)(l + 1), (uint32_t)sweep, (uint32_t)lane, a, sub);
+            su2_draw(seed, (uint32_t)l, (uint32_t)sweep, (uint32_t)lane, a, sub);
 #pragma unroll
-            for (int k = 0; k < 4; k++) hin_a[hb ^ 1][lane][k] = a[k];
-            hin_sub[hb ^ 1][lane] = sub;
+            for (int k = 0; k < 4; k++) draw_a[lane][k] = a[k];
+            draw_sub[lane] = sub;
         }
-        __syncthreads();
-        // 2. the four staple sums in path order, three lanes (a third of the paths each) per
-        //    component, 30 lanes per warp; plaquette and rectangle sums are daggered
-        //    (get_staple_dagger / get_rectangular_dagger), chair and twist are not
-        {
-            const int g = (t >> 5) * 10 + lane / 3, third = lane % 3;
-            double a = 0.0;
-            int cat = 0, comp = 0;
-            if (lane < 30 && g < 72) {
-                cat = g / 18;
-                comp = g % 18;
-                const int p0 = cat == 0 ? 0 : cat == 1 ? 6 : cat == 2 ? 24 : 96;
-                const int n = (cat == 0 ? 6 : cat == 1 ? 18 : 72) / 3;
-                const int e = comp >> 1, part = comp & 1;
-                const int srcc = cat < 2 ? 2 * ((e % 3) * 3 + e / 3) + part : comp;  // element (j, i) for the dagger
-                for (int p = p0 + third * n; p < p0 + (third + 1) * n; p++) a += prod[p][srcc];
+        __syncwarp();
+        if (lane < 9) {
+            const int r = lane / 3, c = lane % 3, b = l % 3;
+            const double(*a)[4] = draw_a;
+            const Su2 m0 = su2_of(a[0][0], a[0][1], a[0][2], a[0][3], draw_sub[0]);
+            const Su2 m1 = su2_of(a[1][0], a[1][1], a[1][2], a[1][3], draw_sub[1]);
+            cplx<double> v[3], v0[3], v1[3], v01[3];
+            const double2* vp = site_link(l >> 2, l & 3);
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const double2 q = vp[3 * k + c];
+                v[k] = v0[k] = v1[k] = mk(q.x, q.y);
             }
-            const int base = lane - third;
-            const double a1 = __shfl_sync(0xffffffffu, a, (base + 1) & 31);
-            const double a2 = __shfl_sync(0xffffffffu, a, (base + 2) & 31);
-            if (lane < 30 && g < 72 && third == 0) {
-                const double sum = (a + a1) + a2;
-                Ssum[cat][comp] = (cat < 2 && (comp & 1)) ? -sum : sum;
-            }
+            apply_su2_col(v0, m0);
+            apply_su2_col(v1, m1);
+#pragma unroll
+            for (int k = 0; k < 3; k++) v01[k] = v0[k];
+            apply_su2_col(v01, m1);
+            const cplx<double> e = pick(v[0], v[1], v[2], r), e0 = pick(v0[0], v0[1], v0[2], r);
+            const cplx<double> e1 = pick(v1[0], v1[1], v1[2], r), e01 = pick(v01[0], v01[1], v01[2], r);
+            cand[b][0][lane] = make_double2(e.re, e.im);
+            cand[b][1][lane] = make_double2(e0.re, e0.im);
+            cand[b][2][lane] = make_double2(e1.re, e1.im);
+            cand[b][3][lane] = make_double2(e01.re, e01.im);
+            ymat[b][0][lane] = make_double2(e.re - e0.re, e.im - e0.im);
+            ymat[b][1][lane] = make_double2(e.re - e1.re, e.im - e1.im);
+            ymat[b][2][lane] = make_double2(e0.re - e01.re, e0.im - e01.im);
         }
-        __syncthreads();
-        // 3. two hits (warp 0; lane 4G + k: demon k; G = 0 the first hit, G = 1 the second after a
-        //    rejected first, G = 2 the second after an accepted first); the other warps stage a
-        //    quarter of the next site's window
-        if (t < 32) {
-            mat3<double> v;
+        __syncwarp();
+    };
+    // the paths of link l (kPathWarps warps): ReTr(Y P) summed over the kind's paths, P daggered
+    // for plaquettes and rectangles (get_staple_dagger / get_rectangular_dagger) and not for
+    // chairs and twists; a path that waits for link l - 1 goes to `tail`
+    auto paths = [&](int l) {
+        const int mu = l & 3, w = warp - kPathWarp0;
+        // rectangles on lanes 0..17 and plaquettes on lanes 24..29 of the first warp, 24 chairs or
+        // twists in each of the others: eight lanes never hold two kinds
+        const int p = w > 0 ? w * kPathsPerWarp + lane : lane < 18 ? 6 + lane : lane - 24;
+        double a[3] = {0.0, 0.0, 0.0};
+        if (w > 0 ? lane < kPathsPerWarp : lane < 18 || (lane >= 24 && lane < 30)) {
+            const uint4 d = path[mu][p];
+            const uint16_t* at = loc[(l >> 2) & 1];
+            const double2* q[kSteps] = {links + at[d.x & 0xffff] * 9, links + at[d.x >> 16] * 9,
+                                        links + at[d.y & 0xffff] * 9, links + at[d.y >> 16] * 9,
+                                        links + at[d.z & 0xffff] * 9};
+            mat3<double> m = load_oriented(q[0], d.z & 0x10000u);
 #pragma unroll
-            for (int c = 0; c < 9; c++) {
-                const double2 q = sbuf[cs][mu][c];
-                v.e[c / 3][c % 3] = mk(q.x, q.y);
-            }
-            const int G = lane < 12 ? lane >> 2 : 0, k = lane & 3;
-            mat3<double> S;
+            for (int i = 1; i < kSteps; i++) m = mul_2r(m, load_oriented(q[i], d.z & (0x10000u << i)));
+            reconstruct_row2(m);
+            if (d.w) {
+                double2* o = tail[l & 1][d.w - 1];
 #pragma unroll
-            for (int c = 0; c < 9; c++) S.e[c / 3][c % 3] = mk(Ssum[k][2 * c], Ssum[k][2 * c + 1]);
-            const Su2 m0 = su2_of(hin_a[hb][0][0], hin_a[hb][0][1], hin_a[hb][0][2], hin_a[hb][0][3], hin_sub[hb][0]);
-            const Su2 m1 = su2_of(hin_a[hb][1][0], hin_a[hb][1][1], hin_a[hb][1][2], hin_a[hb][1][3], hin_sub[hb][1]);
-            mat3<double> vs = v;
-            apply_su2(vs, m0, G == 2);
-            const double dS = delta_s(vs, S, G == 0 ? m0 : m1);
-            double d0[4], d1r[4], d1a[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                d0[q] = __shfl_sync(0xffffffffu, dS, q);
-                d1r[q] = __shfl_sync(0xffffffffu, dS, 4 + q);
-                d1a[q] = __shfl_sync(0xffffffffu, dS, 8 + q);
-            }
-            bool ok0 = true;
-#pragma unroll
-            for (int q = 0; q < 4; q++) ok0 = ok0 && E[q] - d0[q] > -e_max && E[q] - d0[q] < e_max;
-            if (ok0) {
-#pragma unroll
-                for (int q = 0; q < 4; q++) E[q] -= d0[q];
-                acc++;
+                for (int k = 0; k < 9; k++) o[k] = make_double2(m.e[k / 3][k % 3].re, m.e[k / 3][k % 3].im);
             } else {
-                rej++;
-            }
-            bool ok1 = true;
+                double acc[3][3] = {};
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const double d = ok0 ? d1a[q] : d1r[q];
-                ok1 = ok1 && E[q] - d > -e_max && E[q] - d < e_max;
-            }
-            if (ok1) {
+                for (int k = 0; k < 9; k++) {
+                    cplx<double> e;
+                    e.re = w == 0 ? m.e[k / 3][k % 3].re : m.e[k % 3][k / 3].re;
+                    e.im = w == 0 ? m.e[k / 3][k % 3].im : -m.e[k % 3][k / 3].im;
 #pragma unroll
-                for (int q = 0; q < 4; q++) E[q] -= ok0 ? d1a[q] : d1r[q];
-                acc++;
-            } else {
-                rej++;
-            }
-            // the updated link, one element per lane 0..8: column c of v through both decisions
-            {
-                const int e = lane < 9 ? lane : 0, r = e / 3, cc = e % 3;
-                cplx<double> col[3];
-#pragma unroll
-                for (int k = 0; k < 3; k++) col[k] = pick(v.e[k][0], v.e[k][1], v.e[k][2], cc);
-                apply_su2_col(col, m0, ok0);
-                apply_su2_col(col, m1, ok1);
-                const cplx<double> o = pick(col[0], col[1], col[2], r);
-                if (lane < 9) {
-                    const double2 q = make_double2(o.re, o.im);
-                    sbuf[cs][mu][lane] = q;
-                    U[((size_t)s * 4 + mu) * 9 + lane] = q;
+                    for (int G = 0; G < 3; G++) {
+                        const double2 y = ymat[l % 3][G][k];
+                        acc[G][k % 3] = fma(y.y, e.im, fma(y.x, e.re, acc[G][k % 3]));
+                    }
                 }
+#pragma unroll
+                for (int G = 0; G < 3; G++) a[G] = (acc[G][0] + acc[G][1]) + acc[G][2];
             }
-        } else if (s + 1 < nsite) {
-            stage_site(s + 1, wb ^ 1, mu, 32, kDemonThreads - 32, s);
         }
+#pragma unroll
+        for (int o = 4; o; o >>= 1)
+#pragma unroll
+            for (int G = 0; G < 3; G++) a[G] += __shfl_xor_sync(0xffffffffu, a[G], o);
+        if ((lane & 7) == 0)
+#pragma unroll
+            for (int G = 0; G < 3; G++) psum[l & 1][w][lane >> 3][G] = a[G];
+    };
+    // the two hits of link l (one warp)
+    auto hits = [&](int l) {
+        const int s = l >> 2, mu = l & 3, b = l % 3;
+        // sums R of the waiting paths by kind: lanes 0..26 an element of rectangles, chairs or
+        // twists each, then lanes 0..8 of the one plaquette
+        {
+            const int k = 1 + lane / 9, e = lane % 9;
+            cplx<double> R[3];
+#pragma unroll
+            for (int x = 0; x < 3; x++) R[x] = mk(0.0, 0.0);
+            if (lane < 27) {
+                const int f0 = sfirst[mu][k], f1 = sfirst[mu][k + 1];
+#pragma unroll
+                for (int i = 0; i < 12; i++)
+                    if (f0 + i < f1) {
+                        const double2 v = tail[l & 1][f0 + i][e];
+                        R[i % 3].re += v.x;
+                        R[i % 3].im += v.y;
+                    }
+                late[k][e] = make_double2((R[0].re + R[1].re) + R[2].re, (R[0].im + R[1].im) + R[2].im);
+            }
+            if (lane < 9) late[0][lane] = sfirst[mu][1] > 0 ? tail[l & 1][0][lane] : make_double2(0.0, 0.0);
+        }
+        // the link they wait for, u: U_(mu-1)(x), or the rectangle's first two links when mu = 0
+        const double2* u = site_link(s, (mu + 3) & 3);
+        if (mu == 0) {
+            const double2* lp = links + loc[s & 1][lslot] * 9;
+            const double2* up = links + loc[s & 1][uslot] * 9;
+            if (lane < 9) {
+                cplx<double> o = mk(0.0, 0.0);
+#pragma unroll
+                for (int x = 0; x < 3; x++)
+                    cmac<false, false, false>(o, oriented(lp, lfwd, lane / 3, x), oriented(up, ufwd, x, lane % 3));
+                lu[lane] = make_double2(o.re, o.im);
+            }
+            u = lu;
+            __syncwarp();
+        }
+        // u^+ Y for the daggered kinds, Y u for the others
+#pragma unroll
+        for (int round = 0; round < 2; round++) {
+            const int j = lane + 32 * round;
+            if (j < 54) {
+                const int h = j / 27, G = (j % 27) / 9, r = (j % 9) / 3, c = j % 3;
+                const double2* y = ymat[b][G];
+                const double2* pa = h ? y + 3 * r : u + r;
+                const double2* pb = h ? u + c : y + c;
+                cplx<double> o = mk(0.0, 0.0);
+#pragma unroll
+                for (int x = 0; x < 3; x++) {
+                    const double2 va = pa[h ? x : 3 * x], vb = pb[3 * x];
+                    cmac<false, false, false>(o, mk(va.x, h ? va.y : -va.y), mk(vb.x, vb.y));
+                }
+                yu[h][G][3 * r + c] = make_double2(o.re, o.im);
+            }
+        }
+        __syncwarp();
+        // lane 4 G + k: demon k; G = 0 the first hit, G = 1 the second after a rejected first,
+        // G = 2 the second after an accepted first (ReTr(v S) - ReTr(m v S), field-demon.h:75-78)
+        const int G = lane < 12 ? lane >> 2 : 0, k = lane & 3;
+        double d[3] = {0.0, 0.0, 0.0}, rest[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int e = 0; e < 9; e++) {
+            const double2 y = yu[k >> 1][G][e];
+            const double2 v = late[k][k < 2 ? e : 3 * (e % 3) + e / 3];
+            d[e % 3] = fma(y.x, v.x, d[e % 3]);
+            d[e % 3] = fma(k < 2 ? y.y : -y.y, v.y, d[e % 3]);
+        }
+        // eight-lane sums: 3 of the first warp are rectangles, its fourth the plaquettes; chairs
+        // and twists have three warps each
+        const double(*ps)[4][3] = psum[l & 1] + (k < 2 ? 0 : 3 * k - 5);
+#pragma unroll
+        for (int i = 0; i < 9; i++)
+            if (k >= 2 || (k == 1 && i < 3)) rest[i % 3] += ps[i / 3][i % 3][G];
+        if (k == 0) rest[0] = ps[0][3][G];
+        const double dS = ((rest[0] + rest[1]) + rest[2]) + ((d[0] + d[1]) + d[2]);
+        const double first = E - __shfl_sync(0xffffffffu, dS, k);  // the demon after an accepted first hit
+        const double after = (G == 2 ? first : E) - dS;
+        const unsigned in = __ballot_sync(0xffffffffu, after > -e_max && after < e_max);
+        const bool ok0 = (in & 0xfu) == 0xfu;
+        const bool ok1 = ((in >> (ok0 ? 8 : 4)) & 0xfu) == 0xfu;
+        const double moved = __shfl_sync(0xffffffffu, after, k + (ok1 ? (ok0 ? 8 : 4) : 0));
+        if (ok0 || ok1) {
+            E = moved;
+            if (lane < 9) {
+                const double2 o = cand[b][(ok0 ? 1 : 0) + (ok1 ? 2 : 0)][lane];
+                site_link(s, mu)[lane] = o;
+                U[((size_t)s * 4 + mu) * 9 + lane] = o;
+            }
+        }
+        acc += (ok0 ? 1 : 0) + (ok1 ? 1 : 0);
+        rej += (ok0 ? 0 : 1) + (ok1 ? 0 : 1);
+        __syncwarp();
+    };
+
+    stage_site(0, -1, 0, kDemonThreads / 32);
+    __syncthreads();
+    const int nlink = 4 * nsite;
+    if (warp == kPrepareWarp) prepare(0);
+    __syncthreads();
+    for (int l = 0; l <= nlink; l++) {
+        if (warp == kHitWarp) {
+            if (l > 0) hits(l - 1);
+        } else if (warp == kPrepareWarp) {
+            if (l + 1 < nlink) prepare(l + 1);
+        } else if (warp >= kStageWarp0) {
+            const int s = (l >> 2) + 1;
+            if (s < nsite) stage_site(s, l & 3, kStageWarp0, kStageWarps);
+        }
+        if (!ahead) __syncthreads();
+        if (warp >= kPathWarp0 && warp < kStageWarp0 && l < nlink) paths(l);
         __syncthreads();
     }
-    if (t == 0) {
-#pragma unroll
-        for (int k = 0; k < 4; k++) st->E[k] = E[k];
-        st->accept += acc;
-        st->reject += rej;
+    if (warp == kHitWarp && lane < 4) {
+        st->E[lane] = E;
+        if (lane == 0) {
+            st->accept += acc;
+            st->reject += rej;
+        }
     }
 }
 
@@ -458,10 +520,10 @@ bool build_demon_tables(DemonTables* T) {
     std::memset(T, 0, sizeof(*T));
     int8_t paths[4][kPaths][kSteps];
     demon_paths(paths);
-    // window slots: the distinct (site offset, direction) pairs over the four directions, plus
-    // the unit matrix (direction 4) that pads the three-link paths
+    // the distinct (site offset, direction) pairs over the four directions, and the unit matrix
+    // (direction 4) that pads the three-link paths
     std::vector<int> keys;
-    auto slot_of = [&](const int y[4], int d) {
+    auto key_of = [&](const int y[4], int d) {
         const int key = ((y[0] + 4) & 15) | (((y[1] + 4) & 15) << 4) | (((y[2] + 4) & 15) << 8) |
                         (((y[3] + 4) & 15) << 12) | (d << 16);
         for (size_t k = 0; k < keys.size(); k++)
@@ -469,30 +531,113 @@ bool build_demon_tables(DemonTables* T) {
         keys.push_back(key);
         return (int)keys.size() - 1;
     };
-    for (int mu = 0; mu < 4; mu++)
+    const int zero[4] = {0, 0, 0, 0}, before[4] = {-1, 0, 0, 0};
+    const int unit = key_of(zero, 4);
+    int lkey = -1, ukey = -1;
+    for (int mu = 0; mu < 4; mu++) {
+        // the link updated before this one, and the step at which paths meet it
+        const int prev = mu > 0 ? key_of(zero, mu - 1) : key_of(before, 3), meets = mu > 0 ? 0 : 1;
+        int n = 0;
         for (int p = 0; p < kPaths; p++) {
-            int y[4] = {0, 0, 0, 0};
+            if (p == 0 || p == 6 || p == 24 || p == 96) T->first[mu][p == 0 ? 0 : p == 6 ? 1 : p == 24 ? 2 : 3] = (int8_t)n;
+            int y[4] = {0, 0, 0, 0}, key[kSteps];
+            T->late[mu][p] = -1;
             for (int i = 0; i < kSteps; i++) {
                 const int d = paths[mu][p][i];
-                int sl;
-                if (d < 0) {
-                    const int z[4] = {0, 0, 0, 0};
-                    sl = slot_of(z, 4);
-                    T->fwd[mu][p][i] = 1;
-                } else {
-                    const int a = d & 3;
-                    if (d >= 4) y[a]--;
-                    if (y[a] < -2 || y[a] > 2) return false;
-                    sl = slot_of(y, a);
-                    T->fwd[mu][p][i] = d < 4;
-                    if (d < 4) y[a]++;
+                T->fwd[mu][p][i] = d < 4;
+                key[i] = unit;
+                if (d < 0) continue;
+                const int a = d & 3;
+                if (d >= 4) y[a]--;
+                if (y[a] < -2 || y[a] > 2) return false;
+                key[i] = key_of(y, a);
+                if (d < 4) y[a]++;
+                if (key[i] == prev) {
+                    if (i != meets || T->late[mu][p] >= 0 || n >= kDemonLate) return false;
+                    T->late[mu][p] = (int8_t)n++;
                 }
-                if (sl >= kDemonWindow) return false;
-                T->slot[mu][p][i] = (uint16_t)sl;
             }
+            if (T->late[mu][p] >= 0) {
+                if (mu == 0) {
+                    if (n > 1 || p < 6 || p >= 24) return false;
+                    lkey = key[0];
+                    T->lfwd = T->fwd[mu][p][0];
+                    ukey = key[1];
+                    T->ufwd = T->fwd[mu][p][1];
+                } else if (!T->fwd[mu][p][0]) {
+                    return false;
+                }
+                for (int i = 0; i <= meets; i++) {
+                    key[i] = unit;
+                    T->fwd[mu][p][i] = 1;
+                }
+            }
+            for (int i = 0; i < kSteps; i++) T->slot[mu][p][i] = (uint16_t)key[i];
         }
-    T->nslot = (int)keys.size();
-    for (int k = 0; k < T->nslot; k++) T->packed[k] = keys[k];
+        T->first[mu][4] = (int8_t)n;
+    }
+    // Slots: 16-byte loads are served for eight threads at a time, and the bank group of element e
+    // of a link is (slot + e) % 8; two links that a group reads the same way meet in all nine
+    // elements when their slots agree modulo 8, a link and an adjoint (element 3 c + r against
+    // 3 r + c) in three of them, and in two when the slots differ by 2, 4 or 6.  Greedy choice of
+    // slot % 8, most used link first, then passes that move a link to where it meets fewer
+    const int nkey = (int)keys.size();
+    using Read = std::pair<int, int>;  // link, orientation
+    std::vector<std::vector<Read>> groups;
+    std::vector<std::vector<std::pair<int, int>>> member(nkey);  // group, orientation
+    for (int mu = 0; mu < 4; mu++)
+        for (int i = 0; i < kSteps; i++)
+            for (int p0 = 0, p1; p0 < kPaths; p0 = p1) {
+                // the eight-lane groups: plaquettes, 8 + 8 + 2 rectangles, eights of the others
+                p1 = p0 == 0 ? 6 : p0 == 22 ? 24 : p0 + 8;
+                std::vector<Read> g;
+                for (int p = p0; p < p1; p++) {
+                    const Read k{T->slot[mu][p][i], T->fwd[mu][p][i]};
+                    if (std::find(g.begin(), g.end(), k) == g.end()) g.push_back(k);
+                }
+                for (const Read& k : g) member[k.first].push_back({(int)groups.size(), k.second});
+                groups.push_back(g);
+            }
+    std::vector<int> order(nkey), res(nkey, -1);
+    int used[8] = {0};
+    for (int k = 0; k < nkey; k++) order[k] = k;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return member[a].size() > member[b].size(); });
+    for (int pass = 0; pass < 8; pass++)
+        for (int k : order) {
+            if (res[k] >= 0) used[res[k]]--;
+            int cost[8] = {0};
+            for (const auto& g : member[k])
+                for (const Read& o : groups[g.first])
+                    if (o.first != k && res[o.first] >= 0) {
+                        const int at = res[o.first];
+                        if (o.second == g.second) {
+                            cost[at] += 9;
+                        } else {
+                            cost[at] += 3;
+                            for (int d = 2; d < 8; d += 2) cost[(at + d) & 7] += 2;
+                        }
+                    }
+            int best = -1;
+            for (int r = 0; r < 8; r++)
+                if (used[r] < kDemonWindow / 8 && (best < 0 || cost[r] < cost[best])) best = r;
+            if (best < 0) return false;
+            res[k] = best;
+            used[best]++;
+        }
+    std::vector<int> slot(nkey);
+    int count[8] = {0};
+    for (int n = 0; n < kDemonWindow; n++) T->packed[n] = keys[unit];  // slots without a link
+    for (int k = 0; k < nkey; k++) {
+        slot[k] = res[k] + 8 * count[res[k]]++;
+        T->packed[slot[k]] = keys[k];
+        T->nslot = std::max(T->nslot, slot[k] + 1);
+    }
+    for (int mu = 0; mu < 4; mu++)
+        for (int p = 0; p < kPaths; p++)
+            for (int i = 0; i < kSteps; i++) T->slot[mu][p][i] = (uint16_t)slot[T->slot[mu][p][i]];
+    if (lkey < 0) return false;
+    T->lslot = slot[lkey];
+    T->uslot = slot[ukey];
     return true;
 }
 
