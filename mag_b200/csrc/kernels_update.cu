@@ -73,11 +73,14 @@ __device__ dd2 block_reduce(dd2 v) {
 }
 
 // ------------------------------------------------------------------- updates
+// U <- e^{eps X} U.  Bound by memory (432 B per link with the FP32 copy) on lattices that fill
+// the GPU, by one thread's exponential on small ones.  Blocks of two warps at 146 registers, no
+// spills, spread over all SMs: 3.3 us at 8^4, 14.9 at 16^4, 226 at 32^4 against 4.4, 15.6, 251
+// with blocks of eight warps at 128 registers; at 96 registers it spills (238 us).
+constexpr int kEvolveBlock = 64;
 template <typename TU, typename TX>
-// two resident blocks per SM (at most 128 registers): a streaming kernel needs the warps
-__global__ void __launch_bounds__(kBlock, 2) k_evolve(DevGeom g, LinkPlanes<TU> Uin, LinkPlanes<TU> Uout,
-                                                      AlgPlanes<TX> X, double eps,
-                         LinkPlanes<float> Ucopy) {
+__global__ void __launch_bounds__(kEvolveBlock, 6) k_evolve(DevGeom g, LinkPlanes<TU> Uin, LinkPlanes<TU> Uout,
+                                                            AlgPlanes<TX> X, double eps, LinkPlanes<float> Ucopy) {
     after_previous();
     ChainInfo ci;
     Site st;
@@ -593,7 +596,8 @@ template void launch_fma_probe<double>(double*, int, int, cudaStream_t);
 template <typename TU, typename TX>
 void launch_evolve(const DevGeom& g, LinkPlanes<TU> Uin, LinkPlanes<TU> Uout, AlgPlanes<TX> X, double eps,
                    LinkPlanes<float> Ucopy, cudaStream_t s) {
-    launch_after(k_evolve<TU, TX>, dim3(blocks(g), 4), kBlock, 0, s, g, Uin, Uout, X, eps, Ucopy);
+    launch_after(k_evolve<TU, TX>, dim3((unsigned)((g.vpad + kEvolveBlock - 1) / kEvolveBlock), 4), kEvolveBlock, 0, s, g,
+                 Uin, Uout, X, eps, Ucopy);
 }
 template void launch_evolve<double, double>(const DevGeom&, LinkPlanes<double>, LinkPlanes<double>,
                                             AlgPlanes<double>, double, LinkPlanes<float>, cudaStream_t);
