@@ -554,7 +554,7 @@ struct mag_ctx {
         LinkPlanes<double> cur = U;
         hx(cur);
         for (int k = 0; k < p.n_stout; k++) {
-            forward_level(cur, st64, k);
+            launch_stout_level<double>(geom, cur, st64.lv[k], AlgPlanes<double>{}, st64.rem, stream);
             cur = st64.lv[k];
             hx(cur);
         }

@@ -136,7 +136,7 @@ void launch_stout_chain_force(const DevGeom& g, LinkPlanes<T> Ul, AlgPlanes<T> L
                               int v, cudaStream_t s);
 
 // ---- stout smearing on plaquettes (kernels_smear.cu); S: six plane fields, Rem: twelve
-// one forward level: Q and U' = e^{iQ} U from the plaquettes S of U
+// one forward level: U' = e^{iQ} U, and Q where it is given a place, from the plaquettes S of U
 template <typename T>
 void launch_stout_level(const DevGeom& g, LinkPlanes<T> U, LinkPlanes<T> Uout, AlgPlanes<T> Q, AlgPlanes<T> S,
                         cudaStream_t s);

@@ -109,7 +109,9 @@ __device__ __forceinline__ herm8<T> staple_angle(const LinkPlanes<T>& U, const A
     return sum;
 }
 
-// Q = -i rho TA(stp U^dag) (field-multi.h:32-39), U' = e^{iQ} U
+// Q = -i rho TA(stp U^dag) (field-multi.h:32-39), U' = e^{iQ} U.  Q is kept for the derivative
+// where the caller gives a place for it; without, 256 of 1792 B per site and level less go to
+// memory, which bounds it (Hamiltonian of 24^3 x 48 with three levels 1.80 -> 1.72 ms)
 template <typename T>
 __global__ void __launch_bounds__(kLinkBlock, 5) k_stout_apply(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S,
                                                             LinkPlanes<T> Uout, AlgPlanes<T> Q) {
@@ -119,7 +121,7 @@ __global__ void __launch_bounds__(kLinkBlock, 5) k_stout_apply(DevGeom g, LinkPl
     if (!locate_tile(g, ci, st)) return;
     const int mu = threadIdx.x >> 5;
     const herm8<T> q = scaled(staple_angle(U, S, ci, st, mu), (T)ci.rho);
-    Q.store(mu, st.g, q);
+    if (Q.p) Q.store(mu, st.g, q);
     Uout.store(mu, st.g, exp_times(q, U.load(mu, st.g)));
 }
 
@@ -452,9 +454,10 @@ void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgP
                        cudaStream_t s) {
     // blocks of six warps per SM: two of FP64 (168 registers, no spills; three would spill 1 KB:
     // 1.47 against 0.83 ms at 32^4), three of FP32 (96 registers; 0.369 against 0.431 ms)
-    if (sizeof(T) == 8 && tiles(g) <= kSoloTiles)
-        launch_after(k_plaq_chain<T, 1>, tiles(g), kPlaqBlock, 0, s, g, U, Lam, Loc, Rem);
-    else launch_after(k_plaq_chain<T, sizeof(T) == 8 ? 2 : 3>, tiles(g), kPlaqBlock, 0, s, g, U, Lam, Loc, Rem);
+    if constexpr (sizeof(T) == 8) {
+        if (tiles(g) <= kSoloTiles) return launch_after(k_plaq_chain<T, 1>, tiles(g), kPlaqBlock, 0, s, g, U, Lam, Loc, Rem);
+    }
+    launch_after(k_plaq_chain<T, sizeof(T) == 8 ? 2 : 3>, tiles(g), kPlaqBlock, 0, s, g, U, Lam, Loc, Rem);
 }
 template <typename T>
 void launch_chain_gather(const DevGeom& g, AlgPlanes<T> Loc, AlgPlanes<T> Rem, AlgPlanes<T> Dir, bool top,
@@ -485,9 +488,10 @@ void launch_plaq_rect(const DevGeom& g, LinkPlanes<T> U, RowPlanes<T> Pl, AlgPla
     launch_after(k_plaq<T>, tiles(g), kPlaqBlock, 0, s, g, U, Pl);
     // two blocks of six warps per SM in both precisions (three: 0.81 against 0.75 ms FP32 at 32^4,
     // twice as slow in FP64, from spills)
-    if (sizeof(T) == 8 && tiles(g) <= kSoloTiles)
-        launch_after(k_plaq_rect<T, 1>, tiles(g), kPlaqBlock, 0, s, g, U, Pl, Loc, Rem);
-    else launch_after(k_plaq_rect<T, 2>, tiles(g), kPlaqBlock, 0, s, g, U, Pl, Loc, Rem);
+    if constexpr (sizeof(T) == 8) {
+        if (tiles(g) <= kSoloTiles) return launch_after(k_plaq_rect<T, 1>, tiles(g), kPlaqBlock, 0, s, g, U, Pl, Loc, Rem);
+    }
+    launch_after(k_plaq_rect<T, 2>, tiles(g), kPlaqBlock, 0, s, g, U, Pl, Loc, Rem);
 }
 template <typename T>
 void launch_wilson_force(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> S, AlgPlanes<T> F, cudaStream_t s) {
