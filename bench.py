@@ -88,32 +88,25 @@ COMMON = dict(mag=2, action="iwasaki", c1=-0.331, rho=0.1, tau=1.0, accept="metr
 # algorithmic flops per site of one launch, reference (gather) formulation:
 # 3x3 complex product = 198 flop, matrix add = 18 flop
 FLOPS_PER_SITE = {
-    # extended staple: 12 plaquette + 72 rectangle path products, 25 adds, per link
-    "staple": 4 * (84 * 198 + 25 * 18),
-    # thin-link force: staple + U A^dag + traceless anti-Hermitian part
-    "force": 4 * (85 * 198 + 25 * 18 + 30),
+    # force of the top links: extended staple (12 plaquette + 72 rectangle path products, 25 adds
+    # per link), U A^dag, traceless anti-Hermitian part
+    "plaq_force": 4 * (85 * 198 + 25 * 18 + 30),
     # stout level: 12 staple products + Omega + Q^2 + exp combination + exp(iQ) U
-    "stout_forward": 4 * (15 * 198 + 6 * 18 + 120),
+    "stout_level": 4 * (15 * 198 + 6 * 18 + 120),
     # Lambda: U Z, Q^2, Q W, W Q, Z exp(iQ), three traces of products
-    "stout_lambda": 4 * (5 * 198 + 3 * 66 + 10 * 18 + 150),
+    "chain_gather": 4 * (5 * 198 + 3 * 66 + 10 * 18 + 150),
     # chain rule: C recomputed (12 products), C^dag Lambda, 6 insertions x 3 products x 3 directions
-    "stout_chain": 4 * (67 * 198 + 24 * 18),
+    "plaq_chain": 4 * (67 * 198 + 24 * 18),
 }
 
-# flops per site the kernels execute after reassociation, same conventions
-# (complex multiply 6, complex add 2): general product 198, two-row SU(3)
-# product 132 + 42 for the reconstructed row = 174, Hermitian x general 162
+# flops per site the kernels execute (one per addition or product, two per multiply-add), as ncu
+# counts the FP64 instructions; the FP32 kernels run the same operations, but for the smearing
+# level, one thread per link there: six staples (132 + 174 + 18: a two-row SU(3) product is 132,
+# its third row 42), C U^dag, Q^2, the exponential's combination, exp(iQ) U, coefficients
 EXECUTED_FLOPS_PER_SITE = {
-    # per link: 2 x 3 x (132 + 174 + 18) + 198 for each of the two shared-factor sums,
-    # 3 x 4 x (132 + 174 + 36) for plaquettes and nu-extended rectangles
-    "staple": 4 * (2 * (3 * 2 * (132 + 174 + 18) + 198) + 3 * 4 * (132 + 174 + 36) + 18),
-    "force": 4 * (2 * (3 * 2 * (132 + 174 + 18) + 198) + 3 * 4 * (132 + 174 + 36) + 18 + 198 + 30),
-    # 6 staples (132 + 174 + 18), C U^dag, Q^2, exp combination, exp(iQ) U, coefficients
-    "stout_forward": 4 * (6 * (132 + 174 + 18) + 198 + 30 + 162 + 144 + 198 + 120),
-    "stout_lambda": 4 * (3 * 198 + 3 * 162 + 2 * 144 + 350),
-    # per direction: upper D, E (174 each), three Hermitian products, D x inner (216 with the accumulate);
-    # lower G (174), three Hermitian products, one general product, U^dag x inner (216)
-    "stout_chain": 4 * (3 * ((2 * 174 + 3 * 162 + 216 + 44) + (174 + 3 * 162 + 198 + 216 + 44)) + 36),
+    "fp64": {"plaq_force": 20722, "stout_level": 7567, "plaq_chain": 10468, "chain_gather": 3567},
+    "mixed": {"plaq_force": 20722, "stout_level": 4 * (6 * (132 + 174 + 18) + 198 + 30 + 162 + 144 + 198 + 120),
+              "plaq_chain": 10468, "chain_gather": 3567},
 }
 
 
@@ -439,11 +432,10 @@ def measured_hbm_gbs() -> float:
 
 def wilson_bytes(wl: int, V: int) -> int:
     """Algorithmic HBM bytes of one Wilson-loop measurement (R, T <= wl, three spatial directions) of V
-    sites: per direction the R-line planes (first: read U, write the line; then read U and the previous
-    line, write), per T the temporal line (the same) and the accumulation pass (reads the wl S-line
-    planes and the temporal line once per site; the shifted reads come from L2)."""
-    per_dir = (288 + (wl - 1) * 432) + (288 + (wl - 1) * 432) + wl * (wl + 1) * 144
-    return 3 * per_dir * V
+    sites in the temporal gauge: the time links read and the gauge G written, the spatial links and G
+    read and the transformed links written, these read once for the loops (the lines along R and the
+    shifted slices come from shared memory and L2; the measurement is bound there, not by HBM)."""
+    return (2 * 144 + (3 + 1 + 3) * 144 + 3 * 144) * V
 
 
 def sub_run(M, workload: str, precisions, args, steps: int | None = None, warmup: int | None = None) -> dict:
@@ -574,9 +566,9 @@ def run_gpu(args, params, rank, world, dist):
     kernels_per_traj = c64.graph_kernel_count()
 
     # dominant kernel and its roofline (device-timed on the launching stream)
-    names = ["staple", "stout_forward", "stout_lambda", "stout_chain"] if params["n_stout"] else ["force"]
-    per_eval = {"staple": 1, "force": 1, "stout_forward": params["n_stout"], "stout_lambda": params["n_stout"],
-                "stout_chain": params["n_stout"]}
+    names = ["plaq_force", "stout_level", "plaq_chain", "chain_gather"] if params["n_stout"] else ["plaq_force"]
+    per_eval = {k: 1 if k == "plaq_force" else params["n_stout"] for k in names}
+    flops = EXECUTED_FLOPS_PER_SITE[head_prec]
     kt = {k: c64.time_kernel(k, 5) for k in names}
     share = {k: kt[k] * per_eval[k] for k in names}
     dom = max(share, key=share.get)
@@ -587,19 +579,18 @@ def run_gpu(args, params, rank, world, dist):
     tpath = os.path.join(ROOT, "profiles", "roofline_traffic.json")
     if os.path.exists(tpath):
         traffic = json.load(open(tpath)).get(f"{args.workload}:{head_prec}:{dom}")
-    # achieved = flops the kernel executes per launch (two-row SU(3) and Hermitian products, confirmed
-    # by ncu's FMA/ADD/MUL instruction counts) / its CUDA-event launch time
-    executed = EXECUTED_FLOPS_PER_SITE[dom] * V / (kt[dom] * 1e-3) / 1e12
+    # achieved = flops the kernel executes per launch / its CUDA-event launch time
+    executed = flops[dom] * V / (kt[dom] * 1e-3) / 1e12
     gather = FLOPS_PER_SITE[dom] * V / (kt[dom] * 1e-3) / 1e12
     roofline = {"bound": prec_key, "kernel": dom, "achieved": executed, "peak": peak, "unit": "TFLOP/s",
-                "frac": executed / peak, "traffic": traffic, "flops_per_site": EXECUTED_FLOPS_PER_SITE[dom],
+                "frac": executed / peak, "traffic": traffic, "flops_per_site": flops[dom],
                 "algorithmic_equiv": {"achieved": gather, "frac": gather / peak, "flops_per_site": FLOPS_PER_SITE[dom],
                                       "note": "the reference's gather formulation (85 / 67 products per link); "
                                               "the kernels execute fewer flops, so this can exceed 1"},
                 "peak_source": f"measured CUDA-core {prec_key.upper()} FMA throughput (mag_probe_fma_peak)",
                 "launch_ms": kt[dom], "kernel_ms": kt,
-                "executed_frac": {k: EXECUTED_FLOPS_PER_SITE[k] * V / (kt[k] * 1e-3) / 1e12 / peak for k in names},
-                "force_eval_ms": t_force_eval, "tuned": c64.autotune(3)}
+                "executed_frac": {k: flops[k] * V / (kt[k] * 1e-3) / 1e12 / peak for k in names},
+                "force_eval_ms": t_force_eval}
     ev_ms = c64.time_kernel("evolve", 5)
     bytes_evolve = V * 4 * (144 + 144 + 64) + (V * 4 * 72 if head_prec == "mixed" else 0)
     peaks = {}

@@ -263,8 +263,8 @@ int mag_nersc_read_header(const char* path, mag_nersc_info* info);
    from the same sums and uniform, as the MPI_Bcast of :823 ensures).  Each
    slab is a context over its time slices plus `halo` slices of each
    neighbour; the halos are refreshed wherever a kernel reads across the
-   boundary (the links of each force evaluation, every stout level, the
-   double links, each level's Lambda, and the links of the Hamiltonian's
+   boundary (the links of each force evaluation, every stout level,
+   each level's Lambda, and the links of the Hamiltonian's
    smearing).  The shards live on the current device and are driven by one
    host thread each.  Requirements: dims[3] % nshards == 0; 2 <= halo <=
    dims[3] / nshards; dims[3] / nshards a multiple of mag (constrained

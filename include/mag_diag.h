@@ -22,15 +22,23 @@ int mag_last_measure_ms(mag_ctx* ctx, double* ms);
    context's precision, constraint fix-up included) on the current links */
 int mag_time_force(mag_ctx* ctx, int reps, double* ms_per_eval);
 /* average device time of one launch of a single kernel on the current
-   fields: "force", "staple", "stout_forward", "stout_lambda", "stout_chain",
+   fields.  Kernels of a force evaluation: "plaq_force" (the force terms of
+   the top links, two launches), "stout_level" (one forward level),
+   "chain_gather" (Lambda of a level from the derivative above it),
+   "plaq_chain" (one level of the chain rule) and "lambda" (Lambda of the top
+   level, Wilson action).  Of the one-thread-per-link form (mag_autotune):
+   "force", "staple", "stout_forward", "stout_lambda", "stout_chain".  Also
    "evolve", "kick", "action", and the NERSC payload kernels on chain 0's
    3x3 payload made from the current links: "nersc_swap" (byte order +
    word checksum), "nersc_crc" (segment CRC-32), "nersc_to_links",
    "nersc_from_links", "nersc_plaq" (plaquette and link-trace sums) */
 int mag_time_kernel(mag_ctx* ctx, const char* which, int reps, double* ms_per_launch);
-/* re-run the launch-configuration tuner: time every variant of the staple /
-   force / stout kernels on the live fields (`reps` launches each) and keep the
-   fastest.  Variants: one thread per link at minimum blocks per SM 2..5
+/* Forces are evaluated over plaquettes, with launch shapes that the lattice's
+   size and the precision decide.  The older one-thread-per-link form (matrix
+   derivatives) is kept for what mag_set_kernel_variant selects and as a
+   measure; this is its tuner: time every variant of its staple / force / stout
+   kernels on the live fields (`reps` launches each) and keep the fastest for
+   that form.  It does not change which form a context's forces take.  Variants: one thread per link at minimum blocks per SM 2..5
    ("t1m2".."t1m5", register caps), and for the staple, force and chain-rule
    kernels the direction split "s<NS>r<R>" (NS = 3 or 6 warps per 32-link tile,
    register cap R).  Every variant is timed; the choice is made among the
@@ -42,12 +50,14 @@ int mag_time_kernel(mag_ctx* ctx, const char* which, int reps, double* ms_per_la
    report (may be NULL) receives a JSON object
    {"family": {"fp64": [chosen, {variant: ms, ...}], "fp32": [...]}, ...,
     "block_order": [tile, {"raster": ms, "tile2": ms, "tile4": ms}]}
-   (times only for the families and precisions the context tuned).  The first
-   trajectory, integration or graph build of a context runs the tuner once. */
+   (times only for the families and precisions the context tuned).  A context
+   whose forces take the one-thread-per-link form runs the tuner once, at its
+   first trajectory, integration or graph build. */
 int mag_autotune(mag_ctx* ctx, int reps, char* report, size_t len);
 /* use `variant` (a name as in the mag_autotune report) for kernel `family`
    ("force", "staple", "stout_forward", "stout_lambda", "stout_chain") at
-   precision 0 (FP64) or 1 (FP32) from now on, in place of the tuner's choice */
+   precision 0 (FP64) or 1 (FP32) from now on, in place of the tuner's choice;
+   the context's forces of that precision then take the one-thread-per-link form */
 int mag_set_kernel_variant(mag_ctx* ctx, const char* family, int precision, const char* variant);
 /* number of kernel nodes in the captured trajectory graph (building it if needed) */
 int mag_graph_kernel_count(mag_ctx* ctx, int* kernels);

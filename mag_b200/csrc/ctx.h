@@ -441,7 +441,7 @@ struct mag_ctx {
 
     // A sharded context exchanges halos (hx) after every launch whose output a
     // later kernel reads across the shard boundary: the links whose force is
-    // taken, each smeared level, the double links and Lambda of each level.
+    // taken, each smeared level, and Lambda of each level.
     //
     // Smeared links: the top level's force is the derivative with respect to the top
     // links in the Lie algebra (the force kernel, beta/3 included; everything after it

@@ -1,19 +1,19 @@
-// kernels_force.cu -- staple, gauge-force and stout-smearing kernels (sm_100a).
+// kernels_force.cu -- staple, gauge-force and stout-smearing kernels with one thread per
+// link (sm_100a).  Forces are evaluated over plaquettes (kernels_smear.cu); of these
+// kernels the smearing level runs in every mixed-precision force (FP32), the staple in
+// mag_staple, and the others where mag_set_kernel_variant selects them.
 //
-// One thread per link.  Blocks are ordered direction-fastest: block b covers
-// sites (b / 4) * 128 ... + 127 for mu = b % 4, so the four links of a site
-// range are processed at the same time and their shared neighbour links are
-// still in L2.  A warp covers 32 consecutive sites of one direction, runs one
-// path table and issues coalesced plane loads.  These kernels are bound by the
-// CUDA-core FP pipe (3x3 complex products are not a dense contraction; tensor
-// cores do not apply).
+// Blocks are ordered direction-fastest: block b covers sites (b / 4) * 128 ... + 127
+// for mu = b % 4, so the four links of a site range are processed at the same time
+// and their shared neighbour links are still in L2.  A warp covers 32 consecutive
+// sites of one direction, runs one path table and issues coalesced plane loads.
+// These kernels are bound by the CUDA-core FP pipe (3x3 complex products are not a
+// dense contraction; tensor cores do not apply).
 //
-// Every kernel exists in register-cap variants (__launch_bounds__ minimum
-// blocks per SM 2, 3, 4, 5 -> at most 255, 168, 128, 102 registers per thread);
-// the context's tuner times them on live data and keeps the fastest.  The
-// staple, force and chain-rule kernels also exist as direction-split shapes
-// (3 or 6 warps per 32-link tile, below), which the tuner times for its report
-// and which are selected explicitly (mag_set_kernel_variant).
+// Every kernel exists in register-cap variants (__launch_bounds__ minimum blocks per
+// SM 2, 3, 4, 5 -> at most 255, 168, 128, 102 registers per thread), which the tuner
+// (mag_autotune) times on live data.  The staple, force and chain-rule kernels also
+// exist as direction-split shapes (3 or 6 warps per 32-link tile, below).
 #include "gauge_ops.cuh"
 #include "kernels.h"
 
@@ -180,8 +180,7 @@ __global__ void __launch_bounds__(kForceBlock, MINB) k_stout_chain(DevGeom g, Li
 // _ext or stout_chain_upper / _lower_acc).  The parts meet in shared memory and
 // are added in warp order.  A thread then holds the temporaries of one
 // direction (or half) instead of all three, so more warps fit on an SM at a
-// register cap R; the shape (NS, R) is what the tuner picks from, next to the
-// one-thread-per-link register-cap variants.
+// register cap R.
 __device__ __forceinline__ bool locate_split(const DevGeom& g, ChainInfo& ci, Site& st, int& mu, int& nu, int& w,
                                              int& lane, int& gs) {
     mu = blockIdx.x & 3;

@@ -340,7 +340,7 @@ class Chmc:
         return v.value
 
     def autotune(self, reps: int = 3) -> dict:
-        """Re-run the launch-configuration tuner; returns
+        """Run the tuner of the one-thread-per-link force kernels; returns
         {family: {"fp64": [chosen variant, {variant: ms}], "fp32": [...]}}."""
         import json
 
@@ -349,7 +349,8 @@ class Chmc:
         return json.loads(buf.value.decode())
 
     def set_kernel_variant(self, family: str, precision: str, variant: str) -> None:
-        """Use `variant` (e.g. "t1m3", "s6r128") for `family` at "fp64" or "fp32" in place of the tuner's choice."""
+        """Use `variant` (e.g. "t1m3", "s6r128") for `family` at "fp64" or "fp32"; the
+        context's forces of that precision then take the one-thread-per-link form."""
         check(self._lib.mag_set_kernel_variant(self._h, family.encode(), 0 if precision == "fp64" else 1,
                                                variant.encode()), "mag_set_kernel_variant")
 

@@ -24,7 +24,7 @@ def main(argv=None) -> int:
     ap.add_argument("--mag", type=int, default=2)
     ap.add_argument("--reps", type=int, default=2)
     ap.add_argument("--kernels", nargs="*", default=[])
-    ap.add_argument("--no-tune", action="store_true", help="keep the default variants (255-register cap)")
+    ap.add_argument("--no-tune", action="store_true", help="leave out the tuner of the one-thread-per-link kernels")
     ap.add_argument("--probe", action="store_true", help="also report the FMA throughput probes")
     ap.add_argument("--demon", type=int, default=0, metavar="SWEEPS",
                     help="also run this many per-link demon sweeps (E_max 50) and report their device time")
