@@ -242,26 +242,27 @@ __global__ void __launch_bounds__(kBlock) k_gauge_links(ChainInfo ci, LinkPlanes
     V.store(i, s, mul_nd(mul(G.load(0, s), u), G.load(0, sn)));
 }
 
-// One block: NX spatial sites (blockDim = NX times the groups of three time slices, in
+// One block: NX spatial sites (blockDim = NX times the groups of SL time slices, in
 // whole warps), direction i = blockIdx.y.  Shared memory holds S_R of the sites for
-// t in [0, Lt + Tmax).  A thread extends the lines of its three slices, then takes the
-// traces of its slices with the slices up to T + 2 later, each read once for three
-// loops.  Bound by shared-memory reads (36 cycles per matrix and warp against 9 for a
+// t in [0, Lt + Tmax).  A thread extends the lines of its SL slices, then takes the
+// traces of its slices with the slices up to T + SL - 1 later, each read once for SL
+// loops, TC values of T at a time (4 where Tmax is no more: 16^4 to 4 92 -> 86 us).
+// Bound by shared-memory reads (36 cycles per matrix and warp against 9 for a
 // trace's multiply-adds) and the warps that registers and the 72 KB allow: three slices
 // at 168 registers 0.98 ms at 24^3 x 48 (R, T <= 8), four at 208 or 232 1.25, two at
-// 128 1.11; 48^3 x 96: 15.9, 23.8 and 24.9 ms.  A block walks the groups of NX sites with stride gridDim.x and adds up its
+// 128 1.11; 48^3 x 96: 15.9, 23.8 and 24.9 ms.  A block walks the groups of NX sites
+// with stride gridDim.x and adds up its
 // part[((i Rmax + R-1) Tmax + T-1) gridDim.x + block].
-constexpr int kSlices = 3, kTChunk = 8;
 constexpr int kGaugedBlocks = 592;  // per direction at most: four per SM
-template <int NX>
+template <int NX, int SL, int TC>
 __global__ void __maxnreg__(168) k_wloop_gauged(ChainInfo ci, LinkPlanes<double> V, LinkPlanes<double> P,
                                                       int Rmax, int Tmax, dd2* part) {
     after_previous();
     extern __shared__ __align__(16) unsigned char wsm[];
     cplx<double>* S = reinterpret_cast<cplx<double>*>(wsm);  // [Lt + Tmax][9][NX]
-    __shared__ double red[8][kTChunk];
+    __shared__ double red[8][TC];
     const int Lt = ci.L[3], vs = ci.L[0] * ci.L[1] * ci.L[2], i = blockIdx.y;
-    const int nx = threadIdx.x % NX, t0 = (threadIdx.x / NX) * kSlices;
+    const int nx = threadIdx.x % NX, t0 = (threadIdx.x / NX) * SL;
     const int Li = i == 0 ? ci.L[0] : i == 1 ? ci.L[1] : ci.L[2];
     const int si = i == 0 ? 1 : i == 1 ? ci.L[0] : ci.L[0] * ci.L[1];
     auto put = [&](int t, const mat3<double>& m) {
@@ -286,7 +287,7 @@ __global__ void __maxnreg__(168) k_wloop_gauged(ChainInfo ci, LinkPlanes<double>
             // 1. S_R(t) = S_{R-1}(t) V_i(x + (R-1) i, t) of this thread's slices
             const int xr = site ? along(R - 1) : 0, xe = site ? along(R) : 0;
 #pragma unroll 1
-            for (int t = t0; t < t0 + kSlices && t < Lt; t++) {
+            for (int t = t0; t < t0 + SL && t < Lt; t++) {
                 if (!site) {
                     put(t, zero_mat<double>());
                     continue;
@@ -296,31 +297,31 @@ __global__ void __maxnreg__(168) k_wloop_gauged(ChainInfo ci, LinkPlanes<double>
             }
             // 2. the slices past the boundary, from this thread's own slices
 #pragma unroll 1
-            for (int t = t0; t < t0 + kSlices && t < Lt && t < Tmax; t++)
+            for (int t = t0; t < t0 + SL && t < Lt && t < Tmax; t++)
                 put(Lt + t, site ? mul_nd(mul(P.load(0, x), get(t)), P.load(0, xe)) : zero_mat<double>());
             __syncthreads();
-            // 3. traces, kTChunk values of T at a time
-            mat3<double> a[kSlices];
+            // 3. traces, TC values of T at a time
+            mat3<double> a[SL];
 #pragma unroll
-            for (int j = 0; j < kSlices; j++) {
+            for (int j = 0; j < SL; j++) {
                 if (t0 + j < Lt) a[j] = get(t0 + j);
                 else set_zero(a[j]);
             }
-            for (int Tb = 0; Tb < Tmax; Tb += kTChunk) {
-                double acc[kTChunk];
+            for (int Tb = 0; Tb < Tmax; Tb += TC) {
+                double acc[TC];
 #pragma unroll
-                for (int k = 0; k < kTChunk; k++) acc[k] = 0.0;
+                for (int k = 0; k < TC; k++) acc[k] = 0.0;
 #pragma unroll
-                for (int u = 1; u < kTChunk + kSlices; u++) {
+                for (int u = 1; u < TC + SL; u++) {
                     const int t = t0 + Tb + u;
                     const mat3<double> b = get(t < last ? t : last);  // beyond the last slice: only a[j] = 0 or T > Tmax
 #pragma unroll
-                    for (int j = 0; j < kSlices; j++)
-                        if (u - j >= 1 && u - j <= kTChunk) acc[u - j - 1] += retr_mul_nd(a[j], b);
+                    for (int j = 0; j < SL; j++)
+                        if (u - j >= 1 && u - j <= TC) acc[u - j - 1] += retr_mul_nd(a[j], b);
                 }
-                // the warp's sums: eight values over 32 lanes, half of them kept at each of three steps
+                // the warp's sums: TC values over 32 lanes, half of them kept at each step
 #pragma unroll
-                for (int h = kTChunk / 2, o = 16; h >= 1; h /= 2, o /= 2) {
+                for (int h = TC / 2, o = 16; h >= 1; h /= 2, o /= 2) {
                     const bool up = lane & o;
 #pragma unroll
                     for (int k = 0; k < h; k++) {
@@ -328,12 +329,12 @@ __global__ void __maxnreg__(168) k_wloop_gauged(ChainInfo ci, LinkPlanes<double>
                         acc[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
                     }
                 }
-                acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
-                acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
-                // lane bits 4, 3, 2 select the value
-                if ((lane & 3) == 0) red[wid][lane >> 2] = acc[0];
+#pragma unroll
+                for (int o = 16 / TC; o >= 1; o /= 2) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+                // the lane's upper bits select the value
+                if (lane % (32 / TC) == 0) red[wid][lane / (32 / TC)] = acc[0];
                 __syncthreads();
-                if (threadIdx.x < kTChunk && Tb + (int)threadIdx.x < Tmax) {
+                if (threadIdx.x < TC && Tb + (int)threadIdx.x < Tmax) {
                     dd2 v{red[0][threadIdx.x], 0.0};
                     for (int w = 1; w < nw; w++) v = dd_add(v, dd2{red[w][threadIdx.x], 0.0});
                     dd2* p = part + ((size_t)(i * Rmax + R - 1) * Tmax + Tb + threadIdx.x) * gridDim.x + blockIdx.x;
@@ -360,16 +361,34 @@ unsigned blocks(const DevGeom& g) { return (unsigned)((g.vpad + kBlock - 1) / kB
 
 }  // namespace
 
-// Shapes of k_wloop_gauged: the most spatial sites per block (32 down to 1) whose lines
-// take at most 72 KB (three blocks per SM) and whose slice groups fit 256 threads;
-// 0: none, the chain is too long in time.
-int wilson_gauged_sites(const ChainInfo& ci, int Tmax) {
-    if (Tmax > ci.L[3]) return 0;
-    const int groups = (ci.L[3] + kSlices - 1) / kSlices;
+// Shape of k_wloop_gauged: slices per thread and the most spatial sites per block (32 down
+// to 1) whose lines take at most 72 KB (three blocks per SM) and whose slice groups fit 256
+// threads; 0 sites: none, the chain is too long in time.
+struct GaugedShape {
+    int nx, sl;
+};
+static int gauged_fit(const ChainInfo& ci, int Tmax, int sl) {
+    const int groups = (ci.L[3] + sl - 1) / sl;
     for (int nx = 32; nx >= 1; nx /= 2)
         if ((size_t)nx * (ci.L[3] + Tmax) * 144 <= 72 * 1024 && nx * groups <= 256) return nx;
     return 0;
 }
+static GaugedShape gauged_shape(const ChainInfo& ci, int Tmax) {
+    if (Tmax > ci.L[3]) return {0, 3};
+    const int vs = ci.L[0] * ci.L[1] * ci.L[2];
+    // Three slices per thread read each line for three traces.  Chains that leave an SM fewer
+    // than about six warps of such threads are bound by a thread's own work: one slice each, in
+    // blocks that spread over the SMs.  One measurement, three slices against one: 8^4 to R, T
+    // = 4 40 against 31 us, 12^4 56 against 52, 8^3 x 16 to 8 87 against 62, 10^3 x 20 to 6 80
+    // against 72 (21,000 threads); 12^3 x 24 to 8 109 against 136 (41,000).
+    if (3L * vs * ((ci.L[3] + 2) / 3) < 30000) {
+        int nx = gauged_fit(ci, Tmax, 1);
+        while (nx > 4 && 3 * ((vs + nx - 1) / nx) < 148) nx /= 2;
+        if (nx) return {nx, 1};
+    }
+    return {gauged_fit(ci, Tmax, 3), 3};
+}
+int wilson_gauged_sites(const ChainInfo& ci, int Tmax) { return gauged_shape(ci, Tmax).nx; }
 static int gauged_blocks(const ChainInfo& ci, int nx) {
     const int groups = (ci.L[0] * ci.L[1] * ci.L[2] + nx - 1) / nx;
     return groups < kGaugedBlocks ? groups : kGaugedBlocks;
@@ -379,17 +398,26 @@ size_t wilson_gauged_partials(const ChainInfo& ci, int Rmax, int Tmax) {
     return nx ? (size_t)3 * Rmax * Tmax * gauged_blocks(ci, nx) : 0;
 }
 
-template <int NX>
+template <int NX, int SL, int TC>
 static cudaError_t wloop_gauged(const ChainInfo& ci, LinkPlanes<double> V, LinkPlanes<double> P, int Rmax, int Tmax,
                                 dd2* part, cudaStream_t s) {
-    const int groups = (ci.L[3] + kSlices - 1) / kSlices;
+    const int groups = (ci.L[3] + SL - 1) / SL;
     const int threads = (NX * groups + 31) / 32 * 32;
     const size_t smem = (size_t)NX * (ci.L[3] + Tmax) * 144;
     const cudaError_t e =
-        cudaFuncSetAttribute(k_wloop_gauged<NX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024);
+        cudaFuncSetAttribute(k_wloop_gauged<NX, SL, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024);
     if (e != cudaSuccess) return e;
-    launch_after(k_wloop_gauged<NX>, dim3(gauged_blocks(ci, NX), 3), threads, smem, s, ci, V, P, Rmax, Tmax, part);
+    launch_after(k_wloop_gauged<NX, SL, TC>, dim3(gauged_blocks(ci, NX), 3), threads, smem, s, ci, V, P, Rmax, Tmax, part);
     return cudaGetLastError();
+}
+template <int NX>
+static cudaError_t wloop_gauged(const ChainInfo& ci, int sl, LinkPlanes<double> V, LinkPlanes<double> P, int Rmax,
+                                int Tmax, dd2* part, cudaStream_t s) {
+    if (Tmax <= 4)
+        return sl == 1 ? wloop_gauged<NX, 1, 4>(ci, V, P, Rmax, Tmax, part, s)
+                       : wloop_gauged<NX, 3, 4>(ci, V, P, Rmax, Tmax, part, s);
+    return sl == 1 ? wloop_gauged<NX, 1, 8>(ci, V, P, Rmax, Tmax, part, s)
+                   : wloop_gauged<NX, 3, 8>(ci, V, P, Rmax, Tmax, part, s);
 }
 
 // One chain's planar loops in the temporal gauge: G and V, P scratch planes of the
@@ -399,17 +427,18 @@ static cudaError_t wloop_gauged(const ChainInfo& ci, LinkPlanes<double> V, LinkP
 cudaError_t launch_wilson_gauged(const ChainInfo& ci, LinkPlanes<double> U, int Rmax, int Tmax, LinkPlanes<double> G,
                                  LinkPlanes<double> V, LinkPlanes<double> P, dd2* part, dd2* out, int* bad,
                                  cudaStream_t s) {
-    const int nx = wilson_gauged_sites(ci, Tmax), vs = ci.L[0] * ci.L[1] * ci.L[2];
+    const GaugedShape shape = gauged_shape(ci, Tmax);
+    const int nx = shape.nx, vs = ci.L[0] * ci.L[1] * ci.L[2];
     launch_after(k_temporal_gauge, (vs + kGaugeBlock - 1) / kGaugeBlock, kGaugeBlock, 0, s, ci, U, G, P, bad);
     launch_after(k_gauge_links, dim3((ci.V + kBlock - 1) / kBlock, 3), kBlock, 0, s, ci, U, G, V, bad);
     cudaError_t e = cudaErrorInvalidValue;
     switch (nx) {
-        case 32: e = wloop_gauged<32>(ci, V, P, Rmax, Tmax, part, s); break;
-        case 16: e = wloop_gauged<16>(ci, V, P, Rmax, Tmax, part, s); break;
-        case 8: e = wloop_gauged<8>(ci, V, P, Rmax, Tmax, part, s); break;
-        case 4: e = wloop_gauged<4>(ci, V, P, Rmax, Tmax, part, s); break;
-        case 2: e = wloop_gauged<2>(ci, V, P, Rmax, Tmax, part, s); break;
-        case 1: e = wloop_gauged<1>(ci, V, P, Rmax, Tmax, part, s); break;
+        case 32: e = wloop_gauged<32>(ci, shape.sl, V, P, Rmax, Tmax, part, s); break;
+        case 16: e = wloop_gauged<16>(ci, shape.sl, V, P, Rmax, Tmax, part, s); break;
+        case 8: e = wloop_gauged<8>(ci, shape.sl, V, P, Rmax, Tmax, part, s); break;
+        case 4: e = wloop_gauged<4>(ci, shape.sl, V, P, Rmax, Tmax, part, s); break;
+        case 2: e = wloop_gauged<2>(ci, shape.sl, V, P, Rmax, Tmax, part, s); break;
+        case 1: e = wloop_gauged<1>(ci, shape.sl, V, P, Rmax, Tmax, part, s); break;
         default: return e;
     }
     if (e != cudaSuccess) return e;
