@@ -25,8 +25,8 @@ int mag_time_force(mag_ctx* ctx, int reps, double* ms_per_eval);
    fields.  Kernels of a force evaluation: "plaq_force" (the force terms of
    the top links, two launches), "stout_level" (one forward level),
    "chain_gather" (Lambda of a level from the derivative above it),
-   "plaq_chain" (one level of the chain rule) and "lambda" (Lambda of the top
-   level, Wilson action).  Of the one-thread-per-link form (mag_autotune):
+   "plaq_chain" (one level of the chain rule) and "lambda" (force terms of the
+   top links and Lambda of the top level, Wilson action, two launches).  Of the one-thread-per-link form (mag_autotune):
    "force", "staple", "stout_forward", "stout_lambda", "stout_chain".  Also
    "evolve", "kick", "action", and the NERSC payload kernels on chain 0's
    3x3 payload made from the current links: "nersc_swap" (byte order +

@@ -476,14 +476,12 @@ struct mag_ctx {
             launch_plaq_rect<T>(geom, cur, plaq_buf<T>(), b.loc, b.rem, stream);
             if (L) launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, true, b.Q[L - 1], b.lam, stream);
             else launch_force_gather<T>(geom, Uin, b.loc, b.rem, b.dir, true, use, stream);
+        } else if (L) {
+            launch_wilson_lambda<T>(geom, cur, b.rem, b.Q[L - 1], b.lam, b.dir, stream);
         } else {
             launch_wilson_force<T>(geom, cur, b.rem, use.F, stream);
-            if (L) {
-                launch_lambda<T>(geom, b.Q[L - 1], use.F, b.lam, b.dir, stream);
-            } else {
-                if (any_mag) launch_constraint_fixup<T>(geom, Uin, use.F, stream);
-                apply_use(Uin, use);
-            }
+            if (any_mag) launch_constraint_fixup<T>(geom, Uin, use.F, stream);
+            apply_use(Uin, use);
         }
         for (int k = L - 1; k >= 0; k--) {
             hx(b.lam);
@@ -581,7 +579,7 @@ struct mag_ctx {
     template <typename T>
     void launch_smear(const std::string& w, StoutBufs<T>& b, LinkPlanes<T> Uin, AlgPlanes<T> Fo) {
         if (w == "stout_level") forward_level(Uin, b, 0);
-        else if (w == "lambda") launch_lambda<T>(geom, b.Q[0], Fo, b.lam, b.dir, stream);
+        else if (w == "lambda") launch_wilson_lambda<T>(geom, Uin, b.rem, b.Q[0], b.lam, b.dir, stream);
         else if (w == "plaq_chain") launch_plaq_chain<T>(geom, Uin, b.lam, b.loc, b.rem, stream);
         else if (w == "chain_gather") launch_chain_gather<T>(geom, b.loc, b.rem, b.dir, false, b.Q[0], b.lam, stream);
         else if (iwasaki) launch_plaq_rect<T>(geom, Uin, plaq_buf<T>(), b.loc, b.rem, stream);

@@ -140,10 +140,6 @@ void launch_stout_chain_force(const DevGeom& g, LinkPlanes<T> Ul, AlgPlanes<T> L
 template <typename T>
 void launch_stout_level(const DevGeom& g, LinkPlanes<T> U, LinkPlanes<T> Uout, AlgPlanes<T> Q, AlgPlanes<T> S,
                         cudaStream_t s);
-// Lambda and Dir = e^{-i ad_Q} x of a level from the derivative x = X with respect to its smeared links
-template <typename T>
-void launch_lambda(const DevGeom& g, AlgPlanes<T> Q, AlgPlanes<T> X, AlgPlanes<T> Lam, AlgPlanes<T> Dir,
-                   cudaStream_t s);
 // the plaquette terms of Lambda: those of the links at x into Loc, the others into Rem at x
 template <typename T>
 void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
@@ -181,6 +177,10 @@ void launch_plaq_rect(const DevGeom& g, LinkPlanes<T> U, RowPlanes<T> Pl, AlgPla
 // the Wilson force of U
 template <typename T>
 void launch_wilson_force(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> S, AlgPlanes<T> F, cudaStream_t s);
+// the same of smeared links, as Lambda and Dir = e^{-i ad_Q} F of their level
+template <typename T>
+void launch_wilson_lambda(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> S, AlgPlanes<T> Q, AlgPlanes<T> Lam,
+                          AlgPlanes<T> Dir, cudaStream_t s);
 
 // ---- streaming kernels (kernels_update.cu)
 template <typename TU, typename TX>
