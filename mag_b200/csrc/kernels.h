@@ -309,13 +309,13 @@ void launch_wilson_planar(const DevGeom& g, LinkPlanes<double> U, int Rmax, int 
                           LinkPlanes<double> tl, LinkPlanes<double> tl2, dd2* partial, dd2* out, cudaStream_t s);
 // the same for one chain of unitary links in the temporal gauge: out[(R-1) * Tmax + T-1] = the sum over
 // the three directions and the chain's sites.  nx = wilson_gauged_sites must not be 0; scratch G (one
-// direction) and V (three) of ci.V sites, P of L0 L1 L2 sites (one direction), part of
-// wilson_gauged_partials entries; *bad (zeroed by the caller) is set when a link is not unitary, and the
+// direction) and V (three) of ci.V sites, P of L0 L1 L2 sites (one direction), h of nine reals for each
+// of G's padded sites, part of wilson_gauged_partials entries; *bad (zeroed by the caller) is set when a link is not unitary, and the
 // sums are then not the loops.
 int wilson_gauged_sites(const ChainInfo& ci, int Tmax);
 size_t wilson_gauged_partials(const ChainInfo& ci, int Rmax, int Tmax);
 cudaError_t launch_wilson_gauged(const ChainInfo& ci, LinkPlanes<double> U, int Rmax, int Tmax, LinkPlanes<double> G,
-                                 LinkPlanes<double> V, LinkPlanes<double> P, dd2* part, dd2* out, int* bad,
+                                 LinkPlanes<double> V, LinkPlanes<double> P, double* h, dd2* part, dd2* out, int* bad,
                                  cudaStream_t s);
 // sum over sites (coarse sites x = 0 mod coarse_mag when coarse_mag > 0) and
 // npath closed paths of ReTr; dirs[npath][plen], 0..3 forward, 4..7 backward,

@@ -7,16 +7,24 @@
 //   W_i(R,T)(x) = ReTr( S_R(x) T_T(x+R i) S_R(x+T t)^dag T_T(x)^dag )
 // costs two products and one trace per (x, R, T) instead of 2(R+T)-1 products.
 //
-// Unitary links of one chain go further (launch_wilson_gauged): in the gauge
-// g(x, t) = U_t(x, 0) ... U_t(x, t-1) every temporal link but the last time slice's is
-// one, so with the lines continued over the boundary, S_R(x, t + Lt) =
-// P(x) S_R(x, t) P(x + R i)^dag (P the Polyakov line), a loop is
-//   W_i(R, T)(x, t) = ReTr(S_R(x, t) S_R(x, t + T)^dag):
-// no product at all, 18 multiply-adds.  The lines of a few spatial sites over all t
-// stay in shared memory while R grows; nothing but the gauged links is read.
-// 24^3 x 48, R, T <= 8: 10.9 ms by line products, 0.98 ms so.
-#include "gauge_ops.cuh"
+// Unitary links of one chain go further (launch_wilson_gauged): with the temporal lines
+// G(x, t) = U_t(x, 0) ... U_t(x, t-1), T_T(x, t) = G(x, t)^-1 G(x, t + T) and a loop is
+// the trace of two lines,
+//   W_i(R, T)(x, t) = ReTr(A_R(x, t) B_R(x, t + T)^dag),
+//   B_R(x) = G(x) S_R(x) G(x + R i)^dag,  A_R(x) = G(x)^-dag S_R(x) G(x + R i)^-1:
+// no product at all, 18 multiply-adds.  B_R continues over the boundary as
+// B_R(x, t + Lt) = P(x) B_R(x, t) P(x + R i)^dag (P the Polyakov line).  With exactly
+// unitary links A would be B; links are unitary to rounding (or to what an integration
+// left), and G is their product with nothing added.  With H = G G^dag = 1 + h,
+//   A_R(x) = H(x)^-1 B_R(x) H(x + R i)^-1,  H^-1 = 1 - h
+// up to h^2 (1e-20 for links 1e-12 off).  So the loops are those of the links as they
+// are, of any determinant: 1e-16 from 64-bit loops as the line products are, where G made
+// special unitary and A = B are 5e-15 off (and wrong for a determinant that is not one).
+// The lines of a few spatial sites over all t stay on the SM while R grows; nothing but
+// the gauged links and h is read.  24^3 x 48, R, T <= 8, on the device: 10.7 ms by line
+// products, 1.29 ms so (0.98 ms with A = B).
 #include "kernels.h"
+#include "plaq_ops.cuh"
 
 namespace magb {
 
@@ -187,11 +195,9 @@ __global__ void k_finalize_multi(DevGeom g, const dd2* partial, int nq, dd2* out
 }
 
 // ---------------------------------------------------------- temporal gauge
-// Rows' Gram matrix against the unit matrix: the gauge form needs unitary links.
-// Links within rounding of it (1e-15 after a reunitarisation, 1e-13 after a long
-// integration) move a loop by Lt * 1e-12 at most.
-__device__ __forceinline__ bool is_unitary(const mat3<double>& m) {
-    bool ok = true;
+// h = m m^dag - 1 of a nearly unitary m
+__device__ __forceinline__ herm9<double> gram_off_one(const mat3<double>& m) {
+    herm9<double> h;
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
@@ -199,17 +205,80 @@ __device__ __forceinline__ bool is_unitary(const mat3<double>& m) {
             cplx<double> s = cmul<false, true>(m.e[i][0], m.e[j][0]);
             cmac<false, true, false>(s, m.e[i][1], m.e[j][1]);
             cmac<false, true, false>(s, m.e[i][2], m.e[j][2]);
-            ok = ok && fabs(s.re - (i == j ? 1.0 : 0.0)) <= 1e-12 && fabs(s.im) <= 1e-12;
+            if (i == j) {
+                h.d[i] = s.re - 1.0;
+            } else {
+                h.z[2 * (i + j - 1)] = s.re;
+                h.z[2 * (i + j - 1) + 1] = s.im;
+            }
         }
+    return h;
+}
+// The gauge form takes links within 1e-12 of unitary ones (1e-15 after a reunitarisation,
+// 1e-13 after a long integration), NaN not among them
+__device__ __forceinline__ bool is_unitary(const mat3<double>& m) {
+    const herm9<double> h = gram_off_one(m);
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++) ok = ok && fabs(h.d[k]) <= 1e-12;
+#pragma unroll
+    for (int k = 0; k < 6; k++) ok = ok && fabs(h.z[k]) <= 1e-12;
     return ok;
+}
+// h of every site, element k in row k
+struct HermPlanes {
+    double* p;
+    long vpad;
+    __device__ __forceinline__ herm9<double> load(int s) const {
+        herm9<double> h;
+#pragma unroll
+        for (int k = 0; k < 3; k++) h.d[k] = p[k * vpad + s];
+#pragma unroll
+        for (int k = 0; k < 6; k++) h.z[k] = p[(3 + k) * vpad + s];
+        return h;
+    }
+    __device__ __forceinline__ void store(int s, const herm9<double>& h) const {
+#pragma unroll
+        for (int k = 0; k < 3; k++) p[k * vpad + s] = h.d[k];
+#pragma unroll
+        for (int k = 0; k < 6; k++) p[(3 + k) * vpad + s] = h.z[k];
+    }
+};
+// (x, y, z) += sign (x, y, z) h, a row; with CONJ h's transpose, so that a column (x, y, z)^T
+// gets sign h (x, y, z)^T
+template <bool CONJ>
+__device__ __forceinline__ void add_row_times(cplx<double>& x, cplx<double>& y, cplx<double>& z, const herm9<double>& h,
+                                              double sign) {
+    const cplx<double> h01 = mk(sign * h.z[0], sign * (CONJ ? -h.z[1] : h.z[1]));
+    const cplx<double> h02 = mk(sign * h.z[2], sign * (CONJ ? -h.z[3] : h.z[3]));
+    const cplx<double> h12 = mk(sign * h.z[4], sign * (CONJ ? -h.z[5] : h.z[5]));
+    const cplx<double> a = x, b = y, c = z;
+    x = mk(fma(sign * h.d[0], a.re, a.re), fma(sign * h.d[0], a.im, a.im));
+    cmac<false, true, false>(x, b, h01);
+    cmac<false, true, false>(x, c, h02);
+    y = mk(fma(sign * h.d[1], b.re, b.re), fma(sign * h.d[1], b.im, b.im));
+    cmac<false, false, false>(y, a, h01);
+    cmac<false, true, false>(y, c, h12);
+    z = mk(fma(sign * h.d[2], c.re, c.re), fma(sign * h.d[2], c.im, c.im));
+    cmac<false, false, false>(z, a, h02);
+    cmac<false, false, false>(z, b, h12);
+}
+// m (1 + sign h) and (1 + sign h) m
+__device__ __forceinline__ void scale_right(mat3<double>& m, const herm9<double>& h, double sign) {
+#pragma unroll
+    for (int r = 0; r < 3; r++) add_row_times<false>(m.e[r][0], m.e[r][1], m.e[r][2], h, sign);
+}
+__device__ __forceinline__ void scale_left(mat3<double>& m, const herm9<double>& h, double sign) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) add_row_times<true>(m.e[0][c], m.e[1][c], m.e[2][c], h, sign);
 }
 
 constexpr int kGaugeBlock = 64;
-// G(x, t) = U_t(x, 0) ... U_t(x, t-1) and the Polyakov line P(x) = G(x, Lt); one thread
-// per spatial site, the next link loaded while the current one is multiplied
+// G(x, t) = U_t(x, 0) ... U_t(x, t-1), h of it, and the Polyakov line P(x) = G(x, Lt); one
+// thread per spatial site, the next link loaded while the current one is multiplied
 __global__ void __launch_bounds__(kGaugeBlock) k_temporal_gauge(ChainInfo ci, LinkPlanes<double> U,
-                                                                LinkPlanes<double> G, LinkPlanes<double> P,
-                                                                int* bad) {
+                                                                LinkPlanes<double> G, HermPlanes H,
+                                                                LinkPlanes<double> P, int* bad) {
     after_previous();
     const int vs = ci.L[0] * ci.L[1] * ci.L[2];
     const int x = blockIdx.x * kGaugeBlock + threadIdx.x;
@@ -219,9 +288,9 @@ __global__ void __launch_bounds__(kGaugeBlock) k_temporal_gauge(ChainInfo ci, Li
     for (int t = 0; t < ci.L[3]; t++) {
         const mat3<double> next = U.load(3, ci.off + x + vs * (t + 1 < ci.L[3] ? t + 1 : 0));
         G.store(0, x + vs * t, g);
+        H.store(x + vs * t, gram_off_one(g));
         ok = ok && is_unitary(u);
         g = mul(g, u);
-        if (t % 4 == 3 || t + 1 == ci.L[3]) unitarize(g);  // links 1e-15 off would add up over the slices
         u = next;
     }
     P.store(0, x, g);
@@ -243,20 +312,21 @@ __global__ void __launch_bounds__(kBlock) k_gauge_links(ChainInfo ci, LinkPlanes
 }
 
 // One block: NX spatial sites (blockDim = NX times the groups of SL time slices, in
-// whole warps), direction i = blockIdx.y.  Shared memory holds S_R of the sites for
-// t in [0, Lt + Tmax).  A thread extends the lines of its SL slices, then takes the
-// traces of its slices with the slices up to T + SL - 1 later, each read once for SL
-// loops, TC values of T at a time (4 where Tmax is no more: 16^4 to 4 92 -> 86 us).
-// Bound by shared-memory reads (36 cycles per matrix and warp against 9 for a
-// trace's multiply-adds) and the warps that registers and the 72 KB allow: three slices
-// at 168 registers 0.98 ms at 24^3 x 48 (R, T <= 8), four at 208 or 232 1.25, two at
-// 128 1.11; 48^3 x 96: 15.9, 23.8 and 24.9 ms.  A block walks the groups of NX sites
+// whole warps), direction i = blockIdx.y.  Shared memory holds B_R of the sites for
+// t in [0, Lt + Tmax), a thread A_R of its SL slices.  It extends these lines, then takes
+// the traces of its slices with the slices up to T + SL - 1 later, each read once for SL
+// loops, TC values of T at a time (4 where Tmax is no more).  Bound by the FP64 pipe and
+// shared-memory reads in turn, at the twelve warps per SM that the registers allow: two
+// slices at 168 registers 1.29 ms at 24^3 x 48 (R, T <= 8) and 0.152 at 16^4, at 144 or
+// 128 (spills) 1.50 and 1.59; three slices spill (1.63, 0.25), with A read back from
+// shared memory and corrected there 1.28 and 0.172.  Blocks of 64 contiguous bytes per
+// element instead of 128 (four sites): 1.58 ms.  A block walks the groups of NX sites
 // with stride gridDim.x and adds up its
 // part[((i Rmax + R-1) Tmax + T-1) gridDim.x + block].
 constexpr int kGaugedBlocks = 592;  // per direction at most: four per SM
 template <int NX, int SL, int TC>
-__global__ void __maxnreg__(168) k_wloop_gauged(ChainInfo ci, LinkPlanes<double> V, LinkPlanes<double> P,
-                                                      int Rmax, int Tmax, dd2* part) {
+__global__ void __maxnreg__(168) k_wloop_gauged(ChainInfo ci, LinkPlanes<double> V, HermPlanes H,
+                                                      LinkPlanes<double> P, int Rmax, int Tmax, dd2* part) {
     after_previous();
     extern __shared__ __align__(16) unsigned char wsm[];
     cplx<double>* S = reinterpret_cast<cplx<double>*>(wsm);  // [Lt + Tmax][9][NX]
@@ -278,35 +348,61 @@ __global__ void __maxnreg__(168) k_wloop_gauged(ChainInfo ci, LinkPlanes<double>
     const int last = Lt + Tmax - 1;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int x0 = blockIdx.x * NX; x0 < vs; x0 += gridDim.x * NX) {
+        mat3<double> a[SL];
         for (int R = 1; R <= Rmax; R++) {
             const int x = x0 + nx;
             const bool site = x < vs;
             // coordinate along i and the index of x + k i
             const int xi = i == 0 ? x % ci.L[0] : i == 1 ? x / ci.L[0] % ci.L[1] : x / (ci.L[0] * ci.L[1]);
             auto along = [&](int k) { return x + ((xi + k) % Li - xi) * si; };
-            // 1. S_R(t) = S_{R-1}(t) V_i(x + (R-1) i, t) of this thread's slices
-            const int xr = site ? along(R - 1) : 0, xe = site ? along(R) : 0;
-#pragma unroll 1
-            for (int t = t0; t < t0 + SL && t < Lt; t++) {
-                if (!site) {
-                    put(t, zero_mat<double>());
+            const int xr = site ? along(R - 1) : 0, xe = site ? along(R) : 0, xs = site ? x : 0;
+            // 1. this thread's slices: E_R = A_{R-1} V_i(x + (R-1) i), E_1 = H^-1 V_i; B_R = H E_R goes to
+            // shared memory, A_R = E_R H(x + R i)^-1 stays
+#pragma unroll
+            for (int j = 0; j < SL; j++) {
+                const int t = t0 + j;
+                if (t >= Lt) {
+                    set_zero(a[j]);
                     continue;
                 }
                 const mat3<double> v = V.load(i, xr + vs * t);
-                put(t, R == 1 ? v : mul(get(t), v));
+                const herm9<double> h = H.load(xs + vs * t);
+                if (R == 1) {
+                    if (site) a[j] = v;
+                    else set_zero(a[j]);
+                    scale_left(a[j], h, -1.0);
+                } else {
+                    a[j] = mul(a[j], v);
+                }
+                mat3<double> b = a[j];
+                scale_left(b, h, 1.0);
+                put(t, b);
+                scale_right(a[j], H.load(xe + vs * t), -1.0);
             }
-            // 2. the slices past the boundary, from this thread's own slices
+            // 2. the slices past the boundary, from this thread's own slices, a row at a time
 #pragma unroll 1
-            for (int t = t0; t < t0 + SL && t < Lt && t < Tmax; t++)
-                put(Lt + t, site ? mul_nd(mul(P.load(0, x), get(t)), P.load(0, xe)) : zero_mat<double>());
+            for (int t = t0; t < t0 + SL && t < Lt && t < Tmax; t++) {
+#pragma unroll 1
+                for (int r = 0; r < 3; r++) {
+                    cplx<double> y[3] = {};
+#pragma unroll
+                    for (int k = 0; k < 3; k++) {
+                        const cplx<double> p = P.at(0, xs)[(3 * r + k) * MAG_TILE];
+#pragma unroll
+                        for (int c = 0; c < 3; c++) cmac<false, false, false>(y[c], p, S[(t * 9 + 3 * k + c) * NX + nx]);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        cplx<double> z = mk(0.0, 0.0);
+#pragma unroll
+                        for (int k = 0; k < 3; k++)
+                            cmac<false, true, false>(z, y[k], P.at(0, xe)[(3 * c + k) * MAG_TILE]);
+                        S[((Lt + t) * 9 + 3 * r + c) * NX + nx] = z;
+                    }
+                }
+            }
             __syncthreads();
             // 3. traces, TC values of T at a time
-            mat3<double> a[SL];
-#pragma unroll
-            for (int j = 0; j < SL; j++) {
-                if (t0 + j < Lt) a[j] = get(t0 + j);
-                else set_zero(a[j]);
-            }
             for (int Tb = 0; Tb < Tmax; Tb += TC) {
                 double acc[TC];
 #pragma unroll
@@ -374,19 +470,19 @@ static int gauged_fit(const ChainInfo& ci, int Tmax, int sl) {
     return 0;
 }
 static GaugedShape gauged_shape(const ChainInfo& ci, int Tmax) {
-    if (Tmax > ci.L[3]) return {0, 3};
+    if (Tmax > ci.L[3]) return {0, 2};
     const int vs = ci.L[0] * ci.L[1] * ci.L[2];
-    // Three slices per thread read each line for three traces.  Chains that leave an SM fewer
-    // than about six warps of such threads are bound by a thread's own work: one slice each, in
-    // blocks that spread over the SMs.  One measurement, three slices against one: 8^4 to R, T
-    // = 4 40 against 31 us, 12^4 56 against 52, 8^3 x 16 to 8 87 against 62, 10^3 x 20 to 6 80
-    // against 72 (21,000 threads); 12^3 x 24 to 8 109 against 136 (41,000).
-    if (3L * vs * ((ci.L[3] + 2) / 3) < 30000) {
+    // Two slices per thread read each line for two traces.  Chains that leave an SM fewer than
+    // about five warps of such threads are bound by a thread's own work: one slice each, in
+    // blocks that spread over the SMs.  One measurement, one slice against two: 8^4 to R, T = 4
+    // 30 against 39 us, 8^3 x 16 to 8 63 against 86 (12,000 threads of two), 10^3 x 20 to 6 74
+    // against 72 (30,000), 12^4 to 4 54 against 51, 16^4 to 4 115 against 84.
+    if (3L * vs * ((ci.L[3] + 1) / 2) < 25000) {
         int nx = gauged_fit(ci, Tmax, 1);
         while (nx > 4 && 3 * ((vs + nx - 1) / nx) < 148) nx /= 2;
         if (nx) return {nx, 1};
     }
-    return {gauged_fit(ci, Tmax, 3), 3};
+    return {gauged_fit(ci, Tmax, 2), 2};
 }
 int wilson_gauged_sites(const ChainInfo& ci, int Tmax) { return gauged_shape(ci, Tmax).nx; }
 static int gauged_blocks(const ChainInfo& ci, int nx) {
@@ -399,46 +495,49 @@ size_t wilson_gauged_partials(const ChainInfo& ci, int Rmax, int Tmax) {
 }
 
 template <int NX, int SL, int TC>
-static cudaError_t wloop_gauged(const ChainInfo& ci, LinkPlanes<double> V, LinkPlanes<double> P, int Rmax, int Tmax,
-                                dd2* part, cudaStream_t s) {
+static cudaError_t wloop_gauged(const ChainInfo& ci, LinkPlanes<double> V, HermPlanes H, LinkPlanes<double> P, int Rmax,
+                                int Tmax, dd2* part, cudaStream_t s) {
     const int groups = (ci.L[3] + SL - 1) / SL;
     const int threads = (NX * groups + 31) / 32 * 32;
     const size_t smem = (size_t)NX * (ci.L[3] + Tmax) * 144;
     const cudaError_t e =
         cudaFuncSetAttribute(k_wloop_gauged<NX, SL, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024);
     if (e != cudaSuccess) return e;
-    launch_after(k_wloop_gauged<NX, SL, TC>, dim3(gauged_blocks(ci, NX), 3), threads, smem, s, ci, V, P, Rmax, Tmax, part);
+    launch_after(k_wloop_gauged<NX, SL, TC>, dim3(gauged_blocks(ci, NX), 3), threads, smem, s, ci, V, H, P, Rmax,
+                 Tmax, part);
     return cudaGetLastError();
 }
 template <int NX>
-static cudaError_t wloop_gauged(const ChainInfo& ci, int sl, LinkPlanes<double> V, LinkPlanes<double> P, int Rmax,
-                                int Tmax, dd2* part, cudaStream_t s) {
+static cudaError_t wloop_gauged(const ChainInfo& ci, int sl, LinkPlanes<double> V, HermPlanes H, LinkPlanes<double> P,
+                                int Rmax, int Tmax, dd2* part, cudaStream_t s) {
     if (Tmax <= 4)
-        return sl == 1 ? wloop_gauged<NX, 1, 4>(ci, V, P, Rmax, Tmax, part, s)
-                       : wloop_gauged<NX, 3, 4>(ci, V, P, Rmax, Tmax, part, s);
-    return sl == 1 ? wloop_gauged<NX, 1, 8>(ci, V, P, Rmax, Tmax, part, s)
-                   : wloop_gauged<NX, 3, 8>(ci, V, P, Rmax, Tmax, part, s);
+        return sl == 1 ? wloop_gauged<NX, 1, 4>(ci, V, H, P, Rmax, Tmax, part, s)
+                       : wloop_gauged<NX, 2, 4>(ci, V, H, P, Rmax, Tmax, part, s);
+    return sl == 1 ? wloop_gauged<NX, 1, 8>(ci, V, H, P, Rmax, Tmax, part, s)
+                   : wloop_gauged<NX, 2, 8>(ci, V, H, P, Rmax, Tmax, part, s);
 }
 
 // One chain's planar loops in the temporal gauge: G and V, P scratch planes of the
-// chain's V (1 and 3 directions) and L0 L1 L2 sites, local site indices;
+// chain's V (1 and 3 directions) and L0 L1 L2 sites, H nine reals per site, local site indices;
 // out[(R-1) Tmax + T-1] = sum over the directions and sites; *bad is set when a link
 // is not unitary (the sums are then not the loops).
 cudaError_t launch_wilson_gauged(const ChainInfo& ci, LinkPlanes<double> U, int Rmax, int Tmax, LinkPlanes<double> G,
-                                 LinkPlanes<double> V, LinkPlanes<double> P, dd2* part, dd2* out, int* bad,
+                                 LinkPlanes<double> V, LinkPlanes<double> P, double* h, dd2* part, dd2* out, int* bad,
                                  cudaStream_t s) {
+    const HermPlanes H{h, G.vpad};
     const GaugedShape shape = gauged_shape(ci, Tmax);
     const int nx = shape.nx, vs = ci.L[0] * ci.L[1] * ci.L[2];
-    launch_after(k_temporal_gauge, (vs + kGaugeBlock - 1) / kGaugeBlock, kGaugeBlock, 0, s, ci, U, G, P, bad);
+    launch_after(k_temporal_gauge, (vs + kGaugeBlock - 1) / kGaugeBlock, kGaugeBlock, 0, s, ci, U, G, H, P,
+                 bad);
     launch_after(k_gauge_links, dim3((ci.V + kBlock - 1) / kBlock, 3), kBlock, 0, s, ci, U, G, V, bad);
     cudaError_t e = cudaErrorInvalidValue;
     switch (nx) {
-        case 32: e = wloop_gauged<32>(ci, shape.sl, V, P, Rmax, Tmax, part, s); break;
-        case 16: e = wloop_gauged<16>(ci, shape.sl, V, P, Rmax, Tmax, part, s); break;
-        case 8: e = wloop_gauged<8>(ci, shape.sl, V, P, Rmax, Tmax, part, s); break;
-        case 4: e = wloop_gauged<4>(ci, shape.sl, V, P, Rmax, Tmax, part, s); break;
-        case 2: e = wloop_gauged<2>(ci, shape.sl, V, P, Rmax, Tmax, part, s); break;
-        case 1: e = wloop_gauged<1>(ci, shape.sl, V, P, Rmax, Tmax, part, s); break;
+        case 32: e = wloop_gauged<32>(ci, shape.sl, V, H, P, Rmax, Tmax, part, s); break;
+        case 16: e = wloop_gauged<16>(ci, shape.sl, V, H, P, Rmax, Tmax, part, s); break;
+        case 8: e = wloop_gauged<8>(ci, shape.sl, V, H, P, Rmax, Tmax, part, s); break;
+        case 4: e = wloop_gauged<4>(ci, shape.sl, V, H, P, Rmax, Tmax, part, s); break;
+        case 2: e = wloop_gauged<2>(ci, shape.sl, V, H, P, Rmax, Tmax, part, s); break;
+        case 1: e = wloop_gauged<1>(ci, shape.sl, V, H, P, Rmax, Tmax, part, s); break;
         default: return e;
     }
     if (e != cudaSuccess) return e;

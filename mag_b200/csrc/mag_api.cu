@@ -856,23 +856,24 @@ static int wilson_gauged(mag_ctx* ctx, int chain, int Rmax, int Tmax, double* ou
     MAG_TRY(ctx->ensure_gauged(RT, wilson_gauged_partials(ci, Rmax, Tmax)));
     const long vp = ((long)ci.V + MAG_TILE - 1) / MAG_TILE * MAG_TILE;
     const LinkPlanes<double> G{ctx->wg_links, vp}, V{ctx->wg_links + 9 * vp, vp}, P{ctx->wg_links + 36 * vp, vp};
+    double* h = reinterpret_cast<double*>(ctx->wg_links + 45 * vp);
     int* bad = reinterpret_cast<int*>(ctx->wg_out + RT);
     MAG_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     MAG_CUDA(cudaMemsetAsync(bad, 0, sizeof(dd2), ctx->stream));
-    MAG_CUDA(launch_wilson_gauged(ci, ctx->U, Rmax, Tmax, G, V, P, ctx->wg_part, ctx->wg_out, bad, ctx->stream));
+    MAG_CUDA(launch_wilson_gauged(ci, ctx->U, Rmax, Tmax, G, V, P, h, ctx->wg_part, ctx->wg_out, bad, ctx->stream));
     MAG_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
-    std::vector<dd2> h(RT + 1);
-    MAG_CUDA(cudaMemcpyAsync(h.data(), ctx->wg_out, sizeof(dd2) * h.size(), cudaMemcpyDeviceToHost, ctx->stream));
+    std::vector<dd2> sums(RT + 1);
+    MAG_CUDA(cudaMemcpyAsync(sums.data(), ctx->wg_out, sizeof(dd2) * sums.size(), cudaMemcpyDeviceToHost, ctx->stream));
     MAG_TRY(ctx->sync("mag_wilson_loops"));
     int flag = 0;
-    std::memcpy(&flag, &h[RT], sizeof flag);
+    std::memcpy(&flag, &sums[RT], sizeof flag);
     *unitary = flag == 0;
     if (flag) return MAG_OK;
     float ms = 0.f;
     MAG_CUDA(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
     ctx->last_measure_ms = ms;
     const double norm = 3.0 * ci.V;  // perm.size() * V (field-wloop.h:98)
-    for (int k = 0; k < RT; k++) out[k] = (h[k].hi + h[k].lo) / norm;
+    for (int k = 0; k < RT; k++) out[k] = (sums[k].hi + sums[k].lo) / norm;
     return MAG_OK;
 }
 
