@@ -824,7 +824,9 @@ struct mag_ctx {
         free_one(wl_partial);
         free_one(wl_out);
         free_one(wl_lines);
+        wl_partial = wl_out = nullptr;
         wl_lines = nullptr;
+        wl_rmax = wl_tmax = 0;
         MAG_TRY(alloc((void**)&wl_partial, sizeof(dd2) * nb * Rmax));
         MAG_TRY(alloc((void**)&wl_out, sizeof(dd2) * ((size_t)3 * Tmax * nchain * Rmax + nchain)));
         if (lines) MAG_TRY(alloc((void**)&wl_lines, sizeof(cplx<double>) * 9 * (size_t)vpad * (Rmax + 2)));
@@ -861,6 +863,17 @@ struct mag_ctx {
             wg_parts = parts;
         }
         return MAG_OK;
+    }
+
+    void free_gauged() {
+        cudaStreamSynchronize(stream);
+        free_one(wg_links);
+        free_one(wg_part);
+        free_one(wg_out);
+        wg_links = nullptr;
+        wg_part = wg_out = nullptr;
+        wg_parts = 0;
+        wg_rt = 0;
     }
 
     int chain_ok(int c) {

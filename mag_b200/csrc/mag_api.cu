@@ -849,11 +849,11 @@ int mag_wilson_loop(mag_ctx* ctx, int chain, const int r[3], int T, double* out)
     return MAG_OK;
 }
 
-// one chain's planar loops in the temporal gauge; *unitary = false: a link is not unitary, out is not written
+// one chain's planar loops in the temporal gauge (after ensure_gauged); *unitary = false: a link is not
+// unitary, out is not written
 static int wilson_gauged(mag_ctx* ctx, int chain, int Rmax, int Tmax, double* out, bool* unitary) {
     const ChainInfo& ci = ctx->hc[chain];
     const int RT = Rmax * Tmax;
-    MAG_TRY(ctx->ensure_gauged(RT, wilson_gauged_partials(ci, Rmax, Tmax)));
     const long vp = ((long)ci.V + MAG_TILE - 1) / MAG_TILE * MAG_TILE;
     const LinkPlanes<double> G{ctx->wg_links, vp}, V{ctx->wg_links + 9 * vp, vp}, P{ctx->wg_links + 36 * vp, vp};
     double* h = reinterpret_cast<double*>(ctx->wg_links + 45 * vp);
@@ -881,13 +881,22 @@ int mag_wilson_loops(mag_ctx* ctx, int chain, int Rmax, int Tmax, double* out) {
     if (!ctx || !out || Rmax < 1 || Tmax < 1 || Rmax > 64 || Tmax > 64)
         return fail(MAG_ERR_ARG, "mag_wilson_loops: bad arguments");
     MAG_TRY(ctx->chain_ok(chain));
-    if (wilson_gauged_sites(ctx->hc[chain], Tmax) > 0) {
+    const ChainInfo& ci = ctx->hc[chain];
+    if (wilson_gauged_sites(ci, Tmax) > 0) {
+        const int r = ctx->ensure_gauged(Rmax * Tmax, wilson_gauged_partials(ci, Rmax, Tmax));
+        if (r != MAG_OK && r != MAG_ERR_NOMEM) return r;
         bool unitary = false;
-        MAG_TRY(wilson_gauged(ctx, chain, Rmax, Tmax, out, &unitary));
+        if (r == MAG_OK) MAG_TRY(wilson_gauged(ctx, chain, Rmax, Tmax, out, &unitary));
         if (unitary) return MAG_OK;
     }
-    // any links, any extent: the line products of every chain
-    MAG_TRY(ctx->ensure_meas(Rmax, Tmax, true));
+    // any links, any extent, and where the gauged form's 792 bytes per site are not to be had (a single
+    // length R takes 432): the line products of every chain
+    int r = ctx->ensure_meas(Rmax, Tmax, true);
+    if (r == MAG_ERR_NOMEM && ctx->wg_links) {
+        ctx->free_gauged();
+        r = ctx->ensure_meas(Rmax, Tmax, true);
+    }
+    MAG_TRY(r);
     const long vp = ctx->vpad;
     LinkPlanes<double> lines{ctx->wl_lines, vp};
     LinkPlanes<double> tl{ctx->wl_lines + (size_t)Rmax * 9 * vp, vp};
