@@ -57,7 +57,9 @@ int mag_autotune(mag_ctx* ctx, int reps, char* report, size_t len);
 /* use `variant` (a name as in the mag_autotune report) for kernel `family`
    ("force", "staple", "stout_forward", "stout_lambda", "stout_chain") at
    precision 0 (FP64) or 1 (FP32) from now on, in place of the tuner's choice;
-   the context's forces of that precision then take the one-thread-per-link form */
+   the context's forces of that precision then take the one-thread-per-link form,
+   and for FP64 so does the Hamiltonian's smearing, in a mixed context too (there the
+   other FP64 families, and FP32 ones in an FP64 context, have nothing to act on) */
 int mag_set_kernel_variant(mag_ctx* ctx, const char* family, int precision, const char* variant);
 /* number of kernel nodes in the captured trajectory graph (building it if needed) */
 int mag_graph_kernel_count(mag_ctx* ctx, int* kernels);

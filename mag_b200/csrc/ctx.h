@@ -507,7 +507,7 @@ struct mag_ctx {
 
     // The force by the one-thread-per-link kernels with matrix derivatives, whose launch
     // shapes mag_set_kernel_variant selects: after such a call the context's forces of
-    // that precision take this form.
+    // that precision (and the Hamiltonian's smearing, FP64) take this form.
     bool gather[2] = {false, false};
     template <typename T>
     int ensure_gather(StoutBufs<T>& b) {
@@ -552,7 +552,8 @@ struct mag_ctx {
         LinkPlanes<double> cur = U;
         hx(cur);
         for (int k = 0; k < p.n_stout; k++) {
-            launch_stout_level<double>(geom, cur, st64.lv[k], AlgPlanes<double>{}, st64.rem, stream);
+            if (gather[0]) launch_stout_forward<double>(geom, cur, st64.lv[k], st64.Q[k], var<double>(KF_STOUT_FWD), stream);
+            else launch_stout_level<double>(geom, cur, st64.lv[k], AlgPlanes<double>{}, st64.rem, stream);
             cur = st64.lv[k];
             hx(cur);
         }

@@ -727,12 +727,11 @@ int mag_set_kernel_variant(mag_ctx* ctx, const char* family, int precision, cons
     if (f < 0) return fail(MAG_ERR_ARG, std::string("mag_set_kernel_variant: unknown family '") + family + "'");
     if (v < 0 || v >= mag_ctx::variants_of((KernelFamily)f))
         return fail(MAG_ERR_ARG, std::string("mag_set_kernel_variant: no variant '") + variant + "' for " + family);
-    // the variants are the one-thread-per-link kernels': this precision's forces take that form
-    if ((precision == 1) == ctx->mixed) {
-        if (ctx->mixed) MAG_TRY(ctx->ensure_gather(ctx->st32));
-        else MAG_TRY(ctx->ensure_gather(ctx->st64));
-        ctx->gather[precision] = true;
-    }
+    // the variants are the one-thread-per-link kernels': this precision's forces take that form, and
+    // FP64 smearing in any context (a mixed one smears in FP64 for the Hamiltonian)
+    if (ctx->mixed && precision == 1) MAG_TRY(ctx->ensure_gather(ctx->st32));
+    else if (!ctx->mixed && precision == 0) MAG_TRY(ctx->ensure_gather(ctx->st64));
+    ctx->gather[precision] = true;
     MAG_TRY(ctx->ensure_tuned());
     ctx->tune[f][precision] = v;
     if (ctx->graph) {  // the captured trajectory holds the previous choice

@@ -350,7 +350,8 @@ class Chmc:
 
     def set_kernel_variant(self, family: str, precision: str, variant: str) -> None:
         """Use `variant` (e.g. "t1m3", "s6r128") for `family` at "fp64" or "fp32"; the
-        context's forces of that precision then take the one-thread-per-link form."""
+        context's forces of that precision then take the one-thread-per-link form, and for
+        "fp64" the Hamiltonian's smearing too, in a mixed context as well."""
         check(self._lib.mag_set_kernel_variant(self._h, family.encode(), 0 if precision == "fp64" else 1,
                                                variant.encode()), "mag_set_kernel_variant")
 
