@@ -441,7 +441,9 @@ struct mag_ctx {
 
     // A sharded context exchanges halos (hx) after every launch whose output a
     // later kernel reads across the shard boundary: the links whose force is
-    // taken, each smeared level, and Lambda of each level.
+    // taken, each smeared level, and Lambda of each level.  Both forms of the force do
+    // so at the same points and with the same fields, so that shards may differ in it: a halo
+    // of two slices holds what an interior link reads of the double links, one slice around it.
     //
     // Smeared links: the top level's force is the derivative with respect to the top
     // links in the Lie algebra (the force kernel, beta/3 included; everything after it
@@ -519,10 +521,7 @@ struct mag_ctx {
     void force_eval_gather(LinkPlanes<T> Uin, AlgPlanes<T> Fout, StoutBufs<T>& b) {
         hx(Uin);
         if (p.n_stout == 0) {
-            if (iwasaki) {
-                launch_double_link<T>(geom, Uin, wbuf<T>(), stream);
-                hx(wbuf<T>());
-            }
+            if (iwasaki) launch_double_link<T>(geom, Uin, wbuf<T>(), stream);
             launch_force<T>(geom, Uin, wbuf<T>(), Fout, iwasaki, var<T>(KF_FORCE), stream);
         } else {
             LinkPlanes<T> cur = Uin;
@@ -531,14 +530,12 @@ struct mag_ctx {
                 cur = b.lv[k];
                 hx(cur);
             }
-            if (iwasaki) {
-                launch_double_link<T>(geom, cur, wbuf<T>(), stream);
-                hx(wbuf<T>());
-            }
+            if (iwasaki) launch_double_link<T>(geom, cur, wbuf<T>(), stream);
             launch_staple_dagger<T>(geom, cur, wbuf<T>(), b.za, iwasaki, var<T>(KF_STAPLE), stream);
             for (int k = p.n_stout - 1; k >= 0; k--) {
                 LinkPlanes<T> ul = k == 0 ? Uin : b.lv[k - 1];
-                launch_stout_lambda<T>(geom, ul, b.Q[k], b.za, b.lam, b.zp, var<T>(KF_STOUT_LAMBDA), stream);
+                launch_stout_lambda<T>(geom, ul, b.Q[k], b.za, b.lam, b.zp, k == p.n_stout - 1, var<T>(KF_STOUT_LAMBDA),
+                                       stream);
                 hx(b.lam);
                 if (k == 0) launch_stout_chain_force<T>(geom, ul, b.lam, b.zp, Fout, var<T>(KF_STOUT_CHAIN), stream);
                 else launch_stout_chain<T>(geom, ul, b.lam, b.zp, b.za, var<T>(KF_STOUT_CHAIN), stream);
@@ -570,7 +567,7 @@ struct mag_ctx {
                 launch_staple_dagger<T>(geom, L ? b.lv[L - 1] : Uin, wbuf<T>(), L ? b.za : zs, iwasaki, v, stream);
                 break;
             case KF_STOUT_FWD: launch_stout_forward<T>(geom, Uin, b.lv[0], b.Q[0], v, stream); break;
-            case KF_STOUT_LAMBDA: launch_stout_lambda<T>(geom, Uin, b.Q[0], b.za, b.lam, b.zp, v, stream); break;
+            case KF_STOUT_LAMBDA: launch_stout_lambda<T>(geom, Uin, b.Q[0], b.za, b.lam, b.zp, true, v, stream); break;
             case KF_STOUT_CHAIN: launch_stout_chain<T>(geom, Uin, b.lam, b.zp, b.za, v, stream); break;
             default: break;
         }
@@ -669,13 +666,19 @@ struct mag_ctx {
         return MAG_OK;
     }
 
+    // a shard is tuned by itself, without exchanges that no other shard would meet
     int autotune(int reps) {
+        HaloHook* const hook = halo;
+        halo = nullptr;
+        const int r = autotune_alone(reps);
+        halo = hook;
+        return r;
+    }
+    int autotune_alone(int reps) {
         if (mixed) MAG_TRY(tune_precision<float>(reps, st32, U32, F32, Uaux32));
         else MAG_TRY(tune_precision<double>(reps, st64, U, F, Uaux));
-        if (!halo) {
-            if (mixed) MAG_TRY(tune_order<float>(reps, st32, U32, F32));
-            else MAG_TRY(tune_order<double>(reps, st64, U, F));
-        }
+        if (mixed) MAG_TRY(tune_order<float>(reps, st32, U32, F32));
+        else MAG_TRY(tune_order<double>(reps, st64, U, F));
         tuned = true;
         return MAG_OK;
     }

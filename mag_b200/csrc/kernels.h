@@ -125,9 +125,10 @@ void launch_constraint_fixup(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> F, 
 template <typename T>
 void launch_stout_forward(const DevGeom& g, LinkPlanes<T> Uin, LinkPlanes<T> Uout, AlgPlanes<T> Q, int v,
                           cudaStream_t s);
+// top: Z is the staple sum of the action, taken times beta/3
 template <typename T>
 void launch_stout_lambda(const DevGeom& g, LinkPlanes<T> Ul, AlgPlanes<T> Q, LinkPlanes<T> Z, AlgPlanes<T> Lam,
-                         LinkPlanes<T> Zp, int v, cudaStream_t s);
+                         LinkPlanes<T> Zp, bool top, int v, cudaStream_t s);
 template <typename T>
 void launch_stout_chain(const DevGeom& g, LinkPlanes<T> Ul, AlgPlanes<T> Lam, LinkPlanes<T> Zp, LinkPlanes<T> Zout,
                         int v, cudaStream_t s);

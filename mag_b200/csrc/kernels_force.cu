@@ -141,17 +141,20 @@ __global__ void __launch_bounds__(kForceBlock, MINB) k_stout_forward(DevGeom g, 
     Uout.store(mu, st.g, mul(expiQ(q), u));
 }
 
+// top: Z is the staple sum, the action's beta/3 is applied to it here (so that Lambda is
+// the same field as in the plaquette form, whose shards exchange it with this form's)
 template <typename T, int MINB>
 __global__ void __launch_bounds__(kForceBlock, MINB) k_stout_lambda(DevGeom g, LinkPlanes<T> Ul, AlgPlanes<T> Q,
                                                                   LinkPlanes<T> Z, AlgPlanes<T> Lam,
-                                                                  LinkPlanes<T> Zp) {
+                                                                  LinkPlanes<T> Zp, bool top) {
     ChainInfo ci;
     Site st;
     int mu;
     if (!locate_link(g, ci, st, mu)) return;
     herm8<T> lam;
     mat3<T> zp;
-    stout_lambda(Q.load(mu, st.g), Z.load(mu, st.g), Ul.load(mu, st.g), lam, zp);
+    const T scale = top ? (T)(ci.beta / 3.0) : T(1);
+    stout_lambda(Q.load(mu, st.g), scaled(Z.load(mu, st.g), scale), Ul.load(mu, st.g), lam, zp);
     Lam.store(mu, st.g, lam);
     Zp.store(mu, st.g, zp);
 }
@@ -166,8 +169,8 @@ __global__ void __launch_bounds__(kForceBlock, MINB) k_stout_chain(DevGeom g, Li
     if (!locate_link(g, ci, st, mu)) return;
     const mat3<T> z = stout_chain(Ul, Lam, Zp, ci, st, mu);
     if (TO_FORCE) {
-        // thin level: F = i beta/3 TA(U Z)
-        F.store(mu, st.g, i_times_ta(mul(Ul.load(mu, st.g), z), (T)(ci.beta / 3.0)));
+        // thin level: F = i TA(U Z)
+        F.store(mu, st.g, i_times_ta(mul(Ul.load(mu, st.g), z), T(1)));
     } else {
         Zout.store(mu, st.g, z);
     }
@@ -315,10 +318,10 @@ __global__ void __maxnreg__(R) k_stout_chain_split(DevGeom g, LinkPlanes<T> Ul, 
     const T rho = (T)ci.rho;
     if (TO_FORCE) {
         if (w != 0) return;
-        // thin level: F = i beta/3 TA(U Z), Z = Z' e^{iQ} + i rho sum of the parts
+        // thin level: F = i TA(U Z), Z = Z' e^{iQ} + i rho sum of the parts
         mat3<T> z = Zp.load(mu, gs);
         add_to(z, times_i(part_total<NS>(sm, lane), rho));
-        F.store(mu, gs, i_times_ta(mul(Ul.load(mu, gs), z), (T)(ci.beta / 3.0)));
+        F.store(mu, gs, i_times_ta(mul(Ul.load(mu, gs), z), T(1)));
     } else {
         split_store<NS>(Zout, mu, gs, w, [&](int k) {
             const cplx<T> p = part_elem<NS>(sm, k, lane), z = elem_load(Zp, mu, gs, k);
@@ -403,8 +406,8 @@ void launch_stout_forward(const DevGeom& g, LinkPlanes<T> Uin, LinkPlanes<T> Uou
 }
 template <typename T>
 void launch_stout_lambda(const DevGeom& g, LinkPlanes<T> Ul, AlgPlanes<T> Q, LinkPlanes<T> Z, AlgPlanes<T> Lam,
-                         LinkPlanes<T> Zp, int v, cudaStream_t s) {
-#define L_(M) k_stout_lambda<T, M><<<link_blocks(g), kForceBlock, 0, s>>>(g, Ul, Q, Z, Lam, Zp);
+                         LinkPlanes<T> Zp, bool top, int v, cudaStream_t s) {
+#define L_(M) k_stout_lambda<T, M><<<link_blocks(g), kForceBlock, 0, s>>>(g, Ul, Q, Z, Lam, Zp, top);
     MAG_BY_VARIANT(v, L_)
 #undef L_
 }
@@ -453,7 +456,7 @@ void launch_stout_chain_force(const DevGeom& g, LinkPlanes<T> Ul, AlgPlanes<T> L
     template void launch_stout_forward<T>(const DevGeom&, LinkPlanes<T>, LinkPlanes<T>, AlgPlanes<T>, int,     \
                                           cudaStream_t);                                                        \
     template void launch_stout_lambda<T>(const DevGeom&, LinkPlanes<T>, AlgPlanes<T>, LinkPlanes<T>,          \
-                                         AlgPlanes<T>, LinkPlanes<T>, int, cudaStream_t);                      \
+                                         AlgPlanes<T>, LinkPlanes<T>, bool, int, cudaStream_t);                \
     template void launch_stout_chain<T>(const DevGeom&, LinkPlanes<T>, AlgPlanes<T>, LinkPlanes<T>,           \
                                         LinkPlanes<T>, int, cudaStream_t);                                     \
     template void launch_stout_chain_force<T>(const DevGeom&, LinkPlanes<T>, AlgPlanes<T>, LinkPlanes<T>,     \

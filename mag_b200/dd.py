@@ -7,7 +7,7 @@ reference keeps such a slab per MPI rank in a qlat Field with an expanded Geomet
 (expansion(2, 2, 2, 2), field-hmc.h:777-781) and refreshes its halo with
 fetch_expanded_chart before every force (field-hmc.h:544-558); here the halos are
 refreshed after every kernel whose output is read across a slab boundary (links,
-each stout level, the double links, each level's Lambda), the sums of
+each stout level, each level's Lambda), the sums of
 get_hamiltonian are added over the slabs (its MPI_Allreduce, field-hmc.h:628) and
 every slab takes the same accept decision (the MPI_Bcast of field-hmc.h:823).
 
