@@ -259,9 +259,17 @@ struct mag_ctx {
             MAG_TRY(alloc_links(b.lv[k]));
             MAG_TRY(alloc_alg(b.Q[k]));
         }
-        // a forward-only set needs the six plane fields of the smearing (in rem) and nothing else
-        if (backward || p.n_stout > 0) MAG_TRY(alloc_alg(b.rem, backward ? 12 : 6));
-        if (!backward) return MAG_OK;
+        if (compact) {
+            if (backward && p.n_stout > 0) {
+                MAG_TRY(alloc_alg(b.lam));
+                MAG_TRY(ensure_gather(b));
+            }
+            return MAG_OK;
+        }
+        // six plane fields (in rem) serve the smearing and the thin Wilson force
+        const bool six = !backward || (p.n_stout == 0 && !iwasaki);
+        if (backward || p.n_stout > 0) MAG_TRY(alloc_alg(b.rem, six ? 6 : 12));
+        if (six) return MAG_OK;
         MAG_TRY(alloc_alg(b.loc));
         if (p.n_stout > 0) {
             MAG_TRY(alloc_alg(b.lam));
@@ -315,8 +323,28 @@ struct mag_ctx {
         return MAG_OK;
     }
 
+    // Without the fields of the plaquette form, its forces and smearing by the one-thread-per-link
+    // kernels: 128 (smeared or mixed) to 1024 bytes per site less (thin FP64 Iwasaki: 3392 of 4416).
+    // Taken by a context whose fields do not fit otherwise.
+    bool compact = false;
+
+    // the arena and the fields in it
+    int alloc_arena(int n, long nchunk) {
+        arena = nullptr;
+        arena_used = 0;
+        carve = true;
+        MAG_TRY(alloc_fields(n, nchunk));  // counts
+        carve = false;
+        MAG_TRY(alloc((void**)&arena, arena_used));
+        arena_used = 0;
+        carve = true;
+        MAG_TRY(alloc_fields(n, nchunk));
+        carve = false;
+        return MAG_OK;
+    }
+
     // shard != nullptr: {nshards, rank, halo} of a lattice split along x3 (n == 1)
-    int init(const mag_params* params, int n, const int* shard = nullptr) {
+    int init(const mag_params* params, int n, const int* shard = nullptr, bool small = false) {
         p = params[0];
         nchain = n;
         if (shard) {
@@ -379,14 +407,14 @@ struct mag_ctx {
         MAG_CUDA(cudaEventCreate(&ev0));
         MAG_CUDA(cudaEventCreate(&ev1));
         const long nchunk = vpad / MAG_CHUNK;
-        carve = true;
-        MAG_TRY(alloc_fields(n, nchunk));  // counts
-        carve = false;
-        MAG_TRY(alloc((void**)&arena, arena_used));
-        arena_used = 0;
-        carve = true;
-        MAG_TRY(alloc_fields(n, nchunk));
-        carve = false;
+        compact = small;
+        int fields = alloc_arena(n, nchunk);
+        if (fields == MAG_ERR_NOMEM && !compact) {
+            compact = true;
+            fields = alloc_arena(n, nchunk);
+        }
+        MAG_TRY(fields);
+        gather[0] = gather[1] = compact;
         std::vector<uint16_t> c2c(nchunk, 0);
         for (int c = 0; c < n; c++)
             for (long k = hc[c].off / MAG_CHUNK; k < (hc[c].off + hc[c].V + MAG_CHUNK - 1) / MAG_CHUNK; k++)

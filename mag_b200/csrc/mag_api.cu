@@ -647,6 +647,7 @@ int mag_time_kernel(mag_ctx* ctx, const char* which, int reps, double* ms) {
     } else if (w == "stout_level" || w == "lambda" || w == "plaq_chain" || w == "chain_gather" ||
                w == "plaq_force") {
         if (L == 0 && w != "plaq_force") return fail(MAG_ERR_STATE, "mag_time_kernel: no stout levels in this context");
+        if (ctx->compact) return fail(MAG_ERR_STATE, "mag_time_kernel: this context has no fields for '" + w + "'");
         fn = [&]() {
             if (m) ctx->launch_smear<float>(w, ctx->st32, ctx->U32, ctx->F32);
             else ctx->launch_smear<double>(w, ctx->st64, ctx->U, ctx->F);

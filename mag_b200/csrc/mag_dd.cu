@@ -257,16 +257,22 @@ int mag_dd_create(const mag_params* p, int nshards, int halo, mag_dd** out) {
     d->n = nshards;
     d->h = halo;
     cudaGetDevice(&d->device);
-    for (int r = 0; r < nshards; r++) {
-        mag_ctx* c = new mag_ctx();
-        const int spec[3] = {nshards, r, halo};
-        const int rc = c->init(p, 1, spec);
-        if (rc != MAG_OK) {
-            delete c;
+    // every shard in its smallest form if they do not all fit otherwise
+    for (const bool small : {false, true}) {
+        int rc = MAG_OK;
+        for (int r = 0; r < nshards && rc == MAG_OK; r++) {
+            mag_ctx* c = new mag_ctx();
+            const int spec[3] = {nshards, r, halo};
+            rc = c->init(p, 1, spec, small);
+            d->shards.push_back(c);
+        }
+        if (rc == MAG_OK) break;
+        for (auto c : d->shards) delete c;
+        d->shards.clear();
+        if (rc != MAG_ERR_NOMEM || small) {
             delete d;
             return rc;
         }
-        d->shards.push_back(c);
     }
     d->ready.resize(nshards);
     d->copied.resize(nshards);

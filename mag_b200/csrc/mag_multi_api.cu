@@ -105,15 +105,22 @@ int mag_multi_create(const mag_params* fine, double rho, double eta_sqr, mag_mul
     mag_multi* m = new mag_multi();
     m->rho = rho;
     m->eta_sqr = eta_sqr;
-    m->f = new mag_ctx();
-    m->c = new mag_ctx();
-    int r = m->f->init(&pf, 1);
-    if (r == MAG_OK) r = m->c->init(&pc, 1);
-    if (r == MAG_OK) r = m->c->alloc_alg(m->lam);
-    if (r == MAG_OK) r = m->c->alloc_links(m->zp);
-    const long nb = 4 * ((m->c->hc[0].V + 127) / 128);
-    if (r == MAG_OK) r = m->c->alloc((void**)&m->partial, sizeof(dd2) * nb);
-    if (r == MAG_OK) r = m->c->alloc((void**)&m->energy, sizeof(dd2));
+    int r = MAG_OK;
+    // both lattices in their smallest form if they do not fit otherwise
+    for (const bool small : {false, true}) {
+        delete m->f;
+        delete m->c;
+        m->f = new mag_ctx();
+        m->c = new mag_ctx();
+        r = m->f->init(&pf, 1, nullptr, small);
+        if (r == MAG_OK) r = m->c->init(&pc, 1, nullptr, small);
+        if (r == MAG_OK) r = m->c->alloc_alg(m->lam);
+        if (r == MAG_OK) r = m->c->alloc_links(m->zp);
+        const long nb = r == MAG_OK ? 4 * ((m->c->hc[0].V + 127) / 128) : 0;
+        if (r == MAG_OK) r = m->c->alloc((void**)&m->partial, sizeof(dd2) * nb);
+        if (r == MAG_OK) r = m->c->alloc((void**)&m->energy, sizeof(dd2));
+        if (r != MAG_ERR_NOMEM) break;
+    }
     if (r == MAG_OK) r = m->f->ensure_tuned();
     if (r != MAG_OK) {
         delete m;
