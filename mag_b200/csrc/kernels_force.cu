@@ -138,7 +138,8 @@ __global__ void __launch_bounds__(kForceBlock, MINB) k_stout_forward(DevGeom g, 
     const mat3<T> u = Uin.load(mu, st.g);
     const herm8<T> q = i_times_ta(mul_nd(stp, u), (T)(-ci.rho));
     Q.store(mu, st.g, q);
-    Uout.store(mu, st.g, mul(expiQ(q), u));
+    if constexpr (sizeof(T) == 4) Uout.store(mu, st.g, exp_apply(q, u));
+    else Uout.store(mu, st.g, mul(expiQ(q), u));
 }
 
 // top: Z is the staple sum, the action's beta/3 is applied to it here (so that Lambda is

@@ -78,7 +78,7 @@ struct site_terms {
 
 // S = (P - P^dag) / 2i of every plaquette (plane fields 0..5 of S)
 template <typename T>
-__global__ void __launch_bounds__(kPlaqBlock, 4) k_plaq_sin(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S) {
+__global__ void __launch_bounds__(kPlaqBlock, sizeof(T) == 8 ? 4 : 3) k_plaq_sin(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S) {
     after_previous();
     ChainInfo ci;
     Site st;
@@ -87,9 +87,7 @@ __global__ void __launch_bounds__(kPlaqBlock, 4) k_plaq_sin(DevGeom g, LinkPlane
     int p, q;
     plane_of(w, p, q);
     const int gp = nb_sel(ci, st, p, 1), gq = nb_sel(ci, st, q, 1);
-    const mat3<T> P =
-        plaquette(U.load_rows01(p, st.g), U.load(q, gp), U.load(p, gq), U.load_rows01(q, st.g));
-    S.store(w, st.g, plaq_sin(P, T(1)));
+    S.store(w, st.g, herm_convert<T>(plaq_sin(plaquette_wide(U, st.g, gp, gq, p, q), 1.0)));
 }
 
 // -i TA(stp U^dag) of link (x, mu), stp its six staples, from the plaquettes at x and x - nu
@@ -147,9 +145,7 @@ __global__ void __launch_bounds__(kPlaqBlock, sizeof(T) == 8 ? 2 : 4) k_plaq(Dev
     const int w = threadIdx.x >> 5;
     int p, q;
     plane_of(w, p, q);
-    const mat3<T> x = mul_2r(U.load_rows01(p, st.g), U.load(q, nb_sel(ci, st, p, 1)));
-    const mat3<T> y = mul_su3(U.load_rows01(q, st.g), U.load(p, nb_sel(ci, st, q, 1)));
-    Pl.store(w, st.g, mul_nd_2r(x, y));
+    Pl.store(w, st.g, convert<T>(plaquette_wide(U, st.g, nb_sel(ci, st, p, 1), nb_sel(ci, st, q, 1), p, q)));
 }
 
 // Iwasaki force i TA(U A^dag) without its beta/3, A = c0 staples + c1 rectangles
@@ -187,7 +183,8 @@ __global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_rect(DevGeom g, LinkP
         auto fresh = []() {
             if (MINB > 1) asm volatile("" ::: "memory");
         };
-        herm8<T> lb, lc, t;
+        // the rectangles' terms are added up before R0, which is ten times their size
+        herm8<T> lb, lc, t, u;
         {
             const int gm = nb_sel(ci, st, q, -1);
             mat3<T> x = mul_dn_2r(U.load_cols01(q, gm), Pl.load(w, gm));
@@ -208,16 +205,14 @@ __global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_rect(DevGeom g, LinkP
             herm_add(lb, r);
             herm_add(lc, transport_dn(Pl.load(w, st.g), r));
         }
-        herm_add(lb, t);
-        herm_add(lc, t);
         fresh();
         {
             mat3<T> x = mul_2r(U.load_rows01(p, st.g), Pl.load(w, nb_sel(ci, st, p, 1)));
             x = mul_nd_2r(x, U.load(p, st.g));
-            const herm8<T> r = plaq_sin(mul_su3(x, Pl.load(w, st.g)), k1);  // RA
-            herm_add(lc, r);
-            herm_add(t, r);
+            u = plaq_sin(mul_su3(x, Pl.load(w, st.g)), k1);  // RA
+            herm_add(lc, u);
         }
+        herm_add(lc, t);
         fresh();
         Rem.store(ip, st.g, transport_dn(U.load(q, st.g), lc));
         {
@@ -225,17 +220,19 @@ __global__ void __launch_bounds__(kPlaqBlock, MINB) k_plaq_rect(DevGeom g, LinkP
             x = mul_2r(x, Pl.load(w, nb_sel(ci, st, q, 1)));
             const herm8<T> r = plaq_sin(mul_nd_su3(x, U.load(q, st.g)), k1);  // RD
             herm_add(lb, r);
-            herm_add(t, r);
+            herm_add(u, r);
         }
+        herm_add(lb, t);
         fresh();
 #pragma unroll
         for (int k = 0; k < 8; k++) lb.h[k] = -lb.h[k];
         Rem.store(iq, st.g, transport_dn(U.load(p, st.g), lb));
         herm8<T> y = sm.get(ip, lane);
 #pragma unroll
-        for (int k = 0; k < 8; k++) y.h[k] = -t.h[k] - y.h[k];
+        for (int k = 0; k < 8; k++) y.h[k] = -t.h[k] - (u.h[k] + y.h[k]);
         sm.put(ip, lane, y);
-        herm_add(t, sm.get(iq, lane));
+        herm_add(u, sm.get(iq, lane));
+        herm_add(t, u);
         sm.put(iq, lane, t);
     }
     __syncthreads();
@@ -331,16 +328,24 @@ template <typename T, bool TOP>
 __device__ __forceinline__ herm8<T> gathered(const AlgPlanes<T>& Loc, const AlgPlanes<T>& Rem, const AlgPlanes<T>& Dir,
                                              const ChainInfo& ci, const Site& st, int mu) {
     herm8<T> x = Loc.load(mu, st.g);
-    if (!TOP) herm_add(x, Dir.load(mu, st.g));
+    herm8<T> d = herm_zero<T>();
+    if (!TOP) d = Dir.load(mu, st.g);
     herm8<T> r[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) {
         const int nu = i + (i >= mu ? 1 : 0);
         r[i] = Rem.load(3 * mu + i, nb_sel(ci, st, nu, -1));
     }
+    // in double: the terms are of one size and an FP32 addition's rounding is as large as theirs;
+    // bound by memory, the kernels take no longer
 #pragma unroll
-    for (int i = 0; i < 3; i++) herm_add(x, r[i]);
-    if (TOP) x = scaled(x, (T)(ci.beta / 3.0));
+    for (int k = 0; k < 8; k++) {
+        double a = (double)x.h[k];
+        if (!TOP) a += (double)d.h[k];
+        a = ((a + (double)r[0].h[k]) + (double)r[1].h[k]) + (double)r[2].h[k];
+        if (TOP) a *= ci.beta / 3.0;
+        x.h[k] = (T)a;
+    }
     return x;
 }
 
