@@ -214,7 +214,6 @@ int mag_action(mag_ctx* ctx, int chain, double* plaq, double* rect, double* acti
     if (!ctx) return MAG_ERR_ARG;
     MAG_TRY(ctx->chain_ok(chain));
     LinkPlanes<double> top = ctx->smear64();
-    MAG_TRY(ctx->ensure_h_sums());
     const OneChain one = ctx->one_chain(chain);
     launch_action_sums(ctx->geom, top, true, ctx->partial, ctx->sums, SLOT_PLAQ_THIN, SLOT_RECT_THIN, ctx->stream,
                        &one);
@@ -232,7 +231,6 @@ int mag_action(mag_ctx* ctx, int chain, double* plaq, double* rect, double* acti
 int mag_plaquette(mag_ctx* ctx, int chain, double* avg) {
     if (!ctx || !avg) return MAG_ERR_ARG;
     MAG_TRY(ctx->chain_ok(chain));
-    MAG_TRY(ctx->ensure_h_sums());
     const OneChain one = ctx->one_chain(chain);
     launch_action_sums(ctx->geom, ctx->U, false, ctx->partial, ctx->sums, SLOT_SCRATCH, SLOT_SCRATCH, ctx->stream,
                        &one);
@@ -247,7 +245,6 @@ int mag_plaquette(mag_ctx* ctx, int chain, double* avg) {
 int mag_kinetic(mag_ctx* ctx, int chain, double* kin) {
     if (!ctx || !kin) return MAG_ERR_ARG;
     MAG_TRY(ctx->chain_ok(chain));
-    MAG_TRY(ctx->ensure_h_sums());
     const OneChain one = ctx->one_chain(chain);
     launch_kinetic_sum(ctx->geom, ctx->P, ctx->partial, ctx->sums, SLOT_SCRATCH, ctx->stream, &one);
     MAG_TRY(ctx->check("mag_kinetic"));
