@@ -529,7 +529,7 @@ struct mag_ctx {
     // grows by 15-30% with the transports of its angles.
     template <typename T>
     void forward_level(LinkPlanes<T> cur, StoutBufs<T>& b, int k) {
-        if constexpr (sizeof(T) == 8) launch_stout_level<T>(geom, cur, b.lv[k], b.Q[k], b.rem, stream);
+        if constexpr (sizeof(T) == 8) launch_stout_level(geom, cur, b.lv[k], b.Q[k], b.rem, stream);
         else launch_stout_forward<T>(geom, cur, b.lv[k], b.Q[k], 3, stream);
     }
     // the plaquettes' rows share the double links' buffer (576 of 576 bytes per site in FP64, 288 of 320 in FP32)
@@ -581,7 +581,7 @@ struct mag_ctx {
         hx(cur);
         for (int k = 0; k < p.n_stout; k++) {
             if (gather[0]) launch_stout_forward<double>(geom, cur, st64.lv[k], st64.Q[k], var<double>(KF_STOUT_FWD), stream);
-            else launch_stout_level<double>(geom, cur, st64.lv[k], AlgPlanes<double>{}, st64.rem, stream);
+            else launch_stout_level(geom, cur, st64.lv[k], AlgPlanes<double>{}, st64.rem, stream);
             cur = st64.lv[k];
             hx(cur);
         }

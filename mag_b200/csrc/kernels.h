@@ -137,10 +137,9 @@ void launch_stout_chain_force(const DevGeom& g, LinkPlanes<T> Ul, AlgPlanes<T> L
                               int v, cudaStream_t s);
 
 // ---- stout smearing on plaquettes (kernels_smear.cu); S: six plane fields, Rem: twelve
-// one forward level: U' = e^{iQ} U, and Q where it is given a place, from the plaquettes S of U
-template <typename T>
-void launch_stout_level(const DevGeom& g, LinkPlanes<T> U, LinkPlanes<T> Uout, AlgPlanes<T> Q, AlgPlanes<T> S,
-                        cudaStream_t s);
+// one forward level (FP64): U' = e^{iQ} U, and Q where it is given a place, from the plaquettes S of U
+void launch_stout_level(const DevGeom& g, LinkPlanes<double> U, LinkPlanes<double> Uout, AlgPlanes<double> Q,
+                        AlgPlanes<double> S, cudaStream_t s);
 // the plaquette terms of Lambda: those of the links at x into Loc, the others into Rem at x
 template <typename T>
 void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgPlanes<T> Loc, AlgPlanes<T> Rem,

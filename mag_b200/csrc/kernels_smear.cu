@@ -110,15 +110,14 @@ __device__ __forceinline__ herm8<T> staple_angle(const LinkPlanes<T>& U, const A
 // Q = -i rho TA(stp U^dag) (field-multi.h:32-39), U' = e^{iQ} U.  Q is kept for the derivative
 // where the caller gives a place for it; without, 256 of 1792 B per site and level less go to
 // memory, which bounds it (Hamiltonian of 24^3 x 48 with three levels 1.80 -> 1.72 ms)
-template <typename T>
-__global__ void __launch_bounds__(kLinkBlock, 5) k_stout_apply(DevGeom g, LinkPlanes<T> U, AlgPlanes<T> S,
-                                                            LinkPlanes<T> Uout, AlgPlanes<T> Q) {
+__global__ void __launch_bounds__(kLinkBlock, 5) k_stout_apply(DevGeom g, LinkPlanes<double> U, AlgPlanes<double> S,
+                                                            LinkPlanes<double> Uout, AlgPlanes<double> Q) {
     after_previous();
     ChainInfo ci;
     Site st;
     if (!locate_tile(g, ci, st)) return;
     const int mu = threadIdx.x >> 5;
-    const herm8<T> q = scaled(staple_angle(U, S, ci, st, mu), (T)ci.rho);
+    const herm8<double> q = scaled(staple_angle(U, S, ci, st, mu), ci.rho);
     if (Q.p) Q.store(mu, st.g, q);
     Uout.store(mu, st.g, exp_times(q, U.load(mu, st.g)));
 }
@@ -447,11 +446,10 @@ unsigned tiles(const DevGeom& g) { return (unsigned)(g.vpad / MAG_TILE); }
 
 }  // namespace
 
-template <typename T>
-void launch_stout_level(const DevGeom& g, LinkPlanes<T> U, LinkPlanes<T> Uout, AlgPlanes<T> Q, AlgPlanes<T> S,
-                        cudaStream_t s) {
-    launch_after(k_plaq_sin<T>, tiles(g), kPlaqBlock, 0, s, g, U, S);
-    launch_after(k_stout_apply<T>, tiles(g), kLinkBlock, 0, s, g, U, S, Uout, Q);
+void launch_stout_level(const DevGeom& g, LinkPlanes<double> U, LinkPlanes<double> Uout, AlgPlanes<double> Q,
+                        AlgPlanes<double> S, cudaStream_t s) {
+    launch_after(k_plaq_sin<double>, tiles(g), kPlaqBlock, 0, s, g, U, S);
+    launch_after(k_stout_apply, tiles(g), kLinkBlock, 0, s, g, U, S, Uout, Q);
 }
 template <typename T>
 void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
@@ -510,8 +508,6 @@ void launch_wilson_lambda(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> S, Alg
 }
 
 #define MAG_INSTANTIATE(T)                                                                                          \
-    template void launch_stout_level<T>(const DevGeom&, LinkPlanes<T>, LinkPlanes<T>, AlgPlanes<T>, AlgPlanes<T>,   \
-                                        cudaStream_t);                                                              \
     template void launch_wilson_lambda<T>(const DevGeom&, LinkPlanes<T>, AlgPlanes<T>, AlgPlanes<T>, AlgPlanes<T>,  \
                                           AlgPlanes<T>, cudaStream_t);                                              \
     template void launch_plaq_chain<T>(const DevGeom&, LinkPlanes<T>, AlgPlanes<T>, AlgPlanes<T>, AlgPlanes<T>,     \

@@ -297,53 +297,40 @@ MAG_HD mat3<double> plaquette_wide(const LinkPlanes<float>& U, int g, int gp, in
 
 // e^{iQ} U = (f0 + f1 Q + f2 Q^2) U of a special unitary U: rows 0, 1 of e^{iQ} and of
 // the product, the third reconstructed; the coefficients are those of expiQ
-template <typename T>
-MAG_HD mat3<T> exp_times(const herm8<T>& q, const mat3<T>& U) {
-    const T h0 = q.h[0], h1 = q.h[1], h2 = -q.h[0] - q.h[1];
-    const cplx<T> z01 = mk(q.h[2], q.h[3]), z02 = mk(q.h[4], q.h[5]), z12 = mk(q.h[6], q.h[7]);
-    const T n01 = fmaT(z01.re, z01.re, z01.im * z01.im);
-    const T n02 = fmaT(z02.re, z02.re, z02.im * z02.im);
-    const T n12 = fmaT(z12.re, z12.re, z12.im * z12.im);
+MAG_HD mat3<double> exp_times(const herm8<double>& q, const mat3<double>& U) {
+    const double h0 = q.h[0], h1 = q.h[1], h2 = -q.h[0] - q.h[1];
+    const cplx<double> z01 = mk(q.h[2], q.h[3]), z02 = mk(q.h[4], q.h[5]), z12 = mk(q.h[6], q.h[7]);
+    const double n01 = fmaT(z01.re, z01.re, z01.im * z01.im);
+    const double n02 = fmaT(z02.re, z02.re, z02.im * z02.im);
+    const double n12 = fmaT(z12.re, z12.re, z12.im * z12.im);
     // rows 0, 1 of Q^2 (Hermitian): 00, 11 and 01, 02, 12
-    const T s00 = fmaT(h0, h0, n01 + n02), s11 = fmaT(h1, h1, n01 + n12), s22 = fmaT(h2, h2, n02 + n12);
-    cplx<T> s01 = mk(-h2 * z01.re, -h2 * z01.im), s02 = mk(-h1 * z02.re, -h1 * z02.im),
+    const double s00 = fmaT(h0, h0, n01 + n02), s11 = fmaT(h1, h1, n01 + n12), s22 = fmaT(h2, h2, n02 + n12);
+    cplx<double> s01 = mk(-h2 * z01.re, -h2 * z01.im), s02 = mk(-h1 * z02.re, -h1 * z02.im),
             s12 = mk(-h0 * z12.re, -h0 * z12.im);
     cmac<false, true, false>(s01, z02, z12);
     cmac<false, false, false>(s02, z01, z12);
     cmac<true, false, false>(s12, z01, z02);
-    const T c1 = T(0.5) * (s00 + s11 + s22);
-    if (c1 == T(0)) return U;  // the reference's c1 = 0 branch (field-hmc.h:95)
+    const double c1 = 0.5 * (s00 + s11 + s22);
+    if (c1 == 0.0) return U;  // the reference's c1 = 0 branch (field-hmc.h:95)
     // det Q = Tr Q^3 / 3
-    const cplx<T> p = cmul<false, false>(z01, z12);
-    T c0 = fmaT(p.re, z02.re, p.im * z02.im);
-    c0 = fmaT(T(2), c0, h0 * h1 * h2);
+    const cplx<double> p = cmul<false, false>(z01, z12);
+    double c0 = fmaT(p.re, z02.re, p.im * z02.im);
+    c0 = fmaT(2.0, c0, h0 * h1 * h2);
     c0 = fmaT(-h0, n12, c0);
     c0 = fmaT(-h1, n02, c0);
     c0 = fmaT(-h2, n01, c0);
-    cplx<T> f0, f1, f2;
-    if constexpr (sizeof(T) == 4) {
-        ch_coef_f c;
-        if (!ch_series<false>(c0, c1, c)) c = ch_to_float(ch_coefficients<false>((double)c0, (double)c1));
-        f0 = mk(c.f0r, c.f0i);
-        f1 = mk(c.f1r, c.f1i);
-        f2 = mk(c.f2r, c.f2i);
-    } else {
-        double f[6];
-        if (ch_series_exp_d(c0, c1, f)) {
-            f0 = mk<T>(f[0], f[1]);
-            f1 = mk<T>(f[2], f[3]);
-            f2 = mk<T>(f[4], f[5]);
-        } else {
-            const ch_coef c = ch_coefficients<false>(c0, c1);
-            f0 = mk<T>(c.f0r, c.f0i);
-            f1 = mk<T>(c.f1r, c.f1i);
-            f2 = mk<T>(c.f2r, c.f2i);
-        }
+    double f[6];
+    if (!ch_series_exp_d(c0, c1, f)) {
+        const ch_coef c = ch_coefficients<false>(c0, c1);
+        f[0] = c.f0r, f[1] = c.f0i;
+        f[2] = c.f1r, f[3] = c.f1i;
+        f[4] = c.f2r, f[5] = c.f2i;
     }
-    mat3<T> e;
-    auto diag = [&](T x, T s) { return mk(fmaT(f2.re, s, fmaT(f1.re, x, f0.re)), fmaT(f2.im, s, fmaT(f1.im, x, f0.im))); };
-    auto off = [&](cplx<T> x, cplx<T> s) {
-        cplx<T> r = cmul<false, false>(f1, x);
+    const cplx<double> f0 = mk(f[0], f[1]), f1 = mk(f[2], f[3]), f2 = mk(f[4], f[5]);
+    mat3<double> e;
+    auto diag = [&](double x, double s) { return mk(fmaT(f2.re, s, fmaT(f1.re, x, f0.re)), fmaT(f2.im, s, fmaT(f1.im, x, f0.im))); };
+    auto off = [&](cplx<double> x, cplx<double> s) {
+        cplx<double> r = cmul<false, false>(f1, x);
         cmac<false, false, false>(r, f2, s);
         return r;
     };
