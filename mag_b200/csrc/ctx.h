@@ -870,7 +870,7 @@ struct mag_ctx {
         return MAG_OK;
     }
 
-    // loops in the temporal gauge: gauge, gauged links, Polyakov lines and nine reals per site of the
+    // loops in the temporal gauge: gauge, gauged links, Polyakov lines and ten reals per site of the
     // largest chain, block partials, results and the unitarity flag
     cplx<double>* wg_links = nullptr;
     dd2 *wg_part = nullptr, *wg_out = nullptr;
@@ -879,7 +879,7 @@ struct mag_ctx {
     int ensure_gauged(int RT, size_t parts) {
         if (!wg_links) {
             const size_t vp = ((size_t)max_v + MAG_TILE - 1) / MAG_TILE * MAG_TILE;
-            MAG_TRY(alloc((void**)&wg_links, (sizeof(cplx<double>) * 9 * 5 + sizeof(double) * 9) * vp));
+            MAG_TRY(alloc((void**)&wg_links, (sizeof(cplx<double>) * 9 * 5 + sizeof(double) * 10) * vp));
         }
         if (RT > wg_rt) {
             cudaStreamSynchronize(stream);

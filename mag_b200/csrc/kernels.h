@@ -309,8 +309,8 @@ void launch_wilson_planar(const DevGeom& g, LinkPlanes<double> U, int Rmax, int 
                           LinkPlanes<double> tl, LinkPlanes<double> tl2, dd2* partial, dd2* out, cudaStream_t s);
 // the same for one chain of unitary links in the temporal gauge: out[(R-1) * Tmax + T-1] = the sum over
 // the three directions and the chain's sites.  nx = wilson_gauged_sites must not be 0; scratch G (one
-// direction) and V (three) of ci.V sites, P of L0 L1 L2 sites (one direction), h of nine reals for each
-// of G's padded sites, part of wilson_gauged_partials entries; *bad (zeroed by the caller) is set when a link is not unitary, and the
+// direction) and V (three) of ci.V sites, P of L0 L1 L2 sites (one direction), h of ten reals (16-byte
+// aligned) for each of G's padded sites, part of wilson_gauged_partials entries; *bad (zeroed by the caller) is set when a link is not unitary, and the
 // sums are then not the loops.
 int wilson_gauged_sites(const ChainInfo& ci, int Tmax);
 size_t wilson_gauged_partials(const ChainInfo& ci, int Rmax, int Tmax);

@@ -886,7 +886,7 @@ int mag_wilson_loops(mag_ctx* ctx, int chain, int Rmax, int Tmax, double* out) {
         if (r == MAG_OK) MAG_TRY(wilson_gauged(ctx, chain, Rmax, Tmax, out, &unitary));
         if (unitary) return MAG_OK;
     }
-    // any links, any extent, and where the gauged form's 792 bytes per site are not to be had (a single
+    // any links, any extent, and where the gauged form's 800 bytes per site are not to be had (a single
     // length R takes 432): the line products of every chain
     int r = ctx->ensure_meas(Rmax, Tmax, true);
     if (r == MAG_ERR_NOMEM && ctx->wg_links) {

@@ -89,6 +89,17 @@ def test_links_that_drifted_off_unitarity_keep_their_loops(dims, T):
         assert abs(W[r - 1, t - 1] - O.wilson_loop(dims, U, (r, 0, 0), t)) <= 12 * 2.0**-53 * (2 * (r + t) + 4 * dims[3]) / 10
 
 
+@pytest.mark.parametrize("dims,R,T", [((2, 2, 2, 300), 2, 5), ((4, 4, 6, 201), 2, 4), ((6, 5, 6, 97), 2, 8),
+                                      ((8, 8, 8, 33), 2, 4)])
+def test_two_slices_per_thread_and_an_odd_number_of_slots(dims, R, T):
+    """One, two, four and eight spatial sites per block; Lt + Tmax odd, so that the last slot of the second
+    slices stays empty; Lt odd, so that the last thread has one slice."""
+    U = O.gen_hot(dims, 24)
+    with M.Chmc(dims, mag=0) as c:
+        c.set_gauge(U)
+        _compare(c, dims, U, R, T)
+
+
 def test_one_chain_of_an_ensemble():
     dims = [(4, 4, 4, 4), (2, 4, 4, 6)]
     with M.Chmc(chains=[dict(dims=d) for d in dims], mag=2) as c:
