@@ -688,7 +688,7 @@ def run_gpu(args, params, rank, world, dist):
         sub["config1_8x8x8x8_thin_demon"] = sub_run(M, "8x8x8x8_iwasaki_thin", ("fp64",), args)
         sub["config2_16x16x16x32"] = sub_run(M, "16x16x16x32_iwasaki_3stout", ("fp64", "mixed"), args)
         sub["ensemble_96chains"] = sub_run(M, "ensemble_96chains", ("mixed",), args)
-        # 48^3 x 96 (10.6M sites, 72 GB in mixed precision): 4.4 s per trajectory, so 3 warm-up and 3
+        # 48^3 x 96 (10.6M sites, 86 GB in mixed precision): 2.8 s per trajectory, so 3 warm-up and 3
         # timed trajectories, each followed by the Wilson loops R, T <= 8
         sub["config5_48x48x48x96_wloops"] = sub_run(M, "48x48x48x96_iwasaki_3stout_wloops", ("mixed",), args,
                                                     steps=min(args.steps, 3), warmup=min(args.warmup, 3))

@@ -26,7 +26,9 @@ int mag_time_force(mag_ctx* ctx, int reps, double* ms_per_eval);
    the top links, two launches), "stout_level" (one forward level),
    "chain_gather" (Lambda of a level from the derivative above it),
    "plaq_chain" (one level of the chain rule) and "lambda" (force terms of the
-   top links and Lambda of the top level, Wilson action, two launches).  Of the one-thread-per-link form (mag_autotune):
+   top links and Lambda of the top level, Wilson action, two launches);
+   MAG_ERR_STATE in a context made without the plaquette form's fields (which
+   is done where they do not fit).  Of the one-thread-per-link form (mag_autotune):
    "force", "staple", "stout_forward", "stout_lambda", "stout_chain".  Also
    "evolve", "kick", "action", and the NERSC payload kernels on chain 0's
    3x3 payload made from the current links: "nersc_swap" (byte order +
@@ -35,8 +37,8 @@ int mag_time_force(mag_ctx* ctx, int reps, double* ms_per_eval);
 int mag_time_kernel(mag_ctx* ctx, const char* which, int reps, double* ms_per_launch);
 /* Forces are evaluated over plaquettes, with launch shapes that the lattice's
    size and the precision decide.  The older one-thread-per-link form (matrix
-   derivatives) is kept for what mag_set_kernel_variant selects and as a
-   measure; this is its tuner: time every variant of its staple / force / stout
+   derivatives) is kept for what mag_set_kernel_variant selects, for contexts
+   without room for the plaquette form's fields and as a measure; this is its tuner: time every variant of its staple / force / stout
    kernels on the live fields (`reps` launches each) and keep the fastest for
    that form.  It does not change which form a context's forces take.  Variants: one thread per link at minimum blocks per SM 2..5
    ("t1m2".."t1m5", register caps), and for the staple, force and chain-rule

@@ -9,9 +9,10 @@
 // one-thread-per-link chain rule and 156 instead of 450 loaded reals, because a
 // plaquette is formed once for its four links; the price is 1.8 KB per site (FP64)
 // of intermediate results.  Measured at 32^4 (ms per launch): chain rule + Lambda
-// 1.65 + 0.57 FP64, 0.69 + 0.24 FP32 before; k_plaq_chain + k_chain_gather 0.70 +
-// 0.33 FP64, 0.38 + 0.17 FP32.  k_chain_gather (2.0 KB per site) runs at the HBM
-// rate (6.6 TB/s at FP64); k_plaq_chain at about half the FP64 pipe, 12 warps per SM.
+// 1.65 + 0.57 FP64, 0.69 + 0.24 FP32 before; k_plaq_chain + k_chain_gather 0.72 +
+// 0.31 FP64, 0.36 + 0.16 FP32 at the power cap of a run (k_plaq_chain 0.59 by itself at
+// full clock).  k_chain_gather moves 1.7 KB per site at 0.9 of the HBM rate (5.8 TB/s in
+// FP64); k_plaq_chain keeps the FP64 pipe 61% busy at 12 warps per SM.
 #include "kernels.h"
 #include "plaq_ops.cuh"
 
@@ -454,8 +455,8 @@ void launch_stout_level(const DevGeom& g, LinkPlanes<double> U, LinkPlanes<doubl
 template <typename T>
 void launch_plaq_chain(const DevGeom& g, LinkPlanes<T> U, AlgPlanes<T> Lam, AlgPlanes<T> Loc, AlgPlanes<T> Rem,
                        cudaStream_t s) {
-    // blocks of six warps per SM: two of FP64 (168 registers, no spills; three would spill 1 KB:
-    // 1.47 against 0.83 ms at 32^4), three of FP32 (96 registers; 0.369 against 0.431 ms)
+    // blocks of six warps per SM: two of FP64 (168 registers, no spills; three would spill 1 KB
+    // and take 1.8 times as long), three of FP32 (96 registers; two 0.431 against 0.369 ms at 32^4)
     if constexpr (sizeof(T) == 8) {
         if (tiles(g) <= kSoloTiles) return launch_after(k_plaq_chain<T, 1>, tiles(g), kPlaqBlock, 0, s, g, U, Lam, Loc, Rem);
     }
@@ -489,7 +490,7 @@ void launch_plaq_rect(const DevGeom& g, LinkPlanes<T> U, RowPlanes<T> Pl, AlgPla
                       cudaStream_t s) {
     launch_after(k_plaq<T>, tiles(g), kPlaqBlock, 0, s, g, U, Pl);
     // two blocks of six warps per SM in both precisions (three: 0.81 against 0.75 ms FP32 at 32^4,
-    // twice as slow in FP64, from spills)
+    // twice as slow in FP64, from spills; with two FP64 spills 136 bytes at 168 registers)
     if constexpr (sizeof(T) == 8) {
         if (tiles(g) <= kSoloTiles) return launch_after(k_plaq_rect<T, 1>, tiles(g), kPlaqBlock, 0, s, g, U, Pl, Loc, Rem);
     }
